@@ -30,6 +30,7 @@
 #include "sph_kernels.h"
 #include "sph_noise.cuh"
 #include "sph_snapshot.h"
+#include "sph_sort_small.cuh"
 #include "sph_warp.cuh"
 
 using namespace phieng;
@@ -549,14 +550,28 @@ __global__ void __launch_bounds__(256) k_keys3(const float4* __restrict__ pos, u
   count_key(count, k);
 }
 
+// Writes a particle's sorted entries at final slot f.
+struct Gather3 {
+  const float4 *pos, *vel;
+  const float* mass;
+  const uint8_t* phase;
+  uint32_t *skey, *sid;
+  float4 *spos, *svel;
+  float* smass;     // null: uniform
+  uint8_t* sphase;  // null: uniform
+  __device__ __forceinline__ void operator()(uint32_t f, uint32_t k, uint32_t id) const {
+    skey[f] = k;
+    sid[f] = id;
+    spos[f] = pos[id];
+    svel[f] = vel[id];
+    if (smass) smass[f] = mass[id];
+    if (sphase) sphase[f] = phase[id];
+  }
+};
+
 // In-bucket rank by id, then the gather into sorted order.
 __global__ void __launch_bounds__(256) k_fixup3(const uint32_t* __restrict__ tkey, const uint32_t* __restrict__ tid_in,
-                                                const uint32_t* __restrict__ start, uint32_t n,
-                                                uint32_t* __restrict__ skey, uint32_t* __restrict__ sid,
-                                                const float4* __restrict__ pos, const float4* __restrict__ vel,
-                                                const float* __restrict__ mass, const uint8_t* __restrict__ phase,
-                                                float4* __restrict__ spos, float4* __restrict__ svel,
-                                                float* __restrict__ smass, uint8_t* __restrict__ sphase) {
+                                                const uint32_t* __restrict__ start, uint32_t n, Gather3 ga) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t k = tkey[s];
@@ -564,13 +579,7 @@ __global__ void __launch_bounds__(256) k_fixup3(const uint32_t* __restrict__ tke
   const uint32_t lo = start[k], hi = start[k + 1];
   uint32_t rank = 0;
   for (uint32_t j = lo; j < hi; j++) rank += __ldg(&tid_in[j]) < id ? 1u : 0u;
-  const uint32_t f = lo + rank;
-  skey[f] = k;
-  sid[f] = id;
-  spos[f] = pos[id];
-  svel[f] = vel[id];
-  if (smass) smass[f] = mass[id];
-  if (sphase) sphase[f] = phase[id];
+  ga(lo + rank, k, id);
 }
 
 __device__ __forceinline__ uint32_t row_base3(uint32_t by, uint32_t bz, int r, const GridPlan3& g) {
@@ -657,13 +666,16 @@ __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spo
   spres[s] = p;
 }
 
-// One neighbour pair of the force loop (fluid3.rs:1040-1084) and of the XSPH
-// sum (fluid3.rs:1111-1123), accumulated in the reference's order.
+// Terms of one neighbour pair of the force loop (fluid3.rs:1040-1084) and of
+// the XSPH sum (fluid3.rs:1111-1123): the force sum takes na (the negated
+// pressure term), then co (the negated cohesion term, +0 where there is none:
+// a sum that starts at +0 never holds -0, so adding +0 changes nothing), the
+// XSPH sum xs. Adding a negated product is subtracting it.
 template <bool MASS, bool PLAIN>
-__device__ __forceinline__ void pair3(uint32_t j, float4 pi, float4 vi, float rho_i, float q_i, float m_i,
-                                      const float4* __restrict__ spos, const float4* __restrict__ svel,
-                                      const float2* __restrict__ sdq, const float* __restrict__ smass,
-                                      const StepParams3& P, float (&f)[3], float (&sm)[3]) {
+__device__ __forceinline__ void pair3_terms(uint32_t j, float4 pi, float4 vi, float rho_i, float q_i, float m_i,
+                                            const float4* __restrict__ spos, const float4* __restrict__ svel,
+                                            const float2* __restrict__ sdq, const float* __restrict__ smass,
+                                            const StepParams3& P, float (&na)[3], float (&co)[3], float (&xs)[3]) {
   const float4 pj = __ldg(&spos[j]);
   const float2 dqj = __ldg(&sdq[j]);
   const float4 vj = __ldg(&svel[j]);
@@ -691,25 +703,43 @@ __device__ __forceinline__ void pair3(uint32_t j, float4 pi, float4 vi, float rh
     }
   }
   const float mt = __fmul_rn(m_j, term);
-  f[0] = __fsub_rn(f[0], __fmul_rn(g0, mt));
-  f[1] = __fsub_rn(f[1], __fmul_rn(g1, mt));
-  f[2] = __fsub_rn(f[2], __fmul_rn(g2, mt));
+  na[0] = -__fmul_rn(g0, mt);
+  na[1] = -__fmul_rn(g1, mt);
+  na[2] = -__fmul_rn(g2, mt);
+  co[0] = co[1] = co[2] = 0.0f;
   if (!PLAIN && (P.flags & F_COHESION) && dist > kEps) {
     const float c = dist >= P.hk ? 0.0f : __fsub_rn(1.0f, __fdiv_rn(dist, P.hk));
     if (c > 0.0f) {
       const float sc = __fmul_rn(__fmul_rn(__fmul_rn(P.surface_tension, m_i), m_j), c);
-      f[0] = __fsub_rn(f[0], __fmul_rn(__fdiv_rn(dx, dist), sc));
-      f[1] = __fsub_rn(f[1], __fmul_rn(__fdiv_rn(dy, dist), sc));
-      f[2] = __fsub_rn(f[2], __fmul_rn(__fdiv_rn(dz, dist), sc));
+      co[0] = -__fmul_rn(__fdiv_rn(dx, dist), sc);
+      co[1] = -__fmul_rn(__fdiv_rn(dy, dist), sc);
+      co[2] = -__fmul_rn(__fdiv_rn(dz, dist), sc);
     }
   }
+  xs[0] = xs[1] = xs[2] = 0.0f;
   if (PLAIN || (P.flags & F_VISC)) {
     const float rho_bar = __fmul_rn(0.5f, __fadd_rn(rho_i, rho_j));
     const float w = PLAIN ? poly6_nb<false>(d2, P) : poly6_3(d2, P);
     const float mr = __fdiv_rn(m_j, rho_bar);
-    sm[0] = __fadd_rn(sm[0], __fmul_rn(__fmul_rn(__fsub_rn(vj.x, vi.x), mr), w));
-    sm[1] = __fadd_rn(sm[1], __fmul_rn(__fmul_rn(__fsub_rn(vj.y, vi.y), mr), w));
-    sm[2] = __fadd_rn(sm[2], __fmul_rn(__fmul_rn(__fsub_rn(vj.z, vi.z), mr), w));
+    xs[0] = __fmul_rn(__fmul_rn(__fsub_rn(vj.x, vi.x), mr), w);
+    xs[1] = __fmul_rn(__fmul_rn(__fsub_rn(vj.y, vi.y), mr), w);
+    xs[2] = __fmul_rn(__fmul_rn(__fsub_rn(vj.z, vi.z), mr), w);
+  }
+}
+
+// One pair accumulated in the reference's order.
+template <bool MASS, bool PLAIN>
+__device__ __forceinline__ void pair3(uint32_t j, float4 pi, float4 vi, float rho_i, float q_i, float m_i,
+                                      const float4* __restrict__ spos, const float4* __restrict__ svel,
+                                      const float2* __restrict__ sdq, const float* __restrict__ smass,
+                                      const StepParams3& P, float (&f)[3], float (&sm)[3]) {
+  float na[3], co[3], xs[3];
+  pair3_terms<MASS, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, P, na, co, xs);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    f[c] = __fadd_rn(f[c], na[c]);
+    if (!PLAIN) f[c] = __fadd_rn(f[c], co[c]);
+    sm[c] = __fadd_rn(sm[c], xs[c]);
   }
 }
 
@@ -720,10 +750,12 @@ __device__ __forceinline__ void pair3(uint32_t j, float4 pi, float4 vi, float rh
 // pair, fused multiply-adds. The XSPH sum leaves out its constant factor
 // 2 m c_poly6 (m / rho_bar * poly6 = 2 m c_poly6 t^3 / (rho_i + rho_j)),
 // which k_force3 applies once per particle. mq_i = m q_i.
-__device__ __forceinline__ void pair3_fast(uint32_t j, float4 pi, float4 vi, float rho_i, float mq_i,
-                                           const float4* __restrict__ spos, const float4* __restrict__ svel,
-                                           const float2* __restrict__ sdq, const StepParams3& P, float (&f)[3],
-                                           float (&sm)[3]) {
+// pair3_fast_terms gives the factors: the sums are f = fma(-d, c, f) and
+// sm = fma(dv, w, sm) per axis.
+__device__ __forceinline__ void pair3_fast_terms(uint32_t j, float4 pi, float4 vi, float rho_i, float mq_i,
+                                                 const float4* __restrict__ spos, const float4* __restrict__ svel,
+                                                 const float2* __restrict__ sdq, const StepParams3& P, float (&nd)[3],
+                                                 float (&dv)[3], float& c, float& w) {
   const float4 pj = __ldg(&spos[j]);
   const float2 dqj = __ldg(&sdq[j]);
   const float4 vj = __ldg(&svel[j]);
@@ -734,15 +766,24 @@ __device__ __forceinline__ void pair3_fast(uint32_t j, float4 pi, float4 vi, flo
   const float hr = __fsub_rn(P.hk, r);
   const bool grad = r < P.hk && r >= kEps;  // spiky_grad's support
   const float gs = grad ? __fmul_rn(__fmul_rn(__fmul_rn(P.c_spiky, hr), hr), rinv) : 0.0f;
-  const float c = __fmul_rn(gs, __fmaf_rn(P.mass, dqj.y, mq_i));  // m (q_i + q_j)
-  f[0] = __fmaf_rn(-dx, c, f[0]);
-  f[1] = __fmaf_rn(-dy, c, f[1]);
-  f[2] = __fmaf_rn(-dz, c, f[2]);
+  c = __fmul_rn(gs, __fmaf_rn(P.mass, dqj.y, mq_i));  // m (q_i + q_j)
+  nd[0] = -dx, nd[1] = -dy, nd[2] = -dz;
   const float t = __fsub_rn(P.hk2, d2);
-  const float w = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), __fdividef(1.0f, __fadd_rn(rho_i, fmaxf(dqj.x, kEps))));
-  sm[0] = __fmaf_rn(__fsub_rn(vj.x, vi.x), w, sm[0]);
-  sm[1] = __fmaf_rn(__fsub_rn(vj.y, vi.y), w, sm[1]);
-  sm[2] = __fmaf_rn(__fsub_rn(vj.z, vi.z), w, sm[2]);
+  w = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), __fdividef(1.0f, __fadd_rn(rho_i, fmaxf(dqj.x, kEps))));
+  dv[0] = __fsub_rn(vj.x, vi.x), dv[1] = __fsub_rn(vj.y, vi.y), dv[2] = __fsub_rn(vj.z, vi.z);
+}
+
+__device__ __forceinline__ void pair3_fast(uint32_t j, float4 pi, float4 vi, float rho_i, float mq_i,
+                                           const float4* __restrict__ spos, const float4* __restrict__ svel,
+                                           const float2* __restrict__ sdq, const StepParams3& P, float (&f)[3],
+                                           float (&sm)[3]) {
+  float nd[3], dv[3], c, w;
+  pair3_fast_terms(j, pi, vi, rho_i, mq_i, spos, svel, sdq, P, nd, dv, c, w);
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    f[a] = __fmaf_rn(nd[a], c, f[a]);
+    sm[a] = __fmaf_rn(dv[a], w, sm[a]);
+  }
 }
 
 // Ghost pressure on a fluid particle (fluid3.rs:1073-1083), after its fluid
@@ -920,6 +961,91 @@ __global__ void k_resample_prep3(const uint32_t* __restrict__ sid, uint32_t n, u
   if (phase_uniform) phase[s] = phase_value;
 }
 
+// The rest of the force pass from a particle's neighbour sums: integrate and
+// walls (fluid3.rs:1085-1176), the new state (id order), the next key and its
+// bucket count. DEBUG: the force only. Where several lanes hold the same
+// particle, one of them is the writer.
+template <bool DEBUG, bool PLAIN, bool FAST>
+__device__ __forceinline__ void finish3(uint32_t id, bool writer, float4 pi, float4 vi, float rho_i, float q_i,
+                                        float (&f)[3], float (&sm)[3], const StepParams3& P,
+                                        const DevBody3* __restrict__ bodies, float4* __restrict__ pos_out,
+                                        float4* __restrict__ vel_out, uint32_t* __restrict__ key_out,
+                                        uint32_t* __restrict__ count_out, float4* __restrict__ dbg) {
+  if constexpr (FAST) {
+    const float xs = __fmul_rn(__fmul_rn(2.0f, P.mass), P.c_poly6);  // pair3_fast's XSPH factor
+    sm[0] = __fmul_rn(sm[0], xs);
+    sm[1] = __fmul_rn(sm[1], xs);
+    sm[2] = __fmul_rn(sm[2], xs);
+  }
+  if (!PLAIN && (P.flags & F_GHOST)) {  // PLAIN launches exclude F_GHOST
+    const float3 gf = ghost_force3(pi, q_i, f[0], f[1], f[2], P);
+    f[0] = gf.x;
+    f[1] = gf.y;
+    f[2] = gf.z;
+  }
+  if (DEBUG) {
+    if (writer) dbg[id] = make_float4(f[0], f[1], f[2], 0.0f);
+    return;
+  }
+  float ax = __fadd_rn(P.gx, __fdiv_rn(f[0], rho_i));
+  float ay = __fadd_rn(P.gy, __fdiv_rn(f[1], rho_i));
+  float az = __fadd_rn(P.gz, __fdiv_rn(f[2], rho_i));
+  if (!PLAIN && (P.flags & F_TURB)) {  // fluid3.rs:1096-1108, at the pre-step position and the step's clock
+    const float3 tb = turbulence_accel3(pi.x, pi.y, pi.z, *P.clock, P.turb_freq, P.turb_tscale, P.turb_seed,
+                                        P.turb_oct, P.flags & F_TURB_CURL, P.turb_amp);
+    ax = __fadd_rn(ax, tb.x);
+    ay = __fadd_rn(ay, tb.y);
+    az = __fadd_rn(az, tb.z);
+  }
+  float vx = __fadd_rn(vi.x, __fmul_rn(ax, P.dt));
+  float vy = __fadd_rn(vi.y, __fmul_rn(ay, P.dt));
+  float vz = __fadd_rn(vi.z, __fmul_rn(az, P.dt));
+  if (P.flags & F_VISC) {
+    vx = __fadd_rn(vx, __fmul_rn(sm[0], P.visc));
+    vy = __fadd_rn(vy, __fmul_rn(sm[1], P.visc));
+    vz = __fadd_rn(vz, __fmul_rn(sm[2], P.visc));
+  }
+  const float speed = __fsqrt_rn(dot3(vx, vy, vz, vx, vy, vz));
+  if (speed > P.vmax) {
+    const float sc = __fdiv_rn(P.vmax, speed);
+    vx = __fmul_rn(vx, sc);
+    vy = __fmul_rn(vy, sc);
+    vz = __fmul_rn(vz, sc);
+  }
+  if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz)) vx = vy = vz = 0.0f;
+  float x = __fadd_rn(pi.x, __fmul_rn(vx, P.dt));
+  float y = __fadd_rn(pi.y, __fmul_rn(vy, P.dt));
+  float z = __fadd_rn(pi.z, __fmul_rn(vz, P.dt));
+  if (!isfinite(x) || !isfinite(y) || !isfinite(z)) {
+    x = pi.x;
+    y = pi.y;
+    z = pi.z;
+  }
+  if (P.flags & F_QBODIES) {
+    // the engine's bodies (phieng_sph3_step_fluid)
+    const uint32_t r = walls3q(x, y, z, vx, vy, vz, P);
+    if (!writer) return;
+    pos_out[id] = make_float4(x, y, z, 0.0f);
+    vel_out[id] = make_float4(vx, vy, vz, 0.0f);
+    if (P.flags & F_DYNAMIC) {
+      // contacts with bodies that react run in particle order (k_dynamic_walls3)
+      P.dcount[id] = r != kNoDefer ? 1u : 0u;
+      if (r != kNoDefer) {
+        P.defer[id] = r;
+        return;
+      }
+    }
+  } else {
+    walls3(x, y, z, vx, vy, vz, bodies, P);
+    if (!writer) return;
+    pos_out[id] = make_float4(x, y, z, 0.0f);
+    vel_out[id] = make_float4(vx, vy, vz, 0.0f);
+  }
+  const uint32_t nk = bucket_key3(x, y, z, P.grid);
+  key_out[id] = nk;
+  atomicAdd(&count_out[nk], 1u);  // one atomic per particle, as the 2D force pass
+}
+
 // Force + XSPH + integrate + walls (fluid3.rs:1040-1176); writes the new
 // state (id order), the next key and its bucket count. DEBUG: forces only.
 // FAST (tolerance mode; PLAIN, uniform mass): pair3_fast's arithmetic.
@@ -1002,78 +1128,10 @@ __global__ void __launch_bounds__(256) k_force3(const float4* __restrict__ spos,
       }
     }
   }
-  if constexpr (FAST) {
-    const float xs = __fmul_rn(__fmul_rn(2.0f, P.mass), P.c_poly6);  // pair3_fast's XSPH factor
-    sm[0] = __fmul_rn(sm[0], xs);
-    sm[1] = __fmul_rn(sm[1], xs);
-    sm[2] = __fmul_rn(sm[2], xs);
-  }
-  if (!PLAIN && (P.flags & F_GHOST)) {  // PLAIN launches exclude F_GHOST
-    const float3 gf = ghost_force3(pi, q_i, f[0], f[1], f[2], P);
-    f[0] = gf.x;
-    f[1] = gf.y;
-    f[2] = gf.z;
-  }
-  if (DEBUG) {
-    dbg[id] = make_float4(f[0], f[1], f[2], 0.0f);
-    return;
-  }
-  float ax = __fadd_rn(P.gx, __fdiv_rn(f[0], rho_i));
-  float ay = __fadd_rn(P.gy, __fdiv_rn(f[1], rho_i));
-  float az = __fadd_rn(P.gz, __fdiv_rn(f[2], rho_i));
-  if (!PLAIN && (P.flags & F_TURB)) {  // fluid3.rs:1096-1108, at the pre-step position and the step's clock
-    const float3 tb = turbulence_accel3(pi.x, pi.y, pi.z, *P.clock, P.turb_freq, P.turb_tscale, P.turb_seed,
-                                        P.turb_oct, P.flags & F_TURB_CURL, P.turb_amp);
-    ax = __fadd_rn(ax, tb.x);
-    ay = __fadd_rn(ay, tb.y);
-    az = __fadd_rn(az, tb.z);
-  }
-  float vx = __fadd_rn(vi.x, __fmul_rn(ax, P.dt));
-  float vy = __fadd_rn(vi.y, __fmul_rn(ay, P.dt));
-  float vz = __fadd_rn(vi.z, __fmul_rn(az, P.dt));
-  if (P.flags & F_VISC) {
-    vx = __fadd_rn(vx, __fmul_rn(sm[0], P.visc));
-    vy = __fadd_rn(vy, __fmul_rn(sm[1], P.visc));
-    vz = __fadd_rn(vz, __fmul_rn(sm[2], P.visc));
-  }
-  const float speed = __fsqrt_rn(dot3(vx, vy, vz, vx, vy, vz));
-  if (speed > P.vmax) {
-    const float sc = __fdiv_rn(P.vmax, speed);
-    vx = __fmul_rn(vx, sc);
-    vy = __fmul_rn(vy, sc);
-    vz = __fmul_rn(vz, sc);
-  }
-  if (!isfinite(vx) || !isfinite(vy) || !isfinite(vz)) vx = vy = vz = 0.0f;
-  float x = __fadd_rn(pi.x, __fmul_rn(vx, P.dt));
-  float y = __fadd_rn(pi.y, __fmul_rn(vy, P.dt));
-  float z = __fadd_rn(pi.z, __fmul_rn(vz, P.dt));
-  if (!isfinite(x) || !isfinite(y) || !isfinite(z)) {
-    x = pi.x;
-    y = pi.y;
-    z = pi.z;
-  }
-  if (P.flags & F_QBODIES) {
-    // the engine's bodies (phieng_sph3_step_fluid)
-    const uint32_t r = walls3q(x, y, z, vx, vy, vz, P);
-    pos_out[id] = make_float4(x, y, z, 0.0f);
-    vel_out[id] = make_float4(vx, vy, vz, 0.0f);
-    if (P.flags & F_DYNAMIC) {
-      // contacts with bodies that react run in particle order (k_dynamic_walls3)
-      P.dcount[id] = r != kNoDefer ? 1u : 0u;
-      if (r != kNoDefer) {
-        P.defer[id] = r;
-        return;
-      }
-    }
-  } else {
-    walls3(x, y, z, vx, vy, vz, bodies, P);
-    pos_out[id] = make_float4(x, y, z, 0.0f);
-    vel_out[id] = make_float4(vx, vy, vz, 0.0f);
-  }
-  const uint32_t nk = bucket_key3(x, y, z, g);
-  key_out[id] = nk;
-  atomicAdd(&count_out[nk], 1u);  // one atomic per particle, as the 2D force pass
+  finish3<DEBUG, PLAIN, FAST>(id, true, pi, vi, rho_i, q_i, f, sm, P, bodies, pos_out, vel_out, key_out, count_out, dbg);
 }
+
+#include "sph3d_coop.cuh"
 
 __global__ void __launch_bounds__(256) k_vmax3(const float4* __restrict__ vel, uint32_t n, unsigned int* out) {
   float m = 0.0f;
@@ -1774,9 +1832,21 @@ StepParams3 make_params3(const World3* w, float dt) {
   return P;
 }
 
-void enqueue_sort3(World3* w, const StepParams3& P, cudaStream_t st) {
+// Sort by (bucket key, id) and gather. counts: the bucket counts of the keys
+// (consumed as the placement cursor); clear: zeroed after the sort when set
+// (the force pass counts the next keys there).
+void enqueue_sorted3(World3* w, const StepParams3& P, uint32_t* counts, bool by_slot, uint32_t* clear,
+                     cudaStream_t st) {
+  const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
+  const Gather3 ga{w->pos, w->vel, w->mass, w->phase, w->skey, w->sid, w->spos, w->svel, m ? w->smass : nullptr,
+                   ph ? w->sphase : nullptr};
+  const uint32_t nkeys = P.grid.sentinel + 1;
+  if (small_sort_applies(w->n, nkeys)) {
+    launch_sort_small(w->key, w->n, nkeys, w->start, clear, w->count_len, ga, st);
+    return;
+  }
   BucketSort bs;
-  bs.count = w->count;
+  bs.count = counts;
   bs.tilesum = w->tilesum;
   bs.done = w->scalar + 8;  // scan counters [8], [9]
   bs.tstate = w->tstate;
@@ -1786,18 +1856,36 @@ void enqueue_sort3(World3* w, const StepParams3& P, cudaStream_t st) {
   bs.sid_prev = w->sid;
   bs.tkey = w->tkey;
   bs.tid = w->tid;
-  enqueue_bucket_place(bs, w->n, P.grid.sentinel + 1, w->sid_perm_n == w->n, st);
-  const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
-  k_fixup3<<<cdiv(w->n, 256), 256, 0, st>>>(w->tkey, w->tid, w->start, w->n, w->skey, w->sid, w->pos, w->vel, w->mass,
-                                            w->phase, w->spos, w->svel, m ? w->smass : nullptr,
-                                            ph ? w->sphase : nullptr);
-  cudaMemsetAsync(w->count, 0, sizeof(uint32_t) * w->count_len, st);
+  enqueue_bucket_place(bs, w->n, nkeys, by_slot, st);
+  k_fixup3<<<cdiv(w->n, 256), 256, 0, st>>>(w->tkey, w->tid, w->start, w->n, ga);
+  if (clear) cudaMemsetAsync(clear, 0, sizeof(uint32_t) * w->count_len, st);
+}
+
+void enqueue_sort3(World3* w, const StepParams3& P, cudaStream_t st) {
+  enqueue_sorted3(w, P, w->count, w->sid_perm_n == w->n, w->count, st);
 }
 
 void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
   const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
   const uint32_t g = cdiv(w->n, 256);
   const bool wide = (P.flags & F_WIDE_NB) != 0;
+  if (w->n <= kRowsMax3) {
+#define PHIENG_D3C(M, PH, WD)                                                                                \
+  k_density3_rows<M, PH, WD><<<cdiv(w->n, 32), 288, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, \
+                                                             w->start, P, w->sdq, w->spres, w->nmask)
+#define PHIENG_D3G(M, PH)                       \
+  do {                                          \
+    if (wide) PHIENG_D3C(M, PH, true);          \
+    else PHIENG_D3C(M, PH, false);              \
+  } while (0)
+    if (m && ph) PHIENG_D3G(true, true);
+    else if (m) PHIENG_D3G(true, false);
+    else if (ph) PHIENG_D3G(false, true);
+    else PHIENG_D3G(false, false);
+#undef PHIENG_D3G
+#undef PHIENG_D3C
+    return;
+  }
 #define PHIENG_D3(M, PH)                                                                                     \
   do {                                                                                                       \
     if (wide)                                                                                                \
@@ -1822,6 +1910,27 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
   const bool plain = (P.flags & F_VISC) && !(P.flags & (F_AV | F_COHESION | F_WIDE_NB | F_TURB | F_GHOST));
   // tolerance mode: the plain pass with uniform mass runs pair3_fast
   const bool fast = plain && !m && (P.flags & F_FAST);
+  if (w->n <= kCoopMax3) {
+#define PHIENG_F3G(M, D, PL, FA)                                                                           \
+  k_force3_coop<M, D, PL, FA><<<cdiv(w->n, kCoopThreads / kCoopLanes), kCoopThreads, 0, st>>>(             \
+      w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, P, w->dbodies, w->nmask, w->pos, \
+      w->vel, w->key, w->count, dbg)
+    if (fast) {
+      if (dbg) PHIENG_F3G(false, true, true, true);
+      else PHIENG_F3G(false, false, true, true);
+    } else if (dbg) {
+      if (m) PHIENG_F3G(true, true, false, false);
+      else PHIENG_F3G(false, true, false, false);
+    } else if (plain) {
+      if (m) PHIENG_F3G(true, false, true, false);
+      else PHIENG_F3G(false, false, true, false);
+    } else {
+      if (m) PHIENG_F3G(true, false, false, false);
+      else PHIENG_F3G(false, false, false, false);
+    }
+#undef PHIENG_F3G
+    return;
+  }
 #define PHIENG_F3X(M, D, PL, FA)                                                                                    \
   k_force3<M, D, PL, FA><<<g, 128, 0, st>>>(w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
                                             P, w->dbodies, w->nmask, w->pos, w->vel, w->key, w->count, dbg)
@@ -2209,21 +2318,7 @@ void enqueue_resort3(World3* w, const StepParams3& P, cudaStream_t st) {
   const uint32_t g = cdiv(w->n, 256);
   k_dp_to_id3<<<g, 256, 0, st>>>(w->sdq, w->spres, w->sid, w->n, w->d_dq_id, w->d_p_id);
   cudaMemcpyAsync(w->d_count2, w->count, sizeof(uint32_t) * w->count_len, cudaMemcpyDeviceToDevice, st);
-  BucketSort bs;
-  bs.count = w->d_count2;
-  bs.tilesum = w->tilesum;
-  bs.done = w->scalar + 8;
-  bs.tstate = w->tstate;
-  bs.err = w->scalar + 12;
-  bs.start = w->start;
-  bs.key = w->key;
-  bs.sid_prev = w->sid;
-  bs.tkey = w->tkey;
-  bs.tid = w->tid;
-  enqueue_bucket_place(bs, w->n, P.grid.sentinel + 1, true, st);
-  const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
-  k_fixup3<<<g, 256, 0, st>>>(w->tkey, w->tid, w->start, w->n, w->skey, w->sid, w->pos, w->vel, w->mass, w->phase,
-                              w->spos, w->svel, m ? w->smass : nullptr, ph ? w->sphase : nullptr);
+  enqueue_sorted3(w, P, w->d_count2, true, nullptr, st);
   k_dp_from_id3<<<g, 256, 0, st>>>(w->d_dq_id, w->d_p_id, w->sid, w->n, w->sdq, w->spres);
 }
 
