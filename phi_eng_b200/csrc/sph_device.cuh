@@ -224,6 +224,14 @@ __device__ __forceinline__ float eos(float density, float rho0, const PP& P) {
   return fmaxf(__fmul_rn(__fmul_rn(P.stiffness, r0), __fsub_rn(pw, 1.0f)), 0.0f);
 }
 
+// n / d for d > 0 with the zero numerators taken apart: a division with a zero
+// numerator leaves the inline path for a subroutine, and a particle against
+// the flat side of a box has one in every contact.
+__device__ __forceinline__ float div_by_length(float n, float d) {
+  const float q = __fdiv_rn(n == 0.0f ? d : n, d);
+  return n == 0.0f ? n : q;
+}
+
 // Particle vs body (fluid.rs:463-533, circle and box branches). Returns
 // false when separated. With cp: the contact point on the body surface
 // (circle: position + normal * radius; box: transform_point(clamped)).
@@ -414,8 +422,8 @@ __device__ __forceinline__ bool collide(float px, float py, float pr, const DevB
   if (l2 > kEpsSq) {
     float dist = __fsqrt_rn(l2);
     if (dist >= pr) return false;
-    lnx = __fdiv_rn(ddx, dist);
-    lny = __fdiv_rn(ddy, dist);
+    lnx = div_by_length(ddx, dist);
+    lny = div_by_length(ddy, dist);
     depth = __fsub_rn(pr, dist);
   } else {
     float dxp = __fsub_rn(hx, fabsf(lx));
@@ -446,7 +454,8 @@ __device__ __forceinline__ bool collide(float px, float py, float pr, const DevB
 // zero velocity, which the no-slip branch reads. Returns kNoDefer, or the
 // index of the first body marked dyn that the particle touches: the state is
 // then left as it was before that body, for the ordered pass to resume.
-template <bool POLY = true>
+// SHARED: the scene's bodies, in shared memory (body_first not applied).
+template <bool POLY = true, bool SHARED = false>
 __device__ __forceinline__ uint32_t walls(float& x, float& y, float& vx, float& vy,
                                           const DevBody* __restrict__ bodies, const StepParams& P) {
   if (P.flags & F_WBOX) {
@@ -462,10 +471,10 @@ __device__ __forceinline__ uint32_t walls(float& x, float& y, float& vx, float& 
     if (!near) return kNoDefer;
   }
   for (uint32_t k = 0; k < P.nbodies; k++) {
-    const DevBody* bp = bodies + P.body_first + k;
+    const DevBody* bp = bodies + (SHARED ? 0u : P.body_first) + k;
     // bounding-box reject first: only the centre and the padded extents are read
-    if (fabsf(x - __ldg(&bp->px)) > __ldg(&bp->ex) + P.pr_pad || fabsf(y - __ldg(&bp->py)) > __ldg(&bp->ey) + P.pr_pad)
-      continue;
+    auto rd = [](const float* p) { return SHARED ? *p : __ldg(p); };
+    if (fabsf(x - rd(&bp->px)) > rd(&bp->ex) + P.pr_pad || fabsf(y - rd(&bp->py)) > rd(&bp->ey) + P.pr_pad) continue;
     const DevBody b = *bp;
     float nx, ny, depth;
     if (!collide<POLY>(x, y, P.pr, b, nx, ny, depth, nullptr, P.poly)) continue;

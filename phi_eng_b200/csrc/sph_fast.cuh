@@ -203,12 +203,13 @@ __global__ void __launch_bounds__(256) k_density_fast(const float2* __restrict__
 
 // ---------------------------------------------------------------- K6 (tolerance mode)
 // One neighbour pair: pressure force into (fx, fy), the XSPH sum (before its
-// 2 m c_poly6 factor) into (sx, sy).
+// 2 m c_poly6 factor) into (sx, sy). terms() gives the factors of the sums'
+// fused multiply-adds: f += (-dx, -dy) c, s += (vj - vi) w.
 struct FastPair {
   float2 pi, vi;
   float rho_i, mq_i;
-  __device__ __forceinline__ void operator()(float2 pj, float2 vj, float2 dqj, const StepParams& P, float& fx,
-                                             float& fy, float& sx, float& sy) const {
+  __device__ __forceinline__ void terms(float2 pj, float2 vj, float2 dqj, const StepParams& P, float2& nd, float& c,
+                                        float2& dv, float& w) const {
     const float dx = __fsub_rn(pi.x, pj.x);
     const float dy = __fsub_rn(pi.y, pj.y);
     const float d2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
@@ -217,13 +218,21 @@ struct FastPair {
     const float hr = __fsub_rn(P.hk, r);
     const bool grad = r < P.hk && r >= kEps;  // spiky_grad's support (fluid.rs:280)
     const float gs = grad ? __fmul_rn(__fmul_rn(__fmul_rn(P.c_spiky, hr), hr), rinv) : 0.0f;
-    const float c = __fmul_rn(gs, __fmaf_rn(P.mass, dqj.y, mq_i));  // m (q_i + q_j)
-    fx = __fmaf_rn(-dx, c, fx);
-    fy = __fmaf_rn(-dy, c, fy);
+    c = __fmul_rn(gs, __fmaf_rn(P.mass, dqj.y, mq_i));  // m (q_i + q_j)
+    nd = make_float2(-dx, -dy);
     const float t = __fsub_rn(P.hk2, d2);
-    const float w = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), __fdividef(1.0f, __fadd_rn(rho_i, fmaxf(dqj.x, kEps))));
-    sx = __fmaf_rn(__fsub_rn(vj.x, vi.x), w, sx);
-    sy = __fmaf_rn(__fsub_rn(vj.y, vi.y), w, sy);
+    w = __fmul_rn(__fmul_rn(__fmul_rn(t, t), t), __fdividef(1.0f, __fadd_rn(rho_i, fmaxf(dqj.x, kEps))));
+    dv = make_float2(__fsub_rn(vj.x, vi.x), __fsub_rn(vj.y, vi.y));
+  }
+  __device__ __forceinline__ void operator()(float2 pj, float2 vj, float2 dqj, const StepParams& P, float& fx,
+                                             float& fy, float& sx, float& sy) const {
+    float2 nd, dv;
+    float c, w;
+    terms(pj, vj, dqj, P, nd, c, dv, w);
+    fx = __fmaf_rn(nd.x, c, fx);
+    fy = __fmaf_rn(nd.y, c, fy);
+    sx = __fmaf_rn(dv.x, w, sx);
+    sy = __fmaf_rn(dv.y, w, sy);
   }
 };
 

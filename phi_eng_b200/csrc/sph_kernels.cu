@@ -20,6 +20,7 @@
 
 #include "sph_kernels.h"
 #include "sph_noise.cuh"
+#include "sph_sort_small.cuh"
 #include "sph_tc_net.cuh"
 #include "sph_warp.cuh"
 
@@ -600,21 +601,23 @@ __global__ void __launch_bounds__(256) k_density(const float2* __restrict__ spos
 }
 
 // ---------------------------------------------------------------- K6 force + integrate
-// One neighbour pair of the force loop (fluid.rs:947-990) and of the XSPH
-// sum (fluid.rs:1022-1033), accumulated in the reference's order. FEAT also
-// accumulates the closure network's neighbour aggregates (feat_pair). PLAIN:
-// the launch's flags are known to be XSPH on, artificial viscosity and
-// cohesion off, h*h <= hk*hk (plain_flags), so those tests are compiled out.
-template <bool MASS, bool FEAT, bool PLAIN = false>
-__device__ __forceinline__ void pair_terms(uint32_t j, float2 pi, float2 vi, float rho_i, float q_i, float m_i,
-                                           const float2* __restrict__ spos, const float2* __restrict__ svel,
-                                           const float2* __restrict__ sdq, const float* __restrict__ smass,
-                                           const float2* __restrict__ svp, const StepParams& P, float& fx,
-                                           float& fy, float& sx, float& sy, FeatAcc& fa) {
-  const float2 pj = __ldg(&spos[j]);
-  const float2 dqj = __ldg(&sdq[j]);
-  const float2 vj = __ldg(&svel[j]);
-  const float m_j = MASS ? __ldg(&smass[j]) : P.mass;
+// Terms of one neighbour pair of the force loop (fluid.rs:947-990) and of the
+// XSPH sum (fluid.rs:1022-1033), from the neighbour's values: the force sum
+// takes (nx, ny) (the negated pressure term), then (cx, cy) (the negated
+// cohesion term, +0 where there is none: a sum that starts at +0 never holds
+// -0, so adding +0 changes nothing), the XSPH sum (wx, wy). Adding a negated
+// product is subtracting it. (gx, gy) is the spiky gradient, d2 the squared
+// distance. PLAIN: the launch's flags are known to be XSPH on, artificial
+// viscosity and cohesion off, h*h <= hk*hk (plain_flags), so those tests are
+// compiled out.
+struct PairTerms {
+  float nx, ny, cx, cy, wx, wy, gx, gy, d2;
+};
+
+template <bool PLAIN>
+__device__ __forceinline__ PairTerms pair2_terms(float2 pj, float2 vj, float2 dqj, float m_j, float2 pi, float2 vi,
+                                                 float rho_i, float q_i, float m_i, const StepParams& P) {
+  PairTerms t;
   const float rho_j = fmaxf(dqj.x, kEps);
   // delta = p_i - p_j; |delta|^2 equals the neighbour test's d2 bit for bit
   const float dx = __fsub_rn(pi.x, pj.x);
@@ -628,13 +631,6 @@ __device__ __forceinline__ void pair_terms(uint32_t j, float2 pi, float2 vi, flo
     const float sc = __fmul_rn(__fmul_rn(P.c_spiky, hr), hr);
     gxx = __fmul_rn(__fdiv_rn(dx, dist), sc);
     gyy = __fmul_rn(__fdiv_rn(dy, dist), sc);
-  }
-  if constexpr (FEAT) {
-    // PLAIN: d2 < hg2 <= hk2, so poly6's range test passes (and the XSPH
-    // term's poly6_nb is the same value)
-    const float2 vp = __ldg(&svp[j]);
-    feat_pair<!PLAIN>(fa, gxx, gyy, PLAIN ? poly6_nb<false>(d2, P) : poly6(d2, P), vp.x, vp.y, m_j, q_i, dqj.y,
-                      __fsub_rn(vj.x, vi.x), __fsub_rn(vj.y, vi.y));
   }
   float term = __fadd_rn(q_i, dqj.y);
   if (!PLAIN && (P.flags & F_AV) && dist > kEps) {
@@ -651,25 +647,60 @@ __device__ __forceinline__ void pair_terms(uint32_t j, float2 pi, float2 vi, flo
     }
   }
   const float mt = __fmul_rn(m_j, term);
-  fx = __fsub_rn(fx, __fmul_rn(gxx, mt));
-  fy = __fsub_rn(fy, __fmul_rn(gyy, mt));
+  t.nx = -__fmul_rn(gxx, mt);
+  t.ny = -__fmul_rn(gyy, mt);
+  t.cx = t.cy = 0.0f;
   if (!PLAIN && (P.flags & F_COHESION) && dist > kEps) {
     // cohesion (fluid.rs:320-326, applied at :979-985)
     const float c = dist >= P.hk ? 0.0f : __fsub_rn(1.0f, __fdiv_rn(dist, P.hk));
     if (c > 0.0f) {
       const float sc = __fmul_rn(__fmul_rn(__fmul_rn(P.surface_tension, m_i), m_j), c);
-      fx = __fsub_rn(fx, __fmul_rn(__fdiv_rn(dx, dist), sc));
-      fy = __fsub_rn(fy, __fmul_rn(__fdiv_rn(dy, dist), sc));
+      t.cx = -__fmul_rn(__fdiv_rn(dx, dist), sc);
+      t.cy = -__fmul_rn(__fdiv_rn(dy, dist), sc);
     }
   }
+  t.wx = t.wy = 0.0f;
   if (PLAIN || (P.flags & F_VISC)) {
     // XSPH (fluid.rs:1022-1033) against pre-integrate neighbours
     const float rho_bar = __fmul_rn(0.5f, __fadd_rn(rho_i, rho_j));
     const float w = PLAIN ? poly6_nb<false>(d2, P) : poly6(d2, P);
     const float mr = __fdiv_rn(m_j, rho_bar);
-    sx = __fadd_rn(sx, __fmul_rn(__fmul_rn(__fsub_rn(vj.x, vi.x), mr), w));
-    sy = __fadd_rn(sy, __fmul_rn(__fmul_rn(__fsub_rn(vj.y, vi.y), mr), w));
+    t.wx = __fmul_rn(__fmul_rn(__fsub_rn(vj.x, vi.x), mr), w);
+    t.wy = __fmul_rn(__fmul_rn(__fsub_rn(vj.y, vi.y), mr), w);
   }
+  t.gx = gxx;
+  t.gy = gyy;
+  t.d2 = d2;
+  return t;
+}
+
+// One pair accumulated in the reference's order. FEAT also accumulates the
+// closure network's neighbour aggregates (feat_pair).
+template <bool MASS, bool FEAT, bool PLAIN = false>
+__device__ __forceinline__ void pair_terms(uint32_t j, float2 pi, float2 vi, float rho_i, float q_i, float m_i,
+                                           const float2* __restrict__ spos, const float2* __restrict__ svel,
+                                           const float2* __restrict__ sdq, const float* __restrict__ smass,
+                                           const float2* __restrict__ svp, const StepParams& P, float& fx,
+                                           float& fy, float& sx, float& sy, FeatAcc& fa) {
+  const float2 dqj = __ldg(&sdq[j]);
+  const float2 vj = __ldg(&svel[j]);
+  const float m_j = MASS ? __ldg(&smass[j]) : P.mass;
+  const PairTerms t = pair2_terms<PLAIN>(__ldg(&spos[j]), vj, dqj, m_j, pi, vi, rho_i, q_i, m_i, P);
+  if constexpr (FEAT) {
+    // PLAIN: d2 < hg2 <= hk2, so poly6's range test passes (and the XSPH
+    // term's poly6_nb is the same value)
+    const float2 vp = __ldg(&svp[j]);
+    feat_pair<!PLAIN>(fa, t.gx, t.gy, PLAIN ? poly6_nb<false>(t.d2, P) : poly6(t.d2, P), vp.x, vp.y, m_j, q_i, dqj.y,
+                      __fsub_rn(vj.x, vi.x), __fsub_rn(vj.y, vi.y));
+  }
+  fx = __fadd_rn(fx, t.nx);
+  fy = __fadd_rn(fy, t.ny);
+  if (!PLAIN) {
+    fx = __fadd_rn(fx, t.cx);
+    fy = __fadd_rn(fy, t.cy);
+  }
+  sx = __fadd_rn(sx, t.wx);
+  sy = __fadd_rn(sy, t.wy);
 }
 
 // Neighbour sums of sorted slot s: pressure force (fx, fy) and XSPH (sx, sy),
@@ -725,25 +756,24 @@ __device__ __forceinline__ void neighbour_sums(uint32_t s, uint32_t k, uint32_t 
 }
 
 // integrate (fluid.rs:1003-1050) from acceleration (ax, ay) and the XSPH sum,
-// then the wall pass; writes the new state, the next key and its bucket count.
-// Ambient turbulence (F_TURB) joins the acceleration first, at the particle's
-// pre-step position and the step's world clock. EXTRA = false compiles it and
-// the polygon wall test out (the PLAIN variants, whose flags exclude both).
-template <bool EXTRA = true>
-__device__ __forceinline__ void integrate_write(uint32_t id, float2 pi, float2 vi, float ax, float ay, float sx,
-                                                float sy, const StepParams& P, const DevBody* __restrict__ bodies,
-                                                float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
-                                                uint32_t* __restrict__ count_out,
-                                                uint32_t* __restrict__ defer = nullptr,
-                                                uint32_t* __restrict__ dcount = nullptr) {
+// then the wall pass: the new state (x, y, vx, vy). Returns the wall pass's
+// defer index. Ambient turbulence (F_TURB) joins the acceleration first, at the
+// particle's pre-step position and the step's world clock. EXTRA = false
+// compiles it and the polygon wall test out (the PLAIN variants, whose flags
+// exclude both).
+// SHARED: bodies points at this scene's bodies in shared memory.
+template <bool EXTRA, bool SHARED = false>
+__device__ __forceinline__ uint32_t integrate_state(float2 pi, float2 vi, float ax, float ay, float sx, float sy,
+                                                    float dt, const StepParams& P,
+                                                    const DevBody* __restrict__ bodies, float4& out) {
   if (EXTRA && (P.flags & F_TURB)) {
     const float2 tb = turbulence_accel(pi.x, pi.y, *P.clock, P.turb_freq, P.turb_tscale, P.turb_seed, P.turb_oct,
                                        P.flags & F_TURB_CURL, P.turb_amp);
     ax = __fadd_rn(ax, tb.x);
     ay = __fadd_rn(ay, tb.y);
   }
-  float vx = __fadd_rn(vi.x, __fmul_rn(ax, P.dt));
-  float vy = __fadd_rn(vi.y, __fmul_rn(ay, P.dt));
+  float vx = __fadd_rn(vi.x, __fmul_rn(ax, dt));
+  float vy = __fadd_rn(vi.y, __fmul_rn(ay, dt));
   if (P.flags & F_VISC) {
     vx = __fadd_rn(vx, __fmul_rn(sx, P.visc));
     vy = __fadd_rn(vy, __fmul_rn(sy, P.visc));
@@ -758,14 +788,29 @@ __device__ __forceinline__ void integrate_write(uint32_t id, float2 pi, float2 v
     vx = 0.0f;
     vy = 0.0f;
   }
-  float x = __fadd_rn(pi.x, __fmul_rn(vx, P.dt));
-  float y = __fadd_rn(pi.y, __fmul_rn(vy, P.dt));
+  float x = __fadd_rn(pi.x, __fmul_rn(vx, dt));
+  float y = __fadd_rn(pi.y, __fmul_rn(vy, dt));
   if (!finitef(x) || !finitef(y)) {
     x = pi.x;
     y = pi.y;
   }
-  const uint32_t r = walls<EXTRA>(x, y, vx, vy, bodies, P);
-  state_out[id] = make_float4(x, y, vx, vy);
+  const uint32_t r = walls<EXTRA, SHARED>(x, y, vx, vy, bodies, P);
+  out = make_float4(x, y, vx, vy);
+  return r;
+}
+
+// The integrate of the force passes: writes the new state, the next key and
+// its bucket count.
+template <bool EXTRA = true>
+__device__ __forceinline__ void integrate_write(uint32_t id, float2 pi, float2 vi, float ax, float ay, float sx,
+                                                float sy, const StepParams& P, const DevBody* __restrict__ bodies,
+                                                float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
+                                                uint32_t* __restrict__ count_out,
+                                                uint32_t* __restrict__ defer = nullptr,
+                                                uint32_t* __restrict__ dcount = nullptr) {
+  float4 q;
+  const uint32_t r = integrate_state<EXTRA>(pi, vi, ax, ay, sx, sy, P.dt, P, bodies, q);
+  state_out[id] = q;
   if (P.flags & F_DYNAMIC) {
     // contacts with bodies that react run in particle order (enqueue_dynamic_walls)
     dcount[id] = r != kNoDefer ? 1u : 0u;
@@ -774,7 +819,7 @@ __device__ __forceinline__ void integrate_write(uint32_t id, float2 pi, float2 v
       return;
     }
   }
-  const uint32_t nk = bucket_key(x, y, P.grid);
+  const uint32_t nk = bucket_key(q.x, q.y, P.grid);
   key_out[id] = nk;
   // bucket counts of the next substep's sort: one atomic per particle (the
   // warp-aggregated count_key measured 1.8 us slower per 2^20-particle
@@ -1128,6 +1173,7 @@ __global__ void __launch_bounds__(256) k_front_metrics(const float4* __restrict_
 
 #include "sph_fast.cuh"
 #include "sph_closure_tc.cuh"
+#include "sph_small.cuh"
 
 inline uint32_t cdiv(uint32_t a, uint32_t b) { return (a + b - 1) / b; }
 
@@ -1412,6 +1458,73 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
     else PHIENG_FORCE(false, false, false, false);
   }
 #undef PHIENG_FORCE
+}
+
+// The variant's kernel for these flags.
+template <bool FAST>
+const void* small_kernel(bool m, bool ph, bool plain) {
+  if constexpr (FAST) return (const void*)k_small_steps<false, false, true, true>;
+  if (plain) {
+    if (m && ph) return (const void*)k_small_steps<true, true, true, false>;
+    if (m) return (const void*)k_small_steps<true, false, true, false>;
+    if (ph) return (const void*)k_small_steps<false, true, true, false>;
+    return (const void*)k_small_steps<false, false, true, false>;
+  }
+  if (m && ph) return (const void*)k_small_steps<true, true, false, false>;
+  if (m) return (const void*)k_small_steps<true, false, false, false>;
+  if (ph) return (const void*)k_small_steps<false, true, false, false>;
+  return (const void*)k_small_steps<false, false, false, false>;
+}
+
+cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss,
+                                cudaStream_t st, bool* applies) {
+  *applies = false;
+  const uint32_t keys = P.grid.sentinel + 1u;
+  if (n == 0 || n > kSmallMax || keys > kSmallKeys || P.nbodies > kSmallBodies || b.batch.ptab || b.order ||
+      (P.flags & (F_TURB | F_GHOST | F_POLY | F_DYNAMIC | F_WIDE_NB)))
+    return cudaSuccess;
+  const bool fast = fast_flags(P.flags), plain = plain_flags(P.flags);
+  const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
+  const void* kernel = fast ? small_kernel<true>(m, ph, plain) : small_kernel<false>(m, ph, plain);
+  SmallArgs A;
+  A.state = b.state;
+  A.mass = b.mass;
+  A.phase = b.phase;
+  A.bodies = b.bodies;
+  A.sid = b.sid;
+  A.sdq = b.sdq;
+  A.spres = b.spres;
+  A.key = b.key;
+  A.count = b.count;
+  A.count_len = b.count_len;
+  A.substeps = ss.substeps;
+  A.n = n;
+  A.steps = ss.steps;
+  A.dt = P.dt;
+  A.cfl.on = ss.max_substeps > 1 ? 1u : 0u;
+  A.cfl.max_substeps = ss.max_substeps;
+  A.cfl.c0 = ss.c0;
+  A.cfl.cfl_h = ss.cfl_h;
+  const SmallShape sh = small_shape(n);
+  const size_t smem = sizeof(uint32_t) * small_layout(n, keys, sh.share, sh.threads, m, ph, plain).words;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sh.blocks);
+  cfg.blockDim = dim3(sh.threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = sh.blocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (r == cudaSuccess && sh.blocks > 8)
+    r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (r != cudaSuccess) return r;
+  void* args[] = {&A, const_cast<StepParams*>(&P)};
+  *applies = true;
+  return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 size_t closure_smem_bytes() { return sizeof(MlpSmem) + sizeof(__nv_bfloat16) * 256 * kXRow + sizeof(float) * 256 * 2; }

@@ -34,6 +34,8 @@ constexpr uint32_t kMaxParticles2D = 4096;  // MAX_PARTICLES_2D (fluid.rs:30)
 // and has no cap of its own.
 inline uint32_t resample_bound(uint32_t n) { return n + std::min(n, kMaxParticles2D / 2); }
 constexpr uint32_t kClockWord = 16;         // scalar word holding the step's world clock (turbulence)
+constexpr uint32_t kSubstepWord = 24;       // scalar word counting the CFL substeps of whole-step launches
+constexpr uint32_t kSmallStepsPerLaunch = 64;
 
 // AmbientConfig2::default (ambient.rs): springs, drag and turbulence off, air
 // density 1, turbulence frequency 1, time scale 1, 3 octaves.
@@ -100,6 +102,7 @@ struct World2 {
 
   int32_t error = PHIENG_SPH_OK;
   uint64_t substeps = 0;
+  bool substeps_pending = false;  // the device counted more (kSubstepWord): count_substeps
 
   // Batch of independent scenes (empty for an ordinary world): scene k owns
   // particles [first, first + count) and bodies [body_first, +nbodies), and
@@ -484,9 +487,11 @@ bool ensure_bodies(World2* w) {
 
 bool upload_scene_table(World2* w, float dt);
 
+bool ensure_keys(World2* w);
+
 // Everything a substep needs: device, buffers, current state on the device,
-// a bucket grid, the bodies and valid keys.
-bool prepare(World2* w) {
+// a bucket grid, the bodies and (unless the caller takes none) valid keys.
+bool prepare(World2* w, bool keys = true) {
   if (w->error != PHIENG_SPH_OK) return false;
   if (!ensure_device(w)) return false;
   if (!w->dev_state_valid) {
@@ -520,6 +525,11 @@ bool prepare(World2* w) {
   }
   if (!ensure_range(w)) return false;
   if (!ensure_bodies(w)) return false;
+  if (keys) return ensure_keys(w);
+  return cuda_ok(w, cudaGetLastError(), "prepare");
+}
+
+bool ensure_keys(World2* w) {
   if (!w->keys_valid) {
     if (w->is_batch() && !upload_scene_table(w, 0.0f)) return false;  // the keys read each scene's grid
     enqueue_keys(w->d, w->n, w->plan, w->stream);
@@ -716,6 +726,13 @@ bool run_substep(World2* w, const StepParams& P) {
   return true;
 }
 
+// The sound speed of cfl_substeps (fluid.rs:566-572).
+float cfl_sound_speed(const FluidConfig2Ffi& c) {
+  const float rho0 = rmaxf(c.rest_density, kEps);
+  return (c.gamma == 1.0f) ? std::sqrt(rmaxf(c.stiffness, 0.0f))
+                           : std::sqrt(c.gamma * rmaxf(c.stiffness, 0.0f) * rho0);
+}
+
 // cfl_substeps (fluid.rs:562-588); vmax from the current state.
 bool cfl_substeps(World2* w, float dt, uint32_t* out) {
   const FluidConfig2Ffi& c = w->cfg;
@@ -723,9 +740,7 @@ bool cfl_substeps(World2* w, float dt, uint32_t* out) {
   *out = 1;
   if (c.cfl <= 0.0f || mx <= 1) return true;
   const float h = rmaxf(c.smoothing_length, kEps);
-  const float rho0 = rmaxf(c.rest_density, kEps);
-  const float c0 = (c.gamma == 1.0f) ? std::sqrt(rmaxf(c.stiffness, 0.0f))
-                                     : std::sqrt(c.gamma * rmaxf(c.stiffness, 0.0f) * rho0);
+  const float c0 = cfl_sound_speed(c);
   float vmax = 0.0f;
   if (w->host_state_valid) {
     for (uint32_t i = 0; i < w->n; i++) {
@@ -1039,6 +1054,51 @@ bool run_substep_adaptive(World2* w, float dt) {
   return true;
 }
 
+// Up to `steps` steps of dt as one launch, for the worlds that take it
+// (enqueue_small_steps); *done = steps taken (0: not such a world). The world
+// is prepared but for its keys.
+bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
+  *done = 0;
+  const FluidConfig2Ffi& c = w->cfg;
+  if (w->profiling || c.adaptive_resolution || c.boundary_particles) return true;
+  SmallSteps ss;
+  ss.steps = std::min(steps, kSmallStepsPerLaunch);
+  if (c.cfl > 0.0f && c.max_substeps > 1) {
+    ss.max_substeps = c.max_substeps;
+    ss.c0 = cfl_sound_speed(c);
+    ss.cfl_h = c.cfl * rmaxf(c.smoothing_length, kEps);
+    ss.substeps = w->d.scalar + kSubstepWord;
+  }
+  bool applies = false;
+  const cudaError_t r = enqueue_small_steps(w->d, w->n, make_params(w, dt), ss, w->stream, &applies);
+  if (!cuda_ok(w, r, "whole-step launch")) return false;
+  if (!applies) return true;
+  if (ss.substeps)
+    w->substeps_pending = true;
+  else
+    w->substeps += ss.steps;
+  w->sid_perm_n = w->n;
+  w->host_state_valid = false;
+  w->dp_on_device = true;
+  w->keys_valid = true;
+  for (uint32_t k = 0; k < ss.steps; k++) w->time += dt;
+  *done = ss.steps;
+  return true;
+}
+
+// The substeps that whole-step launches counted on the device, into substeps.
+bool count_substeps(World2* w) {
+  if (!w->substeps_pending) return true;
+  unsigned int* word = w->d.scalar + kSubstepWord;
+  if (!cuda_ok(w, cudaMemcpyAsync(w->h_pinned + 9, word, 4, cudaMemcpyDeviceToHost, w->stream), "substeps") ||
+      !cuda_ok(w, cudaMemsetAsync(word, 0, 4, w->stream), "substeps") ||
+      !cuda_ok(w, cudaStreamSynchronize(w->stream), "sync"))
+    return false;
+  w->substeps += w->h_pinned[9];
+  w->substeps_pending = false;
+  return true;
+}
+
 // World2::step (world.rs:706-732) restricted to the fluid phase (1b).
 bool world_step(World2* w, float dt) {
   if (w->is_batch()) {
@@ -1072,6 +1132,22 @@ bool world_step(World2* w, float dt) {
   return true;
 }
 
+// `steps` steps of dt, several per launch where the world takes it.
+bool world_steps(World2* w, float dt, uint32_t steps) {
+  while (steps) {
+    uint32_t done = 0;
+    if (!w->is_batch() && w->cfg.enabled && !w->cfg.adaptive_resolution && w->n > 0 && w->n <= kMaxParticles2D &&
+        dt > 0.0f) {
+      if (!prepare(w, false) || !run_small(w, dt, steps, &done)) return false;
+    }
+    if (!done) {
+      if (!world_step(w, dt)) return false;
+      done = 1;
+    }
+    steps -= done;
+  }
+  return true;
+}
 
 // ---------------------------------------------------------------- bodies that react
 // FluidState2::step_fluid (fluid.rs:541-557) with the caller's bodies: the
@@ -1523,7 +1599,7 @@ void phieng_world_free(World2* w) {
 
 void phieng_world_step(World2* w, float dt) {
   if (!w || !std::isfinite(dt) || dt <= 0.0f) return;
-  world_step(w, std::min(dt, kMaxDt));
+  world_steps(w, std::min(dt, kMaxDt), 1);
 }
 
 void phieng_world_set_gravity(World2* w, float gx, float gy) {
@@ -1831,8 +1907,10 @@ uint32_t phieng_world_fluid_get(const World2* cw, float* out, uint32_t max) {
 }
 
 // ---------------------------------------------------------------- extension
-int32_t phieng_sph_status(const World2* w, PhiengSphStatus* out) {
-  if (!w || !out) return 0;
+int32_t phieng_sph_status(const World2* cw, PhiengSphStatus* out) {
+  if (!cw || !out) return 0;
+  World2* w = const_cast<World2*>(cw);
+  count_substeps(w);
   std::memset(out, 0, sizeof(*out));
   out->error = w->error;
   out->particles = w->n;
@@ -1863,10 +1941,7 @@ int32_t phieng_sph_set_particle_cap(World2* w, uint32_t cap) {
 int32_t phieng_sph_step_n(World2* w, float dt, uint32_t steps) {
   if (!w) return 0;
   if (!std::isfinite(dt) || dt <= 0.0f) return 1;
-  const float d = std::min(dt, kMaxDt);
-  for (uint32_t s = 0; s < steps; s++)
-    if (!world_step(w, d)) return 0;
-  return 1;
+  return world_steps(w, std::min(dt, kMaxDt), steps) ? 1 : 0;
 }
 
 int32_t phieng_sph_set_stream(World2* w, void* stream) {
