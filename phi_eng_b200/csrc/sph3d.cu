@@ -1049,8 +1049,9 @@ __device__ __forceinline__ void finish3(uint32_t id, bool writer, float4 pi, flo
 // Force + XSPH + integrate + walls (fluid3.rs:1040-1176); writes the new
 // state (id order), the next key and its bucket count. DEBUG: forces only.
 // FAST (tolerance mode; PLAIN, uniform mass): pair3_fast's arithmetic.
+constexpr uint32_t kForceThreads3 = 128;  // 128-thread blocks: 286 -> 280 us at 1M (256, 5-block cap: 329 us)
 template <bool MASS, bool DEBUG, bool PLAIN, bool FAST = false>
-__global__ void __launch_bounds__(256) k_force3(const float4* __restrict__ spos, const float4* __restrict__ svel,
+__global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restrict__ spos, const float4* __restrict__ svel,
                                                 const float2* __restrict__ sdq, const uint32_t* __restrict__ skey,
                                                 const uint32_t* __restrict__ sid, const float* __restrict__ smass,
                                                 uint32_t n, const uint32_t* __restrict__ start, StepParams3 P,
@@ -1075,7 +1076,7 @@ __global__ void __launch_bounds__(256) k_force3(const float4* __restrict__ spos,
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
     if (nmask[4 * (size_t)n + s] != 0u) {
       // the nine rows' masks and first slots, loaded up front (independent
-      // loads; none inside the divergent row advance below)
+      // loads; none inside the divergent loops below)
       uint32_t mk[9], bs[9];
 #pragma unroll
       for (int r = 0; r < 9; r++) {
@@ -1083,28 +1084,19 @@ __global__ void __launch_bounds__(256) k_force3(const float4* __restrict__ spos,
         bs[r] = __ldg(&start[row_base3(by, bz, r, g) + bx - 1]);
       }
       mk[4] &= ~(1u << (s - bs[4]));  // the particle's own bit: j != i
-      // one loop over the set bits of all rows (ascending slots, row by row),
-      // so a warp runs as many pair iterations as its busiest lane has
-      // neighbours
-      uint32_t cur = mk[0], base = bs[0];
-      int r = 0;
-      for (;;) {
-        while (cur == 0u && r < 8) {
-          r++;
+      // the set bits plane by plane (three rows each, ascending slots).
+      // One loop over all nine rows chose each next row from nine with selects,
+      // 55 of the ~100 instructions per neighbour; three loops run a few more
+      // iterations per warp, at ~12. 100^3 particles: tolerance mode 172 -> 128
+      // us, exact 327 -> 195 (the rows queued in shared memory: 189).
 #pragma unroll
-          for (int t = 1; t < 9; t++)
-            if (t == r) {
-              cur = mk[t];
-              base = bs[t];
-            }
+      for (int p = 0; p < 9; p += 3) {
+        for (RowWalk w(mk[p], bs[p], mk[p + 1], bs[p + 1], mk[p + 2], bs[p + 2]); w.more();) {
+          if constexpr (FAST)
+            pair3_fast(w.next(), pi, vi, rho_i, mq_i, spos, svel, sdq, P, f, sm);
+          else
+            pair3<MASS, PLAIN>(w.next(), pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, P, f, sm);
         }
-        if (cur == 0u) break;
-        const uint32_t j = base + (uint32_t)(__ffs((int)cur) - 1);
-        cur &= cur - 1u;
-        if constexpr (FAST)
-          pair3_fast(j, pi, vi, rho_i, mq_i, spos, svel, sdq, P, f, sm);
-        else
-          pair3<MASS, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, P, f, sm);
       }
     } else {
 #pragma unroll 1
@@ -1904,7 +1896,7 @@ void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
 
 void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t st) {
   const bool m = (P.flags & F_MASS) != 0;
-  const uint32_t g = cdiv(w->n, 128);  // 128-thread blocks: 286 -> 280 us at 1M (256, 5-block cap: 329 us)
+  const uint32_t g = cdiv(w->n, kForceThreads3);
   // XSPH on, artificial viscosity and cohesion off, h*h <= hk*hk: the
   // optional pair terms compiled out
   const bool plain = (P.flags & F_VISC) && !(P.flags & (F_AV | F_COHESION | F_WIDE_NB | F_TURB | F_GHOST));
@@ -1932,7 +1924,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
     return;
   }
 #define PHIENG_F3X(M, D, PL, FA)                                                                                    \
-  k_force3<M, D, PL, FA><<<g, 128, 0, st>>>(w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
+  k_force3<M, D, PL, FA><<<g, kForceThreads3, 0, st>>>(w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
                                             P, w->dbodies, w->nmask, w->pos, w->vel, w->key, w->count, dbg)
 #define PHIENG_F3(M, D, PL) PHIENG_F3X(M, D, PL, false)
   if (fast) {

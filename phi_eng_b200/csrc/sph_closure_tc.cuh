@@ -86,15 +86,9 @@ __global__ void __launch_bounds__(128, 6) k_closure_tc(
       const uint32_t own = nmask[n + s];
       uint32_t lo[3], hi[3];
       if (candidate_rows(k, start, g, lo, hi) && own != 0u) {
-        uint32_t m[3] = {nmask[s], own & ~(1u << (s - lo[1])), nmask[2 * (size_t)n + s]};
-#pragma unroll
-        for (int r = 0; r < 3; r++) {
-          uint32_t cur = m[r];
-          while (cur) {
-            const uint32_t j = lo[r] + (uint32_t)(__ffs((int)cur) - 1);
-            cur &= cur - 1u;
-            pair(__ldg(&spos[j]), __ldg(&svel[j]), __ldg(&sdq[j]), __ldg(&io.svp[j]), P, fx, fy, sx, sy, fa);
-          }
+        for (RowWalk w(nmask[s], lo[0], own & ~(1u << (s - lo[1])), lo[1], nmask[2 * (size_t)n + s], lo[2]); w.more();) {
+          const uint32_t j = w.next();
+          pair(__ldg(&spos[j]), __ldg(&svel[j]), __ldg(&sdq[j]), __ldg(&io.svp[j]), P, fx, fy, sx, sy, fa);
         }
       } else if (k != g.sentinel) {
         for_each_candidate(k, start, g, [&](int jj) {
@@ -169,15 +163,9 @@ __global__ void __launch_bounds__(256, 4) k_closure_fast(
     const uint32_t own = nmask[n + s];
     uint32_t lo[3], hi[3];
     if (candidate_rows(k, start, g, lo, hi) && own != 0u) {
-      uint32_t m[3] = {nmask[s], own & ~(1u << (s - lo[1])), nmask[2 * (size_t)n + s]};
-#pragma unroll
-      for (int r = 0; r < 3; r++) {
-        uint32_t cur = m[r];
-        while (cur) {
-          const uint32_t j = lo[r] + (uint32_t)(__ffs((int)cur) - 1);
-          cur &= cur - 1u;
-          pair(__ldg(&spos[j]), __ldg(&svel[j]), __ldg(&sdq[j]), __ldg(&io.svp[j]), P, fx, fy, sx, sy, fa);
-        }
+      for (RowWalk w(nmask[s], lo[0], own & ~(1u << (s - lo[1])), lo[1], nmask[2 * (size_t)n + s], lo[2]); w.more();) {
+        const uint32_t j = w.next();
+        pair(__ldg(&spos[j]), __ldg(&svel[j]), __ldg(&sdq[j]), __ldg(&io.svp[j]), P, fx, fy, sx, sy, fa);
       }
     } else if (k != g.sentinel) {
       for_each_candidate(k, start, g, [&](int jj) {

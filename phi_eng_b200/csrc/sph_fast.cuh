@@ -329,18 +329,7 @@ __global__ void __launch_bounds__(256) k_force_fast(
     const uint32_t m1 = own & ~(1u << (s - lo[1])), m2 = nmask[2 * (size_t)n + s];
     // the three rows' set bits as one loop (ascending slots, row by row)
     auto walk = [&](auto pair_at, uint32_t o0, uint32_t o1, uint32_t o2) {
-      uint32_t cur = nmask[s], row = 0, o = o0;
-      for (;;) {
-        while (cur == 0u && row < 2u) {
-          row++;
-          cur = row == 1u ? m1 : m2;
-          o = row == 1u ? o1 : o2;
-        }
-        if (cur == 0u) break;
-        const uint32_t j = o + (uint32_t)(__ffs((int)cur) - 1);
-        cur &= cur - 1u;
-        pair_at(j);
-      }
+      for (RowWalk w(nmask[s], o0, m1, o1, m2, o2); w.more();) pair_at(w.next());
     };
     if (STAGE && win.staged())
       walk([&](uint32_t j) { pair(wp[j], wv[j], wq[j], P, fx, fy, sx, sy); }, lo[0] - win.base[0],

@@ -527,7 +527,14 @@ __device__ __forceinline__ float neighbour_density_term(float d2, float m, const
   return __fmul_rn(m, poly6_nb<WIDE>(d2, P));
 }
 
-template <bool MASS, bool PHASE, bool BATCH, bool WIDE>
+// HEQ: h*h == hk*hk (F_HEQ), every config with h >= EPS: two candidates at a
+// time in packed f32 arithmetic. The pass is bound by instruction issue (~36
+// candidates per particle): 36.4 -> 33.4 us at 2^20 particles, 157 -> 144 for
+// 512 scenes (65 % issue and half the FMA pipe, which takes a packed operation in
+// two cycles; the 3D pass has too many moves between the two and got slower, 165
+// -> 174 us). Otherwise the general form, one
+// candidate at a time with poly6's range test.
+template <bool MASS, bool PHASE, bool BATCH, bool HEQ>
 __global__ void __launch_bounds__(256) k_density(const float2* __restrict__ spos, const uint32_t* __restrict__ skey,
                                                  const float* __restrict__ smass,
                                                  const uint8_t* __restrict__ sphase, uint32_t n,
@@ -547,37 +554,52 @@ __global__ void __launch_bounds__(256) k_density(const float2* __restrict__ spos
     const uint32_t bx = local & g.maskw, by = local >> g.log2w;
     const bool seam = !(bx >= 1u && bx < g.maskw);
     bool masks_ok = !seam;
+    if (HEQ && !seam) {
+      DensityPairs acc(P);
+      const f32x2 npi = pack2(-pi.x, -pi.y), mm = pack2(P.mass, P.mass);
 #pragma unroll
-    for (int oy = 0; oy < 3; oy++) {
-      const uint32_t row = g.base + (((by + (uint32_t)oy - 1u) & g.maskh) << g.log2w);
-      if (!seam) {
+      for (int oy = 0; oy < 3; oy++) {
+        const uint32_t row = g.base + (((by + (uint32_t)oy - 1u) & g.maskh) << g.log2w);
         const uint32_t rs = __ldg(&start[row + bx - 1]);
         const uint32_t re = __ldg(&start[row + bx + 2]);
-        uint32_t m = 0, bit = 1u;  // bit shifts out after 32 slots (then masks_ok is false)
-        for (uint32_t j = rs; j < re; j++) {
-          const float2 a = __ldg(&spos[j]);
-          const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y);
-          const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-          const bool nb = d2 < P.hg2;
-          const float w = neighbour_density_term<WIDE>(d2, MASS ? __ldg(&smass[j]) : P.mass, P);
-          rho = nb ? __fadd_rn(rho, w) : rho;
-          m |= nb ? bit : 0u;
-          bit <<= 1;
+        for (uint32_t j = rs; j < re; j += 2u) {
+          // spos has room past its last slot; a candidate past the row's end
+          // gets an infinite distance
+          const f32x2 da = add2(ldg2(&spos[j]), npi), db = add2(ldg2(&spos[j + 1u]), npi);
+          float ax, ay, bx2, by2;
+          unpack2(mul2(da, da), ax, ay);
+          unpack2(mul2(db, db), bx2, by2);
+          const float d2b = j + 1u < re ? __fadd_rn(bx2, by2) : __int_as_float(0x7f800000);
+          acc.add(__fadd_rn(ax, ay), d2b,
+                  MASS ? pack2(__ldg(&smass[j]), __ldg(&smass[j + 1u < re ? j + 1u : j])) : mm);
         }
-        mrow[oy] = m;
+        mrow[oy] = acc.mask((re - rs + 1u) & ~1u);
         if (re - rs > kMaskBits) masks_ok = false;
-      } else {
+      }
+      rho = acc.rho;
+    } else {
 #pragma unroll 1
-        for (int ox = -1; ox <= 1; ox++) {
+      for (int oy = 0; oy < 3; oy++) {
+        const uint32_t row = g.base + (((by + (uint32_t)oy - 1u) & g.maskh) << g.log2w);
+        uint32_t m = 0, bit = 1u;  // bit shifts out after 32 slots (then masks_ok is false)
+#pragma unroll 1
+        for (int ox = -1; ox <= (seam ? 1 : -1); ox++) {
+          // the row's slot range, on the seam bucket by bucket
           const uint32_t bb = row + ((bx + (uint32_t)ox) & g.maskw);
-          const uint32_t e = __ldg(&start[bb + 1]);
-          for (uint32_t j = __ldg(&start[bb]); j < e; j++) {
+          const uint32_t rs = __ldg(&start[bb]), re = __ldg(&start[bb + (seam ? 1u : 3u)]);
+          for (uint32_t j = rs; j < re; j++) {
             const float2 a = __ldg(&spos[j]);
             const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y);
             const float d2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
             rho = __fadd_rn(rho, density_term(d2, MASS ? __ldg(&smass[j]) : P.mass, P));
+            m |= d2 < P.hg2 ? bit : 0u;
+            bit <<= 1;
           }
+          if (re - rs > kMaskBits) masks_ok = false;
         }
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+          if (r == oy) mrow[r] = m;
       }
     }
     if (!masks_ok) mrow[1] = 0;  // K6 walks the candidates itself
@@ -729,19 +751,9 @@ __device__ __forceinline__ void neighbour_sums(uint32_t s, uint32_t k, uint32_t 
     // the particle's own bit (its slot in its own row, < 32 when the masks
     // are valid) is cleared: j != i (fluid.rs:947-950)
     const uint32_t own_nb = own & ~(1u << (s - rs1));
-    uint32_t cur = m0;
-    uint32_t row = 0, base = rs0;
-    for (;;) {
-      while (cur == 0u && row < 2) {
-        row++;
-        cur = row == 1 ? own_nb : m2;
-        base = row == 1 ? rs1 : rs2;
-      }
-      if (cur == 0u) break;
-      const uint32_t j = base + (uint32_t)(__ffs((int)cur) - 1);
-      cur &= cur - 1u;
-      pair_terms<MASS, FEAT, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, svp, P, fx, fy, sx, sy, fa);
-    }
+    for (RowWalk w(m0, rs0, own_nb, rs1, m2, rs2); w.more();)
+      pair_terms<MASS, FEAT, PLAIN>(w.next(), pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, svp, P, fx, fy, sx, sy,
+                                    fa);
   } else {
     for_each_candidate(k, start, g, [&](int jj) {
       const uint32_t j = (uint32_t)jj;
@@ -1370,7 +1382,7 @@ void enqueue_ghost_density(const FluidBufs& b, const StepParams& P, cudaStream_t
 void enqueue_density(const FluidBufs& b, uint32_t n, const StepParams& P, cudaStream_t st, float2* svp) {
   if (n == 0) return;
   const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0, bat = b.batch.ptab != nullptr;
-  const bool wide = (P.flags & F_WIDE_NB) != 0;  // h <= 0, which only a snapshot can carry
+  const bool heq = (P.flags & F_HEQ) != 0;  // all but h < EPS (for a batch: every scene)
   const uint32_t bs = b.block_density, g = cdiv(n, bs);
   // Tolerance mode with staging asked for: the exact density pass with its
   // neighbour rows staged in shared memory (same bits).
@@ -1384,12 +1396,12 @@ void enqueue_density(const FluidBufs& b, uint32_t n, const StepParams& P, cudaSt
                                                      svp);
     return;
   }
-#define PHIENG_DENSITY(M, PH, BT, WD)                                                                          \
-  k_density<M, PH, BT, WD><<<g, bs, 0, st>>>(b.spos, b.skey, b.smass, b.sphase, n, b.start, P, b.batch, b.sdq, \
+#define PHIENG_DENSITY(M, PH, BT, HE)                                                                          \
+  k_density<M, PH, BT, HE><<<g, bs, 0, st>>>(b.spos, b.skey, b.smass, b.sphase, n, b.start, P, b.batch, b.sdq, \
                                              b.spres, b.nmask, svp)
 #define PHIENG_DENSITY_W(M, PH, BT)       \
   do {                                    \
-    if (wide)                             \
+    if (heq)                              \
       PHIENG_DENSITY(M, PH, BT, true);    \
     else                                  \
       PHIENG_DENSITY(M, PH, BT, false);   \

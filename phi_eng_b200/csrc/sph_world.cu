@@ -274,7 +274,7 @@ bool ensure_capacity(World2* w, uint32_t need) {
   uint32_t c = std::max<uint32_t>(need, 1024);
   bool ok = dalloc(w, d.state, c) && dalloc(w, d.mass, c) && dalloc(w, d.phase, c) && dalloc(w, d.key, c) &&
             dalloc(w, d.tkey, c) && dalloc(w, d.tid, c) &&
-            dalloc(w, d.skey, c) && dalloc(w, d.sid, c) && dalloc(w, d.spos, c) && dalloc(w, d.svel, c) &&
+            dalloc(w, d.skey, c) && dalloc(w, d.sid, c) && dalloc(w, d.spos, (size_t)c + 1) && dalloc(w, d.svel, c) &&
             dalloc(w, d.smass, c) && dalloc(w, d.sphase, c) && dalloc(w, d.sdq, c) && dalloc(w, d.spres, c) &&
             dalloc(w, d.nmask, 3 * (size_t)c);
   if (ok && w->is_batch()) {
@@ -581,6 +581,7 @@ StepParams make_params_for(const FluidConfig2Ffi& c, float gx, float gy, bool ma
   if (!mass_uniform) f |= F_MASS;
   if (!phase_uniform) f |= F_PHASE;
   if (!(P.hg2 <= P.hk2)) f |= F_WIDE_NB;
+  if (P.hg2 == P.hk2) f |= F_HEQ;
   P.flags = f;
   P.nbodies = nbodies;
   P.body_first = body_first;
@@ -650,6 +651,7 @@ StepParams make_params(const World2* w, float dt) {
     if (!sc.phase_uniform) P.flags |= F_PHASE;
     const float hg = sc.cfg.smoothing_length, hk = rmaxf(hg, kEps);
     if (!(hg * hg <= hk * hk)) P.flags |= F_WIDE_NB;
+    if (hg * hg != hk * hk) P.flags &= ~F_HEQ;
   }
   if (w->precision == PHIENG_SPH_TOLERANCE) {
     // the tolerance-mode kernels take a batch only if every scene has the
