@@ -47,6 +47,18 @@ constexpr uint32_t kMaxParticles3D = 4096;  // MAX_PARTICLES_3D (fluid3.rs:28)
 inline uint32_t resample_bound3(uint32_t n) { return n + std::min(n, kMaxParticles3D / 2); }
 constexpr uint32_t kMaskBits3 = 32;
 
+// The density pass's quick distance test works on positions in units of h /
+// kCellUnits modulo 256, a byte per axis (cell_word): four cells of range, so
+// the bytes' differences are the displacements of everything in the 27 cells.
+// d . d of two such words, one subtraction and one four-byte dot product, is
+// off by: under one unit per axis for the two roundings down, 0.5 for the f32
+// product of positions below kQuickUnits, one for the borrow from the byte
+// below. A neighbour (64 units at most) is thus under 64 + |(1.5, 2.5, 2.5)| =
+// 67.84 units away, plus one for the borrow into the fourth byte: kQuickD2.
+constexpr float kCellUnits = 64.0f;
+constexpr float kQuickUnits = 2097152.0f;  // 2^21
+constexpr int kQuickD2 = 4604;
+
 struct GridPlan3 {
   int32_t cx0, cy0, cz0;
   uint32_t log2w, log2h, log2d;
@@ -125,6 +137,7 @@ struct StepParams3 {
   const float4* hullv;
   uint32_t* defer;
   uint32_t* dcount;
+  float cell_units;  // kCellUnits / smoothing_length (NaN where that is not positive)
 };
 
 // Static body: shape 0 sphere (a = radius), 1 box (a, b, c half extents),
@@ -162,6 +175,75 @@ __device__ __forceinline__ float poly6_3(float r2, const StepParams3& P) {
 // Candidate j's density term m_j * poly6(d2) when d2 < h*h (a neighbour), else +0
 __device__ __forceinline__ float contrib3(float d2, float m, const StepParams3& P) {
   return d2 < P.hg2 ? __fmul_rn(m, poly6_3(d2, P)) : 0.0f;
+}
+
+__device__ __forceinline__ uint32_t cell_word(float x, float y, float z, float units) {
+  const uint32_t a = (uint32_t)__float2int_rd(__fmul_rn(x, units)) & 255u;
+  const uint32_t b = (uint32_t)__float2int_rd(__fmul_rn(y, units)) & 255u;
+  const uint32_t c = (uint32_t)__float2int_rd(__fmul_rn(z, units)) & 255u;
+  return a | b << 8 | c << 16;
+}
+
+// Whether the quick test holds for a particle's neighbours.
+__device__ __forceinline__ bool quick_range(float x, float y, float z, float units) {
+  return fmaxf(fmaxf(fabsf(x), fabsf(y)), fabsf(z)) * units < kQuickUnits;  // false for NaN units
+}
+
+// hit(j) for the slots j of [rs, re), ascending, that can hold a neighbour of
+// the particle with word qi: those that pass the quick test, or all. hit
+// returns whether the slot does hold one; those of the first 64 slots are the
+// row's mask (bit t of mask[t / 32]: slot rs + t). sq is readable up to three
+// entries past any slot.
+template <class F>
+__device__ __forceinline__ void row_candidates3(uint32_t rs, uint32_t re, bool quick, uint32_t qi,
+                                                const uint32_t* __restrict__ sq, uint32_t (&mask)[2], F&& hit) {
+  mask[0] = mask[1] = 0u;
+  if (!quick) {
+#pragma unroll 1
+    for (uint32_t j = rs; j < re; j++) {
+      const bool nb = hit(j);
+      const uint32_t t = j - rs;
+      if (t < 32u) mask[0] |= (nb ? 1u : 0u) << t;
+      else if (t < 64u) mask[1] |= (nb ? 1u : 0u) << (t - 32u);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (uint32_t a = rs & ~3u; a < re; a += 32u) {  // 32 slots, their results shifted into a word from the right
+    const uint32_t end = min(a + 32u, re);
+    uint32_t bits = 0, j = a;
+    for (; j < end; j += 4u) {
+      const uint4 q = __ldg(reinterpret_cast<const uint4*>(sq + j));
+      auto test = [&](uint32_t w) {
+        const int d = (int)(w - qi);
+        bits = __funnelshift_l((uint32_t)__dp4a(d, d, -kQuickD2), bits, 1);  // negative: near
+      };
+      test(q.x);
+      test(q.y);
+      test(q.z);
+      test(q.w);
+    }
+    // slot a + t is bit (j - a) - 1 - t; slots before rs and from re on do not count
+    const uint32_t top = j - 1u;
+    bits &= 0xFFFFFFFFu << (j - end);
+    if (a < rs) bits &= 0xFFFFFFFFu >> (32u - (j - rs));
+    uint32_t found = 0;
+    while (bits) {
+      uint32_t f;
+      asm("bfind.u32 %0, %1;" : "=r"(f) : "r"(bits));
+      const uint32_t bit = 1u << f;
+      bits ^= bit;
+      found |= hit(top - f) ? bit : 0u;
+    }
+    // bit f is slot top - f, reversed bit b slot top - 31 + b
+    const int at = (int)(top - 31u - rs);  // its place in the row's mask: -31 .. 28 for the first word
+    const unsigned long long r = __brev(found);
+    if (at < 64) {
+      const unsigned long long m = at >= 0 ? r << at : r >> -at;
+      mask[0] |= (uint32_t)m;
+      mask[1] |= (uint32_t)(m >> 32);
+    }
+  }
 }
 
 // Particle vs static body (fluid3.rs:471-590) with the identity rotation.
@@ -555,14 +637,17 @@ struct Gather3 {
   const float4 *pos, *vel;
   const float* mass;
   const uint8_t* phase;
-  uint32_t *skey, *sid;
+  uint32_t *skey, *sid, *sq;
+  float units;
   float4 *spos, *svel;
   float* smass;     // null: uniform
   uint8_t* sphase;  // null: uniform
   __device__ __forceinline__ void operator()(uint32_t f, uint32_t k, uint32_t id) const {
     skey[f] = k;
     sid[f] = id;
-    spos[f] = pos[id];
+    const float4 p = pos[id];
+    spos[f] = p;
+    sq[f] = cell_word(p.x, p.y, p.z, units);
     svel[f] = vel[id];
     if (smass) smass[f] = mass[id];
     if (sphase) sphase[f] = phase[id];
@@ -587,13 +672,46 @@ __device__ __forceinline__ uint32_t row_base3(uint32_t by, uint32_t bz, int r, c
   return (((bz + oz) & g.maskd) << (g.log2w + g.log2h)) | (((by + oy) & g.maskh) << g.log2w);
 }
 
-// Density + EOS (fluid3.rs:639-658) in sorted order; per-row neighbour masks
-// (bit t of nmask[r * n + s]: slot row_start + t is a neighbour). A zero mask
-// for the particle's own row (r = 4) means no masks (seam or > 32 slots).
+// The candidates of row r for a particle in column bx: one slot range, the
+// three x cells' consecutive buckets; on the x seam two, the part before the
+// wrap and the part after it.
+struct RowRange3 {
+  uint32_t rs, re;    // first (or only) range
+  uint32_t rs2, re2;  // the second, on the seam
+};
+__device__ __forceinline__ bool on_seam3(uint32_t bx, const GridPlan3& g) { return !(bx >= 1u && bx < g.maskw); }
+__device__ __forceinline__ uint32_t row_first3(uint32_t row, uint32_t bx, const GridPlan3& g,
+                                               const uint32_t* __restrict__ start) {
+  return __ldg(&start[row + ((bx - 1u) & g.maskw)]);
+}
+__device__ __forceinline__ RowRange3 row_range3(uint32_t row, uint32_t bx, bool seam, const GridPlan3& g,
+                                                const uint32_t* __restrict__ start) {
+  RowRange3 q;
+  q.rs = row_first3(row, bx, g, start);
+  q.re = __ldg(&start[row + (seam ? g.maskw + 1u : bx + 2u)]);
+  q.rs2 = q.re2 = 0u;
+  if (seam) {
+    q.rs2 = __ldg(&start[row]);
+    q.re2 = __ldg(&start[row + ((bx + 1u) & g.maskw) + 1u]);
+  }
+  return q;
+}
+
+// Density + EOS (fluid3.rs:639-658) in sorted order; per-row neighbour masks:
+// bit t of nmask[r * n + s] is slot rs + t of row r (the particle itself
+// included). A row of 33 to 64 slots, as a compressed fluid has them, goes on
+// in nmask[(9 + r) * n + s] with slot rs + 32 + t, a row on the seam with slot
+// rs2 + t. nmask[18 * n + s]: bit r set where row r has that second word,
+// kNoMasks where the particle has no masks (a row of more than 64 slots, or of
+// more than 32 in a part on the seam): the force pass then walks its
+// candidates.
+constexpr uint32_t kMaskWords3 = 19;
+constexpr uint32_t kNoMasks = 0x80000000u;
 template <bool MASS, bool PHASE, bool WIDE>
 __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spos, const uint32_t* __restrict__ skey,
                                                   const float* __restrict__ smass, const uint8_t* __restrict__ sphase,
-                                                  uint32_t n, const uint32_t* __restrict__ start, StepParams3 P,
+                                                  uint32_t n, const uint32_t* __restrict__ start,
+                                                  const uint32_t* __restrict__ sq, StepParams3 P,
                                                   float2* __restrict__ sdq, float* __restrict__ spres,
                                                   uint32_t* __restrict__ nmask) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -601,61 +719,55 @@ __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spo
   const uint32_t k = skey[s];
   const float4 pi = spos[s];
   float rho = 0.0f;
+  uint32_t flags = kNoMasks;
   const GridPlan3& g = P.grid;
   if (k != g.sentinel) {
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
-    if (bx >= 1u && bx < g.maskw) {
-      // the three x cells of each row are consecutive buckets: one slot range
-      bool masked = true;
-      uint32_t m_own = 0;
+    const bool seam = on_seam3(bx, g);
+    flags = 0u;
+    const bool quick = quick_range(pi.x, pi.y, pi.z, P.cell_units);
+    const uint32_t qi = sq[s];
+    auto hit = [&](uint32_t j) {
+      const float4 a = __ldg(&spos[j]);
+      const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
+      const float d2 = dot3(dx, dy, dz, dx, dy, dz);
+      const bool nb = d2 < P.hg2;
+      const float w = __fmul_rn(MASS ? __ldg(&smass[j]) : P.mass, poly6_nb<WIDE>(d2, P));
+      rho = nb ? __fadd_rn(rho, w) : rho;
+      return nb;
+    };
+    uint32_t m[2];
+    if (!seam) {
       // the rows' slot ranges, loaded up front
       uint32_t rsa[9], rea[9];
 #pragma unroll
       for (int r = 0; r < 9; r++) {
         const uint32_t row = row_base3(by, bz, r, g);
-        rsa[r] = __ldg(&start[row + bx - 1]);
-        rea[r] = __ldg(&start[row + bx + 2]);
+        rsa[r] = __ldg(&start[row + bx - 1u]);
+        rea[r] = __ldg(&start[row + bx + 2u]);
       }
 #pragma unroll
       for (int r = 0; r < 9; r++) {
-        const uint32_t rs = rsa[r], re = rea[r];
-        uint32_t m = 0, bit = 1u;  // bit shifts out after 32 slots (then masked is false)
-        for (uint32_t j = rs; j < re; j++) {
-          const float4 a = __ldg(&spos[j]);
-          const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
-          const float d2 = dot3(dx, dy, dz, dx, dy, dz);
-          const bool nb = d2 < P.hg2;
-          const float w = __fmul_rn(MASS ? __ldg(&smass[j]) : P.mass, poly6_nb<WIDE>(d2, P));
-          rho = nb ? __fadd_rn(rho, w) : rho;
-          m |= nb ? bit : 0u;
-          bit <<= 1;
+        const uint32_t len = rea[r] - rsa[r];
+        row_candidates3(rsa[r], rea[r], quick, qi, sq, m, hit);
+        nmask[(size_t)r * n + s] = m[0];
+        if (len > kMaskBits3) {
+          nmask[(size_t)(9 + r) * n + s] = m[1];
+          flags |= len > 2u * kMaskBits3 ? kNoMasks : 1u << r;
         }
-        if (re - rs > kMaskBits3) masked = false;
-        if (r == 4) m_own = m;
-        else nmask[(size_t)r * n + s] = m;
       }
-      nmask[4 * (size_t)n + s] = masked ? m_own : 0u;
     } else {
-      // seam column: the x cells wrap, visit bucket by bucket
 #pragma unroll 1
-      for (int r = 0; r < 9; r++) {
-        const uint32_t row = row_base3(by, bz, r, g);
-#pragma unroll 1
-        for (int ox = -1; ox <= 1; ox++) {
-          const uint32_t bb = row | ((bx + (uint32_t)ox) & g.maskw);
-          const uint32_t e = __ldg(&start[bb + 1]);
-          for (uint32_t j = __ldg(&start[bb]); j < e; j++) {
-            const float4 a = __ldg(&spos[j]);
-            const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
-            rho = __fadd_rn(rho, contrib3(dot3(dx, dy, dz, dx, dy, dz), MASS ? __ldg(&smass[j]) : P.mass, P));
-          }
-        }
+      for (uint32_t t = 0; t < 18u; t++) {  // row t / 2's part before the wrap, then the one after it
+        const RowRange3 q = row_range3(row_base3(by, bz, (int)(t / 2u), g), bx, true, g, start);
+        const uint32_t rs = t & 1u ? q.rs2 : q.rs, re = t & 1u ? q.re2 : q.re;
+        row_candidates3(rs, re, quick, qi, sq, m, hit);
+        nmask[(size_t)(t / 2u + (t & 1u ? 9u : 0u)) * n + s] = m[0];
+        flags |= re - rs > kMaskBits3 ? kNoMasks : 1u << t / 2u;
       }
-      nmask[4 * (size_t)n + s] = 0u;
     }
-  } else {
-    nmask[4 * (size_t)n + s] = 0u;
   }
+  nmask[18 * (size_t)n + s] = flags;
   float dens = rho;
   if (dens < 0.0f) dens = 0.0f;
   if (dens > P.rho_cap) dens = P.rho_cap;
@@ -1074,23 +1186,39 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
   const GridPlan3& g = P.grid;
   if (k != g.sentinel) {
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
-    if (nmask[4 * (size_t)n + s] != 0u) {
+    const uint32_t flags = nmask[18 * (size_t)n + s];
+    if (!(flags & kNoMasks)) {
       // the nine rows' masks and first slots, loaded up front (independent
       // loads; none inside the divergent loops below)
-      uint32_t mk[9], bs[9];
+      uint32_t mk[18], bs[18];
 #pragma unroll
       for (int r = 0; r < 9; r++) {
         mk[r] = nmask[(size_t)r * n + s];
-        bs[r] = __ldg(&start[row_base3(by, bz, r, g) + bx - 1]);
+        bs[r] = row_first3(row_base3(by, bz, r, g), bx, g, start);
       }
-      mk[4] &= ~(1u << (s - bs[4]));  // the particle's own bit: j != i
-      // the set bits plane by plane (three rows each, ascending slots).
+      int words = 9;
+      if (__any_sync(__activemask(), flags != 0u)) {
+        // second words in the warp: all its lanes take two words per row
+#pragma unroll
+        for (int r = 8; r >= 0; r--) {
+          mk[2 * r + 1] = (flags >> r & 1u) ? nmask[(size_t)(9 + r) * n + s] : 0u;
+          bs[2 * r + 1] = on_seam3(bx, g) ? __ldg(&start[row_base3(by, bz, r, g)]) : bs[r] + kMaskBits3;
+          mk[2 * r] = mk[r];
+          bs[2 * r] = bs[r];
+        }
+        words = 18;
+        if (s - bs[8] < kMaskBits3) mk[8] &= ~(1u << (s - bs[8]));  // the particle's own bit: j != i
+        else mk[9] &= ~(1u << (s - bs[9]));
+      } else {
+        mk[4] &= ~(1u << (s - bs[4]));
+      }
+      // the set bits three words at a time (ascending slots), as a rule a plane.
       // One loop over all nine rows chose each next row from nine with selects,
       // 55 of the ~100 instructions per neighbour; three loops run a few more
       // iterations per warp, at ~12. 100^3 particles: tolerance mode 172 -> 128
       // us, exact 327 -> 195 (the rows queued in shared memory: 189).
-#pragma unroll
-      for (int p = 0; p < 9; p += 3) {
+#pragma unroll 1
+      for (int p = 0; p < words; p += 3) {
         for (RowWalk w(mk[p], bs[p], mk[p + 1], bs[p + 1], mk[p + 2], bs[p + 2]); w.more();) {
           if constexpr (FAST)
             pair3_fast(w.next(), pi, vi, rho_i, mq_i, spos, svel, sdq, P, f, sm);
@@ -1353,6 +1481,7 @@ struct World3 {
   float *mass = nullptr, *smass = nullptr, *spres = nullptr, *tmp = nullptr;
   uint8_t *phase = nullptr, *sphase = nullptr;
   uint32_t *key = nullptr, *tkey = nullptr, *tid = nullptr, *skey = nullptr, *sid = nullptr, *nmask = nullptr;
+  uint32_t* sq = nullptr;  // sorted cell_word
   float2* sdq = nullptr;
   uint32_t *count = nullptr, *start = nullptr, *tilesum = nullptr, *scalar = nullptr;
   unsigned long long* tstate = nullptr;  // single-pass scan tile states
@@ -1410,7 +1539,7 @@ void release_graph3(World3* w) {
 void free_particles3(World3* w) {
   dfree3(w->pos), dfree3(w->vel), dfree3(w->spos), dfree3(w->svel), dfree3(w->mass), dfree3(w->smass);
   dfree3(w->spres), dfree3(w->tmp), dfree3(w->phase), dfree3(w->sphase), dfree3(w->key), dfree3(w->tkey);
-  dfree3(w->tid), dfree3(w->skey), dfree3(w->sid), dfree3(w->nmask), dfree3(w->sdq);
+  dfree3(w->tid), dfree3(w->skey), dfree3(w->sid), dfree3(w->nmask), dfree3(w->sdq), dfree3(w->sq);
   w->dcap = 0;
 }
 
@@ -1442,7 +1571,7 @@ bool ensure_capacity3(World3* w, uint32_t need) {
                   dalloc3(w, w->mass, c) && dalloc3(w, w->smass, c) && dalloc3(w, w->spres, c) &&
                   dalloc3(w, w->tmp, 2 * (size_t)c) && dalloc3(w, w->phase, c) && dalloc3(w, w->sphase, c) &&
                   dalloc3(w, w->key, c) && dalloc3(w, w->tkey, c) && dalloc3(w, w->tid, c) && dalloc3(w, w->skey, c) &&
-                  dalloc3(w, w->sid, c) && dalloc3(w, w->nmask, 9 * (size_t)c) && dalloc3(w, w->sdq, c);
+                  dalloc3(w, w->sid, c) && dalloc3(w, w->nmask, kMaskWords3 * (size_t)c) && dalloc3(w, w->sdq, c) && dalloc3(w, w->sq, (size_t)c + 4);
   if (!ok) {
     free_particles3(w);
     return false;
@@ -1820,6 +1949,7 @@ StepParams3 make_params3(const World3* w, float dt) {
   P.flags = f;
   P.nbodies = (uint32_t)w->bodies.size();
   P.uniform_phase = w->phase_value;
+  P.cell_units = c.smoothing_length > 0.0f ? kCellUnits / c.smoothing_length : NAN;
   if (w->precision == PHIENG_SPH_TOLERANCE) P.flags |= F_FAST;
   return P;
 }
@@ -1830,7 +1960,7 @@ StepParams3 make_params3(const World3* w, float dt) {
 void enqueue_sorted3(World3* w, const StepParams3& P, uint32_t* counts, bool by_slot, uint32_t* clear,
                      cudaStream_t st) {
   const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
-  const Gather3 ga{w->pos, w->vel, w->mass, w->phase, w->skey, w->sid, w->spos, w->svel, m ? w->smass : nullptr,
+  const Gather3 ga{w->pos, w->vel, w->mass, w->phase, w->skey, w->sid, w->sq, P.cell_units, w->spos, w->svel, m ? w->smass : nullptr,
                    ph ? w->sphase : nullptr};
   const uint32_t nkeys = P.grid.sentinel + 1;
   if (small_sort_applies(w->n, nkeys)) {
@@ -1864,7 +1994,7 @@ void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
   if (w->n <= kRowsMax3) {
 #define PHIENG_D3C(M, PH, WD)                                                                                \
   k_density3_rows<M, PH, WD><<<cdiv(w->n, 32), 288, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, \
-                                                             w->start, P, w->sdq, w->spres, w->nmask)
+                                                             w->start, w->sq, P, w->sdq, w->spres, w->nmask)
 #define PHIENG_D3G(M, PH)                       \
   do {                                          \
     if (wide) PHIENG_D3C(M, PH, true);          \
@@ -1881,10 +2011,10 @@ void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
 #define PHIENG_D3(M, PH)                                                                                     \
   do {                                                                                                       \
     if (wide)                                                                                                \
-      k_density3<M, PH, true><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, P,  \
+      k_density3<M, PH, true><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P,  \
                                                  w->sdq, w->spres, w->nmask);                                \
     else                                                                                                     \
-      k_density3<M, PH, false><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, P, \
+      k_density3<M, PH, false><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P, \
                                                   w->sdq, w->spres, w->nmask);                               \
   } while (0)
   if (m && ph) PHIENG_D3(true, true);
@@ -1902,7 +2032,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
   const bool plain = (P.flags & F_VISC) && !(P.flags & (F_AV | F_COHESION | F_WIDE_NB | F_TURB | F_GHOST));
   // tolerance mode: the plain pass with uniform mass runs pair3_fast
   const bool fast = plain && !m && (P.flags & F_FAST);
-  if (w->n <= kCoopMax3) {
+  if (w->n <= (fast ? kCoopMaxFast3 : kCoopMax3)) {
 #define PHIENG_F3G(M, D, PL, FA)                                                                           \
   k_force3_coop<M, D, PL, FA><<<cdiv(w->n, kCoopThreads / kCoopLanes), kCoopThreads, 0, st>>>(             \
       w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, P, w->dbodies, w->nmask, w->pos, \

@@ -17,13 +17,13 @@ constexpr uint32_t kCoopThreads = 256;  // block of the force pass
 // particles (16.3 and 15.5 us per step, 29.1 and 28.4), and 32 waste lanes on
 // more (8,000 particles: 32.6 against 36.1).
 constexpr int kCoopLanes = 8;
-// Largest particle sets that take these passes. Step of a 32^3 block, eight
-// lanes and rows against one thread per particle: 54 against 81 us (exact), 53
-// against 65 (tolerance); of 40^3: 74 / 90 and 74 / 76; of 50^3: 117 / 117 and
-// 117 / 101. The density pass alone turns earlier: 12.3 against 16.4 us at
-// 24^3, 18.4 / 16.4 at 32^3, 26.6 / 22.6 at 40^3.
-constexpr uint32_t kRowsMax3 = 24576;
-constexpr uint32_t kCoopMax3 = 65536;
+// Largest particle sets that take these passes. Steps of 28^3, 36^3 and 40^3
+// particles, density by rows against one thread per particle: 38.2 / 46.5,
+// 46.7 / 49.3, 53.4 / 52.1 us (tolerance mode). Force by eight lanes against one
+// thread, rows in both: exact 36.3 / 47.4, 52.2 / 56.3, 63.3 / 62.0; tolerance
+// mode 36.6 / 38.2, 51.9 / 46.7, 63.8 / 53.4.
+constexpr uint32_t kRowsMax3 = 49152;
+constexpr uint32_t kCoopMax3 = 49152, kCoopMaxFast3 = 24576;
 
 // Density + EOS. Warp r of a block walks row r of the block's 32 particles,
 // one per lane, and keeps the neighbours' terms; warp 0 then sums each
@@ -34,68 +34,60 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
                                                        const uint32_t* __restrict__ skey,
                                                        const float* __restrict__ smass,
                                                        const uint8_t* __restrict__ sphase, uint32_t n,
-                                                       const uint32_t* __restrict__ start, StepParams3 P,
+                                                       const uint32_t* __restrict__ start,
+                                                       const uint32_t* __restrict__ sq, StepParams3 P,
                                                        float2* __restrict__ sdq, float* __restrict__ spres,
                                                        uint32_t* __restrict__ nmask) {
   __shared__ float terms[9][kRowTerms][32];
-  __shared__ uint32_t row_cnt[9][32];  // neighbours of the row; top bit: the row has no mask
-  __shared__ uint32_t own_mask[32];
+  __shared__ uint32_t row_cnt[9][32];  // neighbours of the row; bits 30, 31: it has a second word, no mask
   const uint32_t p = threadIdx.x & 31u, r = threadIdx.x >> 5;
   const uint32_t s = blockIdx.x * 32u + p;
   const bool active = s < n;
   const GridPlan3& g = P.grid;
   const uint32_t k = active ? skey[s] : g.sentinel;
   const float4 pi = spos[active ? s : 0u];
-  uint32_t cnt = 0, m = 0;
-  bool masked = true;
+  uint32_t cnt = 0, m[2] = {0u, 0u}, kind = 2u;
   if (k != g.sentinel) {
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
     const uint32_t row = row_base3(by, bz, (int)r, g);
-    uint32_t bit = 1u;  // shifts out after 32 slots (then the row has no mask)
-    auto span = [&](uint32_t rs, uint32_t re) {
-      for (uint32_t j = rs; j < re; j += 8u) {  // eight candidates in flight
-        float4 a[8];
-#pragma unroll
-        for (uint32_t q = 0; q < 8; q++) a[q] = __ldg(&spos[min(j + q, re - 1u)]);
-#pragma unroll
-        for (uint32_t q = 0; q < 8; q++) {
-          const float dx = __fsub_rn(a[q].x, pi.x), dy = __fsub_rn(a[q].y, pi.y), dz = __fsub_rn(a[q].z, pi.z);
-          const float d2 = dot3(dx, dy, dz, dx, dy, dz);
-          if (j + q < re && d2 < P.hg2) {
-            if (cnt < kRowTerms)
-              terms[r][cnt][p] = __fmul_rn(MASS ? __ldg(&smass[j + q]) : P.mass, poly6_nb<WIDE>(d2, P));
-            cnt++;
-            m |= bit;
-          }
-          bit <<= 1;
-        }
-      }
-    };
-    if (bx >= 1u && bx < g.maskw) {
-      const uint32_t rs = __ldg(&start[row + bx - 1]), re = __ldg(&start[row + bx + 2]);
-      span(rs, re);
-      masked = re - rs <= kMaskBits3;
-    } else {  // seam column: the x cells wrap
+    const bool quick = quick_range(pi.x, pi.y, pi.z, P.cell_units);
+    const uint32_t qi = sq[s];
+    const bool seam = on_seam3(bx, g);
+    const RowRange3 q = row_range3(row, bx, seam, g, start);
 #pragma unroll 1
-      for (int ox = -1; ox <= 1; ox++) {
-        const uint32_t b = row | ((bx + (uint32_t)ox) & g.maskw);
-        span(__ldg(&start[b]), __ldg(&start[b + 1]));
-      }
-      masked = false;
+    for (uint32_t part = 0; part < (seam ? 2u : 1u); part++) {
+      uint32_t found[2];
+      const uint32_t rs = part ? q.rs2 : q.rs, re = part ? q.re2 : q.re;
+      row_candidates3(rs, re, quick, qi, sq, found, [&](uint32_t j) {
+        const float4 a = __ldg(&spos[j]);
+        const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
+        const float d2 = dot3(dx, dy, dz, dx, dy, dz);
+        const bool nb = d2 < P.hg2;
+        // kept where the next neighbour overwrites it unless it counts (a branch costs more)
+        if (cnt < kRowTerms) terms[r][cnt][p] = __fmul_rn(MASS ? __ldg(&smass[j]) : P.mass, poly6_nb<WIDE>(d2, P));
+        cnt += nb ? 1u : 0u;
+        return nb;
+      });
+      if (part) m[1] = found[0];
+      else m[0] = found[0], m[1] = found[1];
     }
+    const uint32_t len = max(q.re - q.rs, q.re2 - q.rs2);
+    kind = len > (seam ? 1u : 2u) * kMaskBits3 ? 2u : seam || len > kMaskBits3 ? 1u : 0u;
   }
-  row_cnt[r][p] = cnt | (masked ? 0u : 0x80000000u);
-  if (r == 4u) own_mask[p] = m;
-  else if (active) nmask[(size_t)r * n + s] = m;
+  row_cnt[r][p] = cnt | kind << 30;
+  if (active) {
+    nmask[(size_t)r * n + s] = m[0];
+    if (kind == 1u) nmask[(size_t)(9u + r) * n + s] = m[1];
+  }
   __syncthreads();
   if (r != 0u || !active) return;
   float rho = 0.0f;
   bool fits = true;
-  masked = k != g.sentinel;
+  uint32_t flags = 0u;
 #pragma unroll
   for (int q = 0; q < 9; q++) {
-    const uint32_t c = row_cnt[q][p] & 0x7FFFFFFFu;
-    masked = masked && (row_cnt[q][p] >> 31) == 0u;
+    const uint32_t c = row_cnt[q][p] & 0x3FFFFFFFu, kd = row_cnt[q][p] >> 30;
+    flags |= kd == 0u ? 0u : kd == 1u ? 1u << q : kNoMasks;
     fits = fits && c <= kRowTerms;
     for (uint32_t i = 0; i < min(c, kRowTerms); i += 4) {
 #pragma unroll
@@ -119,7 +111,7 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
       }
     }
   }
-  nmask[4 * (size_t)n + s] = masked ? own_mask[p] : 0u;
+  nmask[18 * (size_t)n + s] = flags;
   float dens = rho;
   if (dens < 0.0f) dens = 0.0f;
   if (dens > P.rho_cap) dens = P.rho_cap;
@@ -166,20 +158,30 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
   const GridPlan3& g = P.grid;
   const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
   const bool live = active && k != g.sentinel;
-  bool listed = live && nmask[4 * (size_t)n + s] != 0u;
-  // the set bits of the nine row masks as one list of slots in visit order:
+  const uint32_t flags = live ? nmask[18 * (size_t)n + s] : kNoMasks;
+  bool listed = !(flags & kNoMasks);
+  // the set bits of the nine rows' masks as one list of slots in visit order:
   // lane l expands row l, the first row 8 as well
-  uint32_t mk = 0u, bs = 0u, mk8 = 0u, bs8 = 0u;
+  uint32_t mk[2] = {0u, 0u}, bs[2] = {0u, 0u}, mk8[2] = {0u, 0u}, bs8[2] = {0u, 0u};
   if (listed) {
-    mk = nmask[(size_t)l * n + s];
-    bs = __ldg(&start[row_base3(by, bz, (int)l, g) + bx - 1]);
-    if (l == 4u) mk &= ~(1u << (s - bs));  // the particle's own bit: j != i (fluid3.rs:1041)
-    if (l == 0u) {
-      mk8 = nmask[8 * (size_t)n + s];
-      bs8 = __ldg(&start[row_base3(by, bz, 8, g) + bx - 1]);
+    auto row_masks = [&](uint32_t r, uint32_t (&m)[2], uint32_t (&b)[2]) {
+      const uint32_t row = row_base3(by, bz, (int)r, g);
+      m[0] = nmask[(size_t)r * n + s];
+      b[0] = row_first3(row, bx, g, start);
+      if (flags >> r & 1u) {
+        m[1] = nmask[(size_t)(9u + r) * n + s];
+        b[1] = on_seam3(bx, g) ? __ldg(&start[row]) : b[0] + kMaskBits3;
+      }
+    };
+    row_masks(l, mk, bs);
+    if (l == 4u) {  // the particle's own bit: j != i (fluid3.rs:1041)
+      if (s - bs[0] < kMaskBits3) mk[0] &= ~(1u << (s - bs[0]));
+      else mk[1] &= ~(1u << (s - bs[1]));
     }
+    if (l == 0u) row_masks(8u, mk8, bs8);
   }
-  uint32_t off = (uint32_t)__popc(mk);
+  const uint32_t own = (uint32_t)(__popc(mk[0]) + __popc(mk[1]));
+  uint32_t off = own;
 #pragma unroll
   for (int o = 1; o < G; o <<= 1) {
     const uint32_t y = __shfl_up_sync(kAll, off, o, G);
@@ -187,13 +189,17 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
   }
   uint32_t cnt = __shfl_sync(kAll, off, 7, G);
   const uint32_t off8 = cnt;
-  cnt += (uint32_t)__popc(__shfl_sync(kAll, mk8, 0, G));
+  cnt += (uint32_t)__shfl_sync(kAll, __popc(mk8[0]) + __popc(mk8[1]), 0, G);
   if (cnt > kCoopPairs) listed = false;
   if (listed) {
-    off -= (uint32_t)__popc(mk);
-    for (; mk; mk &= mk - 1u) list[off++] = bs + (uint32_t)(__ffs((int)mk) - 1);
+    off -= own;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      for (; mk[h]; mk[h] &= mk[h] - 1u) list[off++] = bs[h] + (uint32_t)(__ffs((int)mk[h]) - 1);
     off = off8;
-    for (; mk8; mk8 &= mk8 - 1u) list[off++] = bs8 + (uint32_t)(__ffs((int)mk8) - 1);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      for (; mk8[h]; mk8[h] &= mk8[h] - 1u) list[off++] = bs8[h] + (uint32_t)(__ffs((int)mk8[h]) - 1);
   }
   __syncwarp();
   float acc = 0.0f;  // lanes 0..2: the force sum's x, y, z; 3..5: the XSPH sum's
@@ -254,7 +260,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
   }
   const bool walk = live && !listed;
   if (__any_sync(kAll, walk)) {
-    // no masks (x seam, or a row longer than 32 slots) or a full list: the
+    // no masks (a row too long for them) or a full list: the
     // candidates, bucket by bucket
 #pragma unroll 1
     for (int t = 0; t < 27; t++) {

@@ -1,6 +1,6 @@
 """3D passes over the sizes at which their launch shape changes (one-launch
-sort up to 8,192 particles, a thread per candidate row up to 24,576, eight
-lanes per particle up to 65,536), against the oracle bit for bit, and a
+sort up to 8,192 particles; a thread per candidate row and eight lanes per
+particle up to 49,152, in the tolerance mode 24,576), against the oracle bit for bit, and a
 block alone against the same block beside a distant one large enough to send
 the world through the one-thread passes: the same bits in both modes."""
 import numpy as np
@@ -12,7 +12,7 @@ from phi_eng_b200._abi import default_config
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 31, 33, 1023, 1025, 8191, 8192, 8193, 24576, 24577, 65536, 65537]
+SIZES = [1, 2, 31, 33, 1023, 1025, 8191, 8192, 8193, 24577, 49152, 49153]
 
 
 def block(n, spacing=0.25, seed=3, order="zyx"):
@@ -100,11 +100,15 @@ def test_steps_match_the_oracle(n, terms):
     np.testing.assert_array_equal(w.fluid.particles, o.state())
 
 
-@pytest.mark.parametrize("spacing", [0.25, 0.12, 0.06])
-def test_dense_blocks_match_the_oracle(spacing):
-    """Rows past the 32 slots of a mask (0.12) and neighbour lists past their
-    buffers (0.06: ~2,400 neighbours)."""
-    q = block(3000, spacing)
+@pytest.mark.parametrize("spacing", [0.25, 0.22, 0.2, 0.17, 0.12, 0.06])
+@pytest.mark.parametrize("n", [3000, 50000])
+def test_dense_blocks_match_the_oracle(spacing, n):
+    """Rows past the 32 slots of a mask word (0.22, 0.2), past its two words
+    (0.17, 0.12) and neighbour lists past their buffers (0.06: ~2,400
+    neighbours), in the passes of small and of large sets."""
+    if spacing < 0.1 and n > 3000:
+        pytest.skip("2,400 neighbours of 50,000 particles: minutes on the oracle")
+    q = block(n, spacing)
     cfg = default_config()
     w, o = gpu_world(q, cfg), oracle_world(q, cfg)
     w.step(1 / 60)
@@ -113,13 +117,37 @@ def test_dense_blocks_match_the_oracle(spacing):
 
 
 @pytest.mark.parametrize("mode", [_abi.EXACT, _abi.TOLERANCE])
-@pytest.mark.parametrize("n", [700, 9000, 30000])
-def test_block_beside_a_distant_one(n, mode):
-    a = block(n)
-    far = block(66000)
+@pytest.mark.parametrize("n, spacing", [(700, 0.25), (9000, 0.25), (30000, 0.25), (9000, 0.2), (30000, 0.15)])
+def test_block_beside_a_distant_one(n, spacing, mode):
+    a = block(n, spacing)
+    far = block(50000)
     far[:, 0] += 100.0
     w1, w2 = gpu_world(a, default_config(), mode=mode), gpu_world(np.concatenate([a, far]), default_config(), mode=mode)
     for _ in range(3):
         w1.step(1 / 60)
         w2.step(1 / 60)
     np.testing.assert_array_equal(w1.fluid.particles, w2.fluid.particles[:n])
+
+
+@pytest.mark.parametrize("n, spacing", [(2000, 0.25), (2000, 0.17), (52000, 0.25), (52000, 0.2)])
+@pytest.mark.parametrize("shift", [0.0, 1.7, -3.3, 1e5])
+def test_blocks_across_the_seam_match_the_oracle(n, spacing, shift):
+    """The bucket grid is planned for the first positions; the block is then
+    moved so that its x cells wrap (and, at 1e5, so far out that the quick
+    distance test does not apply)."""
+    q = block(n, spacing)
+    w, o = gpu_world(q, default_config()), oracle_world(q, default_config())
+    w.step(1 / 60)  # plans the grid
+    o.step(1 / 60, JACOBI)
+    s = o.state()
+    s[:, 3] = shift * 60 * 20 if abs(shift) > 100 else shift * 60
+    cfg = default_config()
+    cfg.max_velocity = 1e9
+    for x in (w.fluid, o):
+        x.set_config(cfg)
+    o.set_state(s)
+    w2 = gpu_world(s, cfg)  # the same state, its grid planned before it moves
+    for _ in range(3):
+        w2.step(1 / 60)
+        o.step(1 / 60, JACOBI)
+    np.testing.assert_array_equal(w2.fluid.particles, o.state())
