@@ -529,6 +529,17 @@ __device__ __forceinline__ void st_t16(unsigned char* m, uint32_t row, uint32_t 
   *reinterpret_cast<uint16_t*>(m + tc::kmajor_offset(row, col, 128)) = (uint16_t)v;
 }
 
+// Rows row, row + 1 (row even) of the column pair that this lane and its
+// neighbour hold: p = this sample's two values. The lanes trade halves, so that
+// each stores one 4-byte pair of samples instead of two 2-byte values (the
+// transposed stores are most of the pass's shared-memory traffic).
+__device__ __forceinline__ void st_t16_rows(unsigned char* m, uint32_t row, uint32_t sample, uint32_t p) {
+  const uint32_t q = __shfl_xor_sync(0xFFFFFFFFu, p, 1);
+  const uint32_t odd = sample & 1u;
+  *reinterpret_cast<uint32_t*>(m + tc::kmajor_offset(row + odd, sample & ~1u, 128)) =
+      __byte_perm(p, q, odd ? 0x3276 : 0x5410);
+}
+
 __global__ void __launch_bounds__(kTrainThreads, 1)
     k_mlp_train_tc(const float* __restrict__ x, const float* __restrict__ tg, uint32_t npairs, uint32_t k0,
                    uint32_t total, uint32_t rounds, uint64_t seed, const uint32_t* __restrict__ iter_ptr, MlpDev mlp,
@@ -537,10 +548,12 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const __nv_bfloat16* img = reinterpret_cast<const __nv_bfloat16*>(mlp.frag);
   const __half* himg = reinterpret_cast<const __half*>(mlp.frag);
+#pragma unroll
   for (uint32_t i = tid; i < 64 * 16; i += kTrainThreads) {
     const uint32_t o = i >> 4, k = i & 15;
     *reinterpret_cast<__nv_bfloat16*>(tsm + kTrW1 + tc::kmajor_offset(o, k, 16)) = img[frag_pos(k, o, 8)];
   }
+#pragma unroll 8
   for (uint32_t i = tid; i < 64 * 64; i += kTrainThreads) {
     const uint32_t o = i >> 6, k = i & 63;
     *reinterpret_cast<__half*>(tsm + kTrW2 + tc::kmajor_offset(o, k, 64)) = himg[4 * kF1 + frag_pos(k, o, 8)];
@@ -613,10 +626,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       *reinterpret_cast<uint4*>(X + tc::kmajor_offset(tid, 0, 16)) = make_uint4(xp[0], xp[1], xp[2], xp[3]);
       *reinterpret_cast<uint4*>(X + tc::kmajor_offset(tid, 8, 16)) = make_uint4(xp[4], xp[5], xp[6], xp[7]);
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        st_t16(GB, 64 + 2 * q, tid, xp[q] & 0xFFFFu);
-        st_t16(GB, 65 + 2 * q, tid, xp[q] >> 16);
-      }
+      for (int q = 0; q < 8; q++) st_t16_rows(GB, 64 + 2 * q, tid, xp[q]);
       tgt[2 * tid] = __fmul_rn(tg[2 * (size_t)idx], inv_os0);
       tgt[2 * tid + 1] = __fmul_rn(tg[2 * (size_t)idx + 1], inv_os1);
     }
@@ -640,9 +650,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 #pragma unroll
         for (int j = 0; j < 8; j++) {
           hp[j] = silu_half_f16x2(__fadd_rn(v[q][2 * j], bias[c + 2 * j]), __fadd_rn(v[q][2 * j + 1], bias[c + 2 * j + 1]));
-          const uint32_t b = f16x2_to_bf16x2(hp[j]);
-          st_t16(GB, c + 2 * j, tid, b & 0xFFFFu);
-          st_t16(GB, c + 2 * j + 1, tid, b >> 16);
+          st_t16_rows(GB, c + 2 * j, tid, f16x2_to_bf16x2(hp[j]));
         }
         *reinterpret_cast<uint4*>(A + tc::kmajor_offset(tid, c, 64)) = make_uint4(hp[0], hp[1], hp[2], hp[3]);
         *reinterpret_cast<uint4*>(A + tc::kmajor_offset(tid, c + 8, 64)) = make_uint4(hp[4], hp[5], hp[6], hp[7]);
@@ -697,11 +705,13 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     // ---- dW3[o][n] = sum_k dY[k][o] H2[k][n] and db3 (f32, sample order; H2 from A)
     {
       const uint32_t o = tid >> 6, n = tid & 63;
-      for (uint32_t kk = 0; kk < kTileRows; kk++)
-        acc_w3 = __fadd_rn(acc_w3, __fmul_rn(dy[2 * kk + o],
-                                             __half2float(*reinterpret_cast<const __half*>(A + tc::kmajor_offset(kk, n, 64)))));
-      if (tid < kOut)
-        for (uint32_t kk = 0; kk < kTileRows; kk++) acc_b3 = __fadd_rn(acc_b3, dy[2 * kk + tid]);
+#pragma unroll 16
+      for (uint32_t kk = 0; kk < kTileRows; kk++) {
+        const float d = dy[2 * kk + o];
+        acc_w3 = __fadd_rn(acc_w3, __fmul_rn(d, __half2float(*reinterpret_cast<const __half*>(
+                                                    A + tc::kmajor_offset(kk, n, 64)))));
+        acc_b3 = __fadd_rn(acc_b3, d);  // db3[o], the same in the 64 threads of o
+      }
     }
     __syncthreads();
     // ---- dZ2 = (dY W3) silu'(z2): row tid of A (bf16) and column tid of GA rows 0..63
@@ -725,8 +735,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
             const float d1 = __fmul_rn(__fadd_rn(__fmul_rn(dy0, w3f[c0 + 1]), __fmul_rn(dy1, w3f[kHidden + c0 + 1])),
                                        dsilu_half(__fadd_rn(v[q][2 * j + 1], bias[kHidden + c0 + 1])));
             dp[j] = pack_bf16(d0, d1);
-            st_t16(GA, c0, tid, dp[j] & 0xFFFFu);
-            st_t16(GA, c0 + 1, tid, dp[j] >> 16);
+            st_t16_rows(GA, c0, tid, dp[j]);
           }
           *reinterpret_cast<uint4*>(A + tc::kmajor_offset(tid, c, 64)) = make_uint4(dp[0], dp[1], dp[2], dp[3]);
           *reinterpret_cast<uint4*>(A + tc::kmajor_offset(tid, c + 8, 64)) = make_uint4(dp[4], dp[5], dp[6], dp[7]);
@@ -759,9 +768,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
           const int c0 = c + 2 * j;
           const float d0 = __fmul_rn(v[q][2 * j], dsilu_half(__fadd_rn(z[q][2 * j], bias[c0])));
           const float d1 = __fmul_rn(v[q][2 * j + 1], dsilu_half(__fadd_rn(z[q][2 * j + 1], bias[c0 + 1])));
-          const uint32_t p = pack_bf16(d0, d1);
-          st_t16(GA, 64 + c0, tid, p & 0xFFFFu);
-          st_t16(GA, 65 + c0, tid, p >> 16);
+          st_t16_rows(GA, 64 + c0, tid, pack_bf16(d0, d1));
         }
       }
     }
@@ -786,13 +793,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         tc::tmem_ld16(tm + lanes + kColG + 16 * q, g);
         tc::tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 16; j++) P[kOffW2 + tid * kHidden + 16 * q + j] = g[j];
+        for (int j = 0; j < 16; j += 4)
+          *reinterpret_cast<float4*>(&P[kOffW2 + tid * kHidden + 16 * q + j]) =
+              make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]);
       }
     } else {
       tc::tmem_ld16(tm + lanes + kColG + 64, g);
       tc::tmem_wait_ld();
 #pragma unroll
-      for (int j = 0; j < 16; j++) P[kOffW1 + (tid - 64) * kFeat + j] = g[j];
+      for (int j = 0; j < 16; j += 4)
+        *reinterpret_cast<float4*>(&P[kOffW1 + (tid - 64) * kFeat + j]) =
+            make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]);
     }
     tc::tmem_ld16(tm + lanes + kColG + 80, g);
     tc::tmem_wait_ld();
@@ -802,7 +813,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
       P[kOffB1 + tid - 64] = g[0];
   }
   P[kOffW3 + tid] = acc_w3;
-  if (tid < kOut) P[kOffB3 + tid] = acc_b3;
+  if ((tid & 63u) == 0u) P[kOffB3 + (tid >> 6)] = acc_b3;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) loss = __fadd_rn(loss, __shfl_xor_sync(0xFFFFFFFFu, loss, o));
   if (lane == 0) wl[warp] = loss;
@@ -820,50 +831,90 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   }
 }
 
-// Sum of the CTA partials (CTA order) per parameter.
-__device__ __forceinline__ float sum_parts(const float* __restrict__ part, uint32_t nparts, int p) {
+// Sums of the CTA partials in CTA order for kAdamParams consecutive parameters
+// from p0 on, by a block of kAdamThreads: the threads read up to 256 partials of
+// each parameter at once into shared memory, then one thread per parameter adds
+// them up (5.5 MB for 256 CTAs: 6.2 us; one thread reading and adding a parameter's
+// partials on 22 SMs took 15.6). Thread t < kAdamParams returns the
+// sum of parameter p0 + t.
+constexpr int kAdamParams = 32, kAdamThreads = 256;
+__device__ __forceinline__ float sum_parts(const float* __restrict__ part, uint32_t nparts, int p0,
+                                           float (&buf)[256][kAdamParams]) {
+  constexpr uint32_t kRows = 256 * kAdamParams / kAdamThreads;  // partials per thread
+  const uint32_t i = threadIdx.x % kAdamParams, q = threadIdx.x / kAdamParams;
   float g = 0.0f;
-  for (uint32_t c = 0; c < nparts; c++) g = __fadd_rn(g, part[(size_t)c * kPartStride + p]);
+  for (uint32_t base = 0; base < nparts; base += 256u) {
+    if (base) __syncthreads();
+    if (p0 + (int)i <= kParams) {
+      float v[kRows];
+#pragma unroll
+      for (uint32_t r = 0; r < kRows; r++) {
+        const uint32_t c = base + q * kRows + r;
+        v[r] = c < nparts ? __ldg(&part[(size_t)c * kPartStride + p0 + i]) : 0.0f;
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < kRows; r++) buf[q * kRows + r][i] = v[r];
+    }
+    __syncthreads();
+    if (threadIdx.x < kAdamParams) {
+      const uint32_t m = min(256u, nparts - base);
+#pragma unroll 16
+      for (uint32_t c = 0; c < m; c++) g = __fadd_rn(g, buf[c][i]);
+    }
+  }
   return g;
 }
 
-__global__ void k_mlp_reduce(const float* __restrict__ part, uint32_t nparts, float inv_2b, float* __restrict__ grad,
-                             float* __restrict__ loss) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < kParams) grad[p] = sum_parts(part, nparts, p);
-  if (p == kParams) *loss = __fmul_rn(sum_parts(part, nparts, kParams), inv_2b);
+__global__ void __launch_bounds__(kAdamThreads)
+    k_mlp_reduce(const float* __restrict__ part, uint32_t nparts, float inv_2b, float* __restrict__ grad,
+                 float* __restrict__ loss) {
+  __shared__ float buf[256][kAdamParams];
+  const int p0 = blockIdx.x * kAdamParams, p = p0 + threadIdx.x;
+  const float g = sum_parts(part, nparts, p0, buf);
+  if (threadIdx.x >= kAdamParams) return;
+  if (p < kParams) grad[p] = g;
+  if (p == kParams) *loss = __fmul_rn(g, inv_2b);
 }
 
 // Adam (Kingma & Ba 2015) on step t = ctr[0] + 1:
 //   m = b1 m + (1 - b1) g,  v = b2 v + (1 - b2) g^2,
 //   w -= lr * (m / (1 - b1^t)) / (sqrt(v / (1 - b2^t)) + eps)
-__global__ void k_mlp_adam(const float* __restrict__ part, uint32_t nparts, float* __restrict__ w, float* __restrict__ m,
-                           float* __restrict__ v, const uint32_t* __restrict__ ctr, float lr, float inv_2b,
-                           float* __restrict__ loss_hist, uint32_t loss_base, uint32_t loss_cap, uint2* frag,
-                           float* bias, float* w3) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// The last block to finish advances the step (ctr[3] counts them, zero between
+// launches).
+__global__ void __launch_bounds__(kAdamThreads)
+    k_mlp_adam(const float* __restrict__ part, uint32_t nparts, float* __restrict__ w, float* __restrict__ m,
+               float* __restrict__ v, uint32_t* __restrict__ ctr, float lr, float inv_2b,
+               float* __restrict__ loss_hist, uint32_t loss_base, uint32_t loss_cap, uint2* frag, float* bias,
+               float* w3) {
+  __shared__ float buf[256][kAdamParams];
+  __shared__ float s_bc[2];
+  const int p0 = blockIdx.x * kAdamParams, p = p0 + threadIdx.x;
   const uint32_t t0 = ctr[0];
-  if (p == kParams) {
-    if (loss_hist && t0 >= loss_base && t0 - loss_base < loss_cap)
-      loss_hist[t0 - loss_base] = __fmul_rn(sum_parts(part, nparts, kParams), inv_2b);
-    return;
+  if (threadIdx.x >= kAdamThreads - 2) {  // 1 - b1^t, 1 - b2^t (by a warp that adds up nothing)
+    const int k = threadIdx.x - (kAdamThreads - 2);
+    s_bc[k] = (float)(1.0 - pow(k == 0 ? (double)kBeta1 : (double)kBeta2, (double)t0 + 1.0));
   }
-  if (p > kParams) return;
-  const float g = sum_parts(part, nparts, p);
-  const double tt = (double)t0 + 1.0;
-  const float bc1 = (float)(1.0 - pow((double)kBeta1, tt));
-  const float bc2 = (float)(1.0 - pow((double)kBeta2, tt));
-  const float mm = __fadd_rn(__fmul_rn(kBeta1, m[p]), __fmul_rn(__fsub_rn(1.0f, kBeta1), g));
-  const float vv = __fadd_rn(__fmul_rn(kBeta2, v[p]), __fmul_rn(__fsub_rn(1.0f, kBeta2), __fmul_rn(g, g)));
-  const float upd = __fdiv_rn(__fdiv_rn(mm, bc1), __fadd_rn(__fsqrt_rn(__fdiv_rn(vv, bc2)), kAdamEps));
-  const float ww = __fsub_rn(w[p], __fmul_rn(lr, upd));
-  m[p] = mm;
-  v[p] = vv;
-  w[p] = ww;
-  write_weight(p, ww, reinterpret_cast<__nv_bfloat16*>(frag), bias, w3);
+  const float g = sum_parts(part, nparts, p0, buf);
+  __syncthreads();
+  if (threadIdx.x >= kAdamParams) return;
+  if (p == kParams) {
+    if (loss_hist && t0 >= loss_base && t0 - loss_base < loss_cap) loss_hist[t0 - loss_base] = __fmul_rn(g, inv_2b);
+  } else if (p < kParams) {
+    const float mm = __fadd_rn(__fmul_rn(kBeta1, m[p]), __fmul_rn(__fsub_rn(1.0f, kBeta1), g));
+    const float vv = __fadd_rn(__fmul_rn(kBeta2, v[p]), __fmul_rn(__fsub_rn(1.0f, kBeta2), __fmul_rn(g, g)));
+    const float upd = __fdiv_rn(__fdiv_rn(mm, s_bc[0]), __fadd_rn(__fsqrt_rn(__fdiv_rn(vv, s_bc[1])), kAdamEps));
+    const float ww = __fsub_rn(w[p], __fmul_rn(lr, upd));
+    m[p] = mm;
+    v[p] = vv;
+    w[p] = ww;
+    write_weight(p, ww, reinterpret_cast<__nv_bfloat16*>(frag), bias, w3);
+  }
+  // every thread of the block has read ctr[0] (the barriers above)
+  if (threadIdx.x == 0 && atomicAdd(&ctr[3], 1u) + 1u == gridDim.x) {
+    ctr[3] = 0u;
+    ctr[0] = t0 + 1u;
+  }
 }
-
-__global__ void k_mlp_advance(uint32_t* ctr) { ctr[0] += 1u; }
 
 __global__ void k_mlp_indices(uint64_t seed, uint32_t iter, uint32_t batch, uint32_t npairs, uint32_t* out) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -934,7 +985,7 @@ struct PhiengMlp {
   float* bias = nullptr;
   float* w3 = nullptr;
   float* norm = nullptr;
-  uint32_t* ctr = nullptr;  // [0] Adam step, [1] iteration for a gradient check
+  uint32_t* ctr = nullptr;  // [0] Adam step, [1] iteration for a gradient check, [2] wait flag, [3] Adam blocks done
   float* part = nullptr;
   uint32_t part_cap = 0;
   float* grad = nullptr;    // kParams + 1 (loss)
@@ -1162,7 +1213,7 @@ int32_t phieng_mlp_grad(PhiengMlp* m, const float* x, const float* t, uint32_t n
   uint32_t nparts = 0;
   if (!launch_tile(m, x, t, npairs, batch, seed, m->ctr + 1, &nparts)) return 0;
   const float inv_2b = (float)(0.5 / (double)batch);
-  k_mlp_reduce<<<cdiv(kParams + 1, 256), 256, 0, m->stream>>>(m->part, nparts, inv_2b, m->grad, m->grad + kParams);
+  k_mlp_reduce<<<cdiv(kParams + 1, kAdamParams), kAdamThreads, 0, m->stream>>>(m->part, nparts, inv_2b, m->grad, m->grad + kParams);
   if (!mlp_ok(m, cudaGetLastError())) return 0;
   if (!mlp_ok(m, cudaMemcpyAsync(m->h_pinned, m->grad, sizeof(float) * (kParams + 1), cudaMemcpyDeviceToHost,
                                  m->stream)) ||
@@ -1193,7 +1244,7 @@ int32_t phieng_mlp_train(PhiengMlp* m, const float* x, const float* t, uint32_t 
   }
   const uint32_t t0 = phieng_mlp_step_count(m);
   const float inv_2b = (float)(0.5 / (double)batch);
-  // one iteration = tile, Adam, advance; replayed from a graph of up to 32
+  // one iteration = tile, Adam; replayed from a graph of up to 32
   const uint32_t per_graph = std::min<uint32_t>(iters, 32u);
   auto enqueue = [&](uint32_t k, cudaStream_t st) -> bool {
     cudaStream_t keep = m->stream;
@@ -1203,10 +1254,9 @@ int32_t phieng_mlp_train(PhiengMlp* m, const float* x, const float* t, uint32_t 
       uint32_t nparts = 0;
       ok = launch_tile(m, x, t, npairs, batch, seed, m->ctr, &nparts);
       if (ok) {
-        k_mlp_adam<<<cdiv(kParams + 1, 256), 256, 0, st>>>(m->part, nparts, m->w, m->m, m->v, m->ctr, lr, inv_2b,
-                                                            loss_hist_host ? m->loss_hist : nullptr, t0, iters,
-                                                            m->frag, m->bias, m->w3);
-        k_mlp_advance<<<1, 1, 0, st>>>(m->ctr);
+        k_mlp_adam<<<cdiv(kParams + 1, kAdamParams), kAdamThreads, 0, st>>>(
+            m->part, nparts, m->w, m->m, m->v, m->ctr, lr, inv_2b, loss_hist_host ? m->loss_hist : nullptr, t0, iters,
+            m->frag, m->bias, m->w3);
         ok = mlp_ok(m, cudaGetLastError());
       }
     }
@@ -1246,16 +1296,15 @@ int32_t phieng_mlp_shard_grad(PhiengMlp* m, const float* x, const float* t, uint
   uint32_t nparts = 0;
   if (!launch_tile(m, x, t, npairs, batch, seed, m->ctr, &nparts, first, total)) return 0;
   // raw sums: the gradient already carries 1 / total, the loss is the sum of squared errors
-  k_mlp_reduce<<<cdiv(kParams + 1, 256), 256, 0, m->stream>>>(m->part, nparts, 1.0f, grad, grad + kParams);
+  k_mlp_reduce<<<cdiv(kParams + 1, kAdamParams), kAdamThreads, 0, m->stream>>>(m->part, nparts, 1.0f, grad, grad + kParams);
   return mlp_ok(m, cudaGetLastError()) ? 1 : 0;
 }
 
 int32_t phieng_mlp_apply_grad(PhiengMlp* m, const float* grad, float lr) {
   if (!m || m->error || !grad || !(lr > 0.0f)) return 0;
   // a single gradient vector is a partial list of length one
-  k_mlp_adam<<<cdiv(kParams + 1, 256), 256, 0, m->stream>>>(grad, 1, m->w, m->m, m->v, m->ctr, lr, 0.0f, nullptr, 0,
-                                                              0, m->frag, m->bias, m->w3);
-  k_mlp_advance<<<1, 1, 0, m->stream>>>(m->ctr);
+  k_mlp_adam<<<cdiv(kParams + 1, kAdamParams), kAdamThreads, 0, m->stream>>>(
+      grad, 1, m->w, m->m, m->v, m->ctr, lr, 0.0f, nullptr, 0, 0, m->frag, m->bias, m->w3);
   return mlp_ok(m, cudaGetLastError()) ? 1 : 0;
 }
 
