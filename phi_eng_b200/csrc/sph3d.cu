@@ -30,6 +30,7 @@
 #include "sph_kernels.h"
 #include "sph_noise.cuh"
 #include "sph_snapshot.h"
+#include "sph_sort_runs.cuh"
 #include "sph_sort_small.cuh"
 #include "sph_warp.cuh"
 
@@ -642,30 +643,25 @@ struct Gather3 {
   float4 *spos, *svel;
   float* smass;     // null: uniform
   uint8_t* sphase;  // null: uniform
-  __device__ __forceinline__ void operator()(uint32_t f, uint32_t k, uint32_t id) const {
+  struct Row {
+    float4 p, v;
+    float m;
+    uint8_t ph;
+  };
+  __device__ __forceinline__ Row load(uint32_t id) const {
+    return {pos[id], vel[id], smass ? mass[id] : 0.0f, sphase ? phase[id] : (uint8_t)0};
+  }
+  __device__ __forceinline__ void store(uint32_t f, uint32_t k, uint32_t id, const Row& r) const {
     skey[f] = k;
     sid[f] = id;
-    const float4 p = pos[id];
-    spos[f] = p;
-    sq[f] = cell_word(p.x, p.y, p.z, units);
-    svel[f] = vel[id];
-    if (smass) smass[f] = mass[id];
-    if (sphase) sphase[f] = phase[id];
+    spos[f] = r.p;
+    sq[f] = cell_word(r.p.x, r.p.y, r.p.z, units);
+    svel[f] = r.v;
+    if (smass) smass[f] = r.m;
+    if (sphase) sphase[f] = r.ph;
   }
+  __device__ __forceinline__ void operator()(uint32_t f, uint32_t k, uint32_t id) const { store(f, k, id, load(id)); }
 };
-
-// In-bucket rank by id, then the gather into sorted order.
-__global__ void __launch_bounds__(256) k_fixup3(const uint32_t* __restrict__ tkey, const uint32_t* __restrict__ tid_in,
-                                                const uint32_t* __restrict__ start, uint32_t n, Gather3 ga) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t k = tkey[s];
-  const uint32_t id = tid_in[s];
-  const uint32_t lo = start[k], hi = start[k + 1];
-  uint32_t rank = 0;
-  for (uint32_t j = lo; j < hi; j++) rank += __ldg(&tid_in[j]) < id ? 1u : 0u;
-  ga(lo + rank, k, id);
-}
 
 __device__ __forceinline__ uint32_t row_base3(uint32_t by, uint32_t bz, int r, const GridPlan3& g) {
   const uint32_t oz = (uint32_t)(r / 3) - 1u, oy = (uint32_t)(r % 3) - 1u;
@@ -1098,8 +1094,8 @@ __global__ void __launch_bounds__(256) k_unpack3(const float2* __restrict__ rows
 // bucket count. DEBUG: the force only. Where several lanes hold the same
 // particle, one of them is the writer.
 template <bool DEBUG, bool PLAIN, bool FAST>
-__device__ __forceinline__ void finish3(uint32_t id, bool writer, float4 pi, float4 vi, float rho_i, float q_i,
-                                        float (&f)[3], float (&sm)[3], const StepParams3& P,
+__device__ __forceinline__ void finish3(uint32_t s, uint32_t id, uint32_t* __restrict__ pid, bool writer,
+                                        float4 pi, float4 vi, float rho_i, float q_i, float (&f)[3], float (&sm)[3], const StepParams3& P,
                                         const DevBody3* __restrict__ bodies, float4* __restrict__ pos_out,
                                         float4* __restrict__ vel_out, uint32_t* __restrict__ key_out,
                                         uint32_t* __restrict__ count_out, float4* __restrict__ dbg) {
@@ -1119,6 +1115,7 @@ __device__ __forceinline__ void finish3(uint32_t id, bool writer, float4 pi, flo
     if (writer) dbg[id] = make_float4(f[0], f[1], f[2], 0.0f);
     return;
   }
+  if (writer) pid[s] = id;
   float ax = __fadd_rn(P.gx, __fdiv_rn(f[0], rho_i));
   float ay = __fadd_rn(P.gy, __fdiv_rn(f[1], rho_i));
   float az = __fadd_rn(P.gz, __fdiv_rn(f[2], rho_i));
@@ -1190,7 +1187,8 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
                                                 const DevBody3* __restrict__ bodies,
                                                 const uint32_t* __restrict__ nmask, float4* __restrict__ pos_out,
                                                 float4* __restrict__ vel_out, uint32_t* __restrict__ key_out,
-                                                uint32_t* __restrict__ count_out, float4* __restrict__ dbg) {
+                                                uint32_t* __restrict__ count_out, float4* __restrict__ dbg,
+                                                uint32_t* __restrict__ pid) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t k = skey[s];
@@ -1268,7 +1266,8 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
       }
     }
   }
-  finish3<DEBUG, PLAIN, FAST>(id, true, pi, vi, rho_i, q_i, f, sm, P, bodies, pos_out, vel_out, key_out, count_out, dbg);
+  finish3<DEBUG, PLAIN, FAST>(s, id, pid, true, pi, vi, rho_i, q_i, f, sm, P, bodies, pos_out, vel_out, key_out,
+                              count_out, dbg);
 }
 
 #include "sph3d_coop.cuh"
@@ -1488,7 +1487,7 @@ struct World3 {
   bool host_valid = true, dev_valid = false, aux_valid = false, keys_valid = false;
   bool dp_dev = false;  // the sorted density / pressure on the device are newer than h_dens / h_pres
   bool plan_valid = false;
-  uint32_t sid_perm_n = 0;
+  uint32_t sid_perm_n = 0;  // pid is a permutation of [0, sid_perm_n)
   GridPlan3 plan{};
   int device = -1;
   cudaStream_t own_stream = nullptr, stream = nullptr;
@@ -1501,7 +1500,9 @@ struct World3 {
   float *mass = nullptr, *smass = nullptr, *spres = nullptr, *tmp = nullptr;
   uint8_t *phase = nullptr, *sphase = nullptr;
   uint32_t *key = nullptr, *tkey = nullptr, *tid = nullptr, *skey = nullptr, *sid = nullptr, *nmask = nullptr;
-  uint32_t* sq = nullptr;  // sorted cell_word
+  uint32_t* sq = nullptr;     // sorted cell_word
+  uint32_t* pid = nullptr;    // the ids in the slot order of the last force pass (the next placement's order)
+  uint32_t* flist = nullptr;  // placement slots left to rank
   float2* sdq = nullptr;
   uint32_t *count = nullptr, *start = nullptr, *tilesum = nullptr, *scalar = nullptr;
   unsigned long long* tstate = nullptr;  // single-pass scan tile states
@@ -1560,6 +1561,7 @@ void free_particles3(World3* w) {
   dfree3(w->pos), dfree3(w->vel), dfree3(w->spos), dfree3(w->svel), dfree3(w->mass), dfree3(w->smass);
   dfree3(w->spres), dfree3(w->tmp), dfree3(w->phase), dfree3(w->sphase), dfree3(w->key), dfree3(w->tkey);
   dfree3(w->tid), dfree3(w->skey), dfree3(w->sid), dfree3(w->nmask), dfree3(w->sdq), dfree3(w->sq);
+  dfree3(w->pid), dfree3(w->flist);
   w->dcap = 0;
 }
 
@@ -1591,7 +1593,8 @@ bool ensure_capacity3(World3* w, uint32_t need) {
                   dalloc3(w, w->mass, c) && dalloc3(w, w->smass, c) && dalloc3(w, w->spres, c) &&
                   dalloc3(w, w->tmp, 2 * (size_t)c) && dalloc3(w, w->phase, c) && dalloc3(w, w->sphase, c) &&
                   dalloc3(w, w->key, c) && dalloc3(w, w->tkey, c) && dalloc3(w, w->tid, c) && dalloc3(w, w->skey, c) &&
-                  dalloc3(w, w->sid, c) && dalloc3(w, w->nmask, kMaskWords3 * (size_t)c) && dalloc3(w, w->sdq, c) && dalloc3(w, w->sq, (size_t)c + 4);
+                  dalloc3(w, w->sid, c) && dalloc3(w, w->nmask, kMaskWords3 * (size_t)c) && dalloc3(w, w->sdq, c) &&
+                  dalloc3(w, w->sq, (size_t)c + 4) && dalloc3(w, w->pid, c) && dalloc3(w, w->flist, c);
   if (!ok) {
     free_particles3(w);
     return false;
@@ -2014,17 +2017,15 @@ StepParams3 make_params3(const World3* w, float dt) {
   return P;
 }
 
-// Sort by (bucket key, id) and gather. counts: the bucket counts of the keys
-// (consumed as the placement cursor); clear: zeroed after the sort when set
-// (the force pass counts the next keys there).
-void enqueue_sorted3(World3* w, const StepParams3& P, uint32_t* counts, bool by_slot, uint32_t* clear,
-                     cudaStream_t st) {
+// Sort by (bucket key, id) and gather. counts: the bucket counts of the keys,
+// zero afterwards.
+void enqueue_sorted3(World3* w, const StepParams3& P, uint32_t* counts, bool by_slot, cudaStream_t st) {
   const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
-  const Gather3 ga{w->pos, w->vel, w->mass, w->phase, w->skey, w->sid, w->sq, P.cell_units, w->spos, w->svel, m ? w->smass : nullptr,
-                   ph ? w->sphase : nullptr};
+  const Gather3 ga{w->pos,  w->vel,  w->mass, w->phase, w->skey, w->sid, w->sq, P.cell_units,
+                   w->spos, w->svel, m ? w->smass : nullptr, ph ? w->sphase : nullptr};
   const uint32_t nkeys = P.grid.sentinel + 1;
   if (small_sort_applies(w->n, nkeys)) {
-    launch_sort_small(w->key, w->n, nkeys, w->start, clear, w->count_len, ga, st);
+    launch_sort_small(w->key, w->n, nkeys, w->start, counts, w->count_len, ga, st);
     return;
   }
   BucketSort bs;
@@ -2035,16 +2036,16 @@ void enqueue_sorted3(World3* w, const StepParams3& P, uint32_t* counts, bool by_
   bs.err = w->scalar + 12;
   bs.start = w->start;
   bs.key = w->key;
-  bs.sid_prev = w->sid;
+  bs.prev = w->pid;
   bs.tkey = w->tkey;
   bs.tid = w->tid;
-  enqueue_bucket_place(bs, w->n, nkeys, by_slot, st);
-  k_fixup3<<<cdiv(w->n, 256), 256, 0, st>>>(w->tkey, w->tid, w->start, w->n, ga);
-  if (clear) cudaMemsetAsync(clear, 0, sizeof(uint32_t) * w->count_len, st);
+  bs.list = w->flist;
+  bs.list_n = w->scalar + 25;
+  enqueue_bucket_sort(bs, w->n, nkeys, by_slot, ga, st);
 }
 
 void enqueue_sort3(World3* w, const StepParams3& P, cudaStream_t st) {
-  enqueue_sorted3(w, P, w->count, w->sid_perm_n == w->n, w->count, st);
+  enqueue_sorted3(w, P, w->count, w->sid_perm_n == w->n, st);
 }
 
 void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
@@ -2096,7 +2097,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
 #define PHIENG_F3G(M, D, PL, FA)                                                                           \
   k_force3_coop<M, D, PL, FA><<<cdiv(w->n, kCoopThreads / kCoopLanes), kCoopThreads, 0, st>>>(             \
       w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, P, w->dbodies, w->nmask, w->pos, \
-      w->vel, w->key, w->count, dbg)
+      w->vel, w->key, w->count, dbg, w->pid)
     if (fast) {
       if (dbg) PHIENG_F3G(false, true, true, true);
       else PHIENG_F3G(false, false, true, true);
@@ -2115,7 +2116,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
   }
 #define PHIENG_F3X(M, D, PL, FA)                                                                                    \
   k_force3<M, D, PL, FA><<<g, kForceThreads3, 0, st>>>(w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
-                                            P, w->dbodies, w->nmask, w->pos, w->vel, w->key, w->count, dbg)
+                                            P, w->dbodies, w->nmask, w->pos, w->vel, w->key, w->count, dbg, w->pid)
 #define PHIENG_F3(M, D, PL) PHIENG_F3X(M, D, PL, false)
   if (fast) {
     if (dbg) PHIENG_F3X(false, true, true, true);
@@ -2245,7 +2246,6 @@ bool run_substep3_adaptive(World3* w, float dt) {
   cudaStream_t st = w->stream;
   StepParams3 P = make_params3(w, dt);
   enqueue_sort3(w, P, st);
-  w->sid_perm_n = w->n;
   enqueue_density3(w, P, st);
   const FluidConfig3Ffi& cf = w->cfg;
   const float rest = std::max(cf.rest_density, kEps);
@@ -2500,7 +2500,7 @@ void enqueue_resort3(World3* w, const StepParams3& P, cudaStream_t st) {
   const uint32_t g = cdiv(w->n, 256);
   k_dp_to_id3<<<g, 256, 0, st>>>(w->sdq, w->spres, w->sid, w->n, w->d_dq_id, w->d_p_id);
   cudaMemcpyAsync(w->d_count2, w->count, sizeof(uint32_t) * w->count_len, cudaMemcpyDeviceToDevice, st);
-  enqueue_sorted3(w, P, w->d_count2, true, nullptr, st);
+  enqueue_sorted3(w, P, w->d_count2, w->sid_perm_n == w->n, st);
   k_dp_from_id3<<<g, 256, 0, st>>>(w->d_dq_id, w->d_p_id, w->sid, w->n, w->sdq, w->spres);
 }
 
@@ -2623,7 +2623,6 @@ bool step_fluid_bodies3(World3* w, PhiengBody3* bodies, uint32_t nb, float dt, c
   const size_t dlen = (size_t)((w->n + 1 + kBucketScanTile - 1) / kBucketScanTile) * kBucketScanTile;
   for (uint32_t k = 0; k < ns; k++) {
     enqueue_sort3(w, P, st);
-    w->sid_perm_n = w->n;
     enqueue_density3(w, P, st);
     if ((P.flags & F_GHOST) && P.nghost) {
       if (P.flags & F_MASS)
@@ -2633,6 +2632,7 @@ bool step_fluid_bodies3(World3* w, PhiengBody3* bodies, uint32_t nb, float dt, c
     }
     if (any_dyn) cudaMemsetAsync(w->d_dcount, 0, sizeof(uint32_t) * dlen, st);
     enqueue_force3(w, P, nullptr, st);
+    w->sid_perm_n = w->n;
     if (any_dyn) {
       enqueue_flag_compact(w->d_dcount, w->n, w->d_dtile, w->scalar + 20, w->d_dstart, w->d_list, st);
       k_dynamic_walls3<<<1, 32, 0, st>>>(w->d_list, w->d_dstart + w->n, w->pos, w->vel, w->mass, w->key, w->count,
@@ -3105,7 +3105,6 @@ uint32_t phieng_sph3_debug_forces(World3* w, float* dens, float* pres, float* fx
   enqueue_sort3(w, P, w->stream);
   enqueue_density3(w, P, w->stream);
   if (fxyz) enqueue_force3(w, P, dbg, w->stream);
-  w->sid_perm_n = w->n;
   w->keys_valid = false;  // the sort consumed the bucket counts
   w->dp_dev = true;
   std::vector<float> f(fxyz ? 4 * (size_t)w->n : 0);

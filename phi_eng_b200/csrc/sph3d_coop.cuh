@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
     const uint32_t* __restrict__ start, StepParams3 P, const DevBody3* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, float4* __restrict__ pos_out,
     float4* __restrict__ vel_out, uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out,
-    float4* __restrict__ dbg) {
+    float4* __restrict__ dbg, uint32_t* __restrict__ pid) {
   constexpr int G = kCoopLanes;
   static_assert(G == 8, "six lanes of a group hold the sums; lanes 0..7 expand rows 0..7");
   constexpr uint32_t kAll = 0xFFFFFFFFu, kGroups = kCoopThreads / G;
@@ -290,6 +290,6 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
     sm[a] = __shfl_sync(kAll, acc, 3 + a, G);
   }
   if (!active) return;
-  finish3<DEBUG, PLAIN, FAST>(id, l == 0u, pi, vi, rho_i, q_i, f, sm, P, bodies, pos_out, vel_out, key_out, count_out,
-                              dbg);
+  finish3<DEBUG, PLAIN, FAST>(s, id, pid, l == 0u, pi, vi, rho_i, q_i, f, sm, P, bodies, pos_out, vel_out, key_out,
+                              count_out, dbg);
 }

@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(128, 6) k_closure_tc(
     const float* __restrict__ spres, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sid, uint32_t n,
     const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, MlpDev mlp, ClosureIO io, float4* __restrict__ state_out,
-    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ err) {
+    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ err,
+    uint32_t* __restrict__ pid) {
   extern __shared__ __align__(1024) unsigned char net_smem[];
   TcNet net = tc_net_init(net_smem, mlp);
   bool ok = true;
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(128, 6) k_closure_tc(
       const float xs = __fmul_rn(__fmul_rn(2.0f, P.mass), P.c_poly6);
       const float ax = __fadd_rn(__fadd_rn(P.gx, __fdiv_rn(fx, pair.rho_i)), __fmul_rn(y[0], acc_scale));
       const float ay = __fadd_rn(__fadd_rn(P.gy, __fdiv_rn(fy, pair.rho_i)), __fmul_rn(y[1], acc_scale));
-      integrate_write<false>(id, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xs), __fmul_rn(sy, xs), P, bodies, state_out,
+      integrate_write<false>(s, id, pid, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xs), __fmul_rn(sy, xs), P, bodies, state_out,
                              key_out, count_out);
     }
   }
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(256, 4) k_closure_fast(
     const float* __restrict__ spres, const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sid, uint32_t n,
     const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, MlpDev mlp, ClosureIO io, float4* __restrict__ state_out,
-    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out) {
+    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ pid) {
   extern __shared__ __align__(16) unsigned char closure_smem[];
   MlpSmem& sm = *reinterpret_cast<MlpSmem*>(closure_smem);
   __nv_bfloat16* sx_all = reinterpret_cast<__nv_bfloat16*>(closure_smem + sizeof(MlpSmem));
@@ -212,6 +213,6 @@ __global__ void __launch_bounds__(256, 4) k_closure_fast(
   const float cy = __fmul_rn(__fmul_rn(ys[2 * lane + 1], sm.norm[2 * kFeat + 1]), acc_scale);
   const float ax = __fadd_rn(__fadd_rn(P.gx, __fdiv_rn(fx, pair.rho_i)), cx);
   const float ay = __fadd_rn(__fadd_rn(P.gy, __fdiv_rn(fy, pair.rho_i)), cy);
-  integrate_write<false>(id, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xsc), __fmul_rn(sy, xsc), P, bodies, state_out,
-                         key_out, count_out);
+  integrate_write<false>(s, id, pid, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xsc), __fmul_rn(sy, xsc), P, bodies,
+                         state_out, key_out, count_out);
 }

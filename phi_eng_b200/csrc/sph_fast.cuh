@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(256) k_force_fast(
     const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
     uint32_t* __restrict__ count_out, float2* __restrict__ dbg_force, uint32_t* __restrict__ defer,
-    uint32_t* __restrict__ dcount) {
+    uint32_t* __restrict__ dcount, uint32_t* __restrict__ pid) {
   static_assert(!(STAGE && BALANCE), "staging windows assume the block's own slot order");
   extern __shared__ __align__(16) float2 fast_win[];
   const uint32_t s = BALANCE ? balanced_slot(nmask, n) : blockIdx.x * blockDim.x + threadIdx.x;
@@ -354,6 +354,6 @@ __global__ void __launch_bounds__(256) k_force_fast(
   const float xs = __fmul_rn(__fmul_rn(2.0f, P.mass), P.c_poly6);  // XSPH: m_j / rho_bar * W = 2 m c t^3 / (rho_i + rho_j)
   const float ax = __fadd_rn(P.gx, __fdiv_rn(fx, pair.rho_i));
   const float ay = __fadd_rn(P.gy, __fdiv_rn(fy, pair.rho_i));
-  integrate_write<false>(id, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xs), __fmul_rn(sy, xs), P, bodies, state_out,
-                         key_out, count_out, defer, dcount);
+  integrate_write<false>(s, id, pid, pair.pi, pair.vi, ax, ay, __fmul_rn(sx, xs), __fmul_rn(sy, xs), P, bodies,
+                         state_out, key_out, count_out, defer, dcount);
 }

@@ -20,6 +20,7 @@
 
 #include "sph_kernels.h"
 #include "sph_noise.cuh"
+#include "sph_sort_runs.cuh"
 #include "sph_sort_small.cuh"
 #include "sph_tc_net.cuh"
 #include "sph_warp.cuh"
@@ -35,14 +36,15 @@ namespace {
 //   count   K1 / K6 add each particle to count[key] (K1 warp-aggregated,
 //           K6 one atomic per particle)
 //   scan    count -> start (exclusive; start doubles as the bucket range
-//           table: bucket b holds slots [start[b], start[b+1])), and count
-//           becomes the placement cursor
-//   place   each particle takes a slot in its bucket from the cursor
-//           (arrival order inside a bucket is arbitrary)
-//   fixup   each particle's final slot = start[b] + (number of ids in its
-//           bucket smaller than its own); gathers the state into that slot
+//           table: bucket b holds slots [start[b], start[b+1]))
+//   place   buckets that arrive as one run in the previous sort's order are
+//           ranked by id and gathered at once; the particles of the others
+//           take a slot of their bucket, counting it down (sph_sort_runs.cuh)
+//   fix     those particles' final slot = start[b] + (number of ids in the
+//           bucket smaller than their own), and their gather
 // Buckets hold a handful of particles (a cell is h wide, the support radius),
-// so the in-bucket rank is a short loop.
+// so the in-bucket rank is a short loop. The counts are zero again after the
+// placement. Small sets take one launch instead (sph_sort_small.cuh).
 constexpr uint32_t kScanTile = kBucketScanTile;  // counts per scan block: 256 threads x 16
 
 // Block-wide inclusive scan of one value per thread (256 threads).
@@ -127,17 +129,16 @@ __global__ void __launch_bounds__(256) k_scan_reduce(const uint32_t* __restrict_
   if (tid == 0) *done = 0;
 }
 
-// start[i] = exclusive prefix of count[i]; count[i] is overwritten with the
-// same value (the placement cursor). Whole scan tiles are written with
+// start[i] = exclusive prefix of count[i]. Whole scan tiles are written with
 // 16-byte stores (the arrays are padded to whole tiles); m = number of keys
 // incl. the sentinel bucket, start[m] = particle count.
-__global__ void __launch_bounds__(256) k_scan_down(uint32_t* __restrict__ count,
+__global__ void __launch_bounds__(256) k_scan_down(const uint32_t* __restrict__ count,
                                                    const uint32_t* __restrict__ tileoff, uint32_t m,
                                                    uint32_t* __restrict__ start) {
   __shared__ uint32_t warp_tot[8];
   const uint32_t tid = threadIdx.x;
   const uint32_t base = blockIdx.x * kScanTile + tid * 16;
-  uint4* c4 = reinterpret_cast<uint4*>(count + base);
+  const uint4* c4 = reinterpret_cast<const uint4*>(count + base);
   uint32_t v[16];
 #pragma unroll
   for (int r = 0; r < 4; r++) {
@@ -161,70 +162,46 @@ __global__ void __launch_bounds__(256) k_scan_down(uint32_t* __restrict__ count,
   uint4* s4 = reinterpret_cast<uint4*>(start + base);
 #pragma unroll
   for (int r = 0; r < 4; r++) {
-    const uint4 q = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
-    c4[r] = q;
-    s4[r] = q;  // the padded tail past m gets the particle count: never read
+    // the padded tail past m gets the particle count: never read
+    s4[r] = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
   }
 }
 
 // Single-pass variant of k_scan_reduce + k_scan_down (decoupled look-back,
 // Merrill & Garland, "Single-pass Parallel Prefix Scan with Decoupled
-// Look-back", 2016), one block per supertile of kBucketScanSuper scan tiles:
-// supertiles are taken in ticket order; each publishes its sum
-// (flag 1) at once, then walks back over its predecessors' published values
-// until it meets an inclusive prefix (flag 2), and publishes its own
-// inclusive prefix. A block only waits for tiles that took an earlier ticket,
-// so are already running; each wait is still bounded (kScanSpinLimit reads,
-// then *err = 1 and the scan goes on with a wrong prefix). The last block to
-// finish clears the tile states and counters for the next scan. ctr[0] =
-// ticket, ctr[1] = finished blocks; both zero between scans. The tile whose
-// ticket equals silent publishes nothing (a test of the bounded waits; the
-// step passes 0xFFFFFFFF).
+// Look-back", 2016), one block per scan tile: tiles are taken in ticket order;
+// each publishes its sum (flag 1) at once, then looks back over its
+// predecessors' published values until it meets an inclusive prefix (flag 2),
+// and publishes its own inclusive prefix. Every thread of the block reads one
+// predecessor, 256 at a time: all tiles run at once and mostly find sums, not
+// prefixes, so a narrower window costs a round trip to L2 for every 32
+// predecessors (2^20 buckets 9.7 -> 8.6 us, 2^22 19 -> 15.3 us). A block only waits for tiles that took
+// an earlier ticket, so are already running; each wait is still bounded
+// (kScanSpinLimit reads, then *err = 1 and the scan goes on with a wrong
+// prefix). The last block to finish clears the tile states and counters for the
+// next scan. ctr[0] = ticket, ctr[1] = finished blocks; both zero between
+// scans. *zero (if not null) is set to 0. The tile whose ticket equals silent
+// publishes nothing (a test of the bounded waits; the step passes 0xFFFFFFFF).
 constexpr uint32_t kScanSpinLimit = 1u << 20;
 constexpr unsigned long long kTileAgg = 1ull << 32, kTileIncl = 2ull << 32;
 
-// Each look-back block of 256 * kLookbackSub threads scans kLookbackSub
-// consecutive scan tiles (a "supertile"), 16 counts per thread: every count
-// is loaded at once, as with one tile per 256-thread block, but the
-// look-back chain (a block walks its predecessors 32 at a time) is
-// kLookbackSub times shorter. The count arrays keep their padding to whole
-// scan tiles: a thread whose tile lies past the last does nothing.
-constexpr uint32_t kLookbackSub = kBucketScanSuper;
-constexpr uint32_t kLookbackThreads = 256 * kLookbackSub;
-
-// Block-wide inclusive scan of one value per thread (kLookbackThreads).
-__device__ __forceinline__ uint32_t block_incl_scan_big(uint32_t v, uint32_t* warp_tot) {
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-    if (lane >= (uint32_t)o) x += y;
-  }
-  if (lane == 31) warp_tot[w] = x;
-  __syncthreads();
-  uint32_t add = 0;
-  for (uint32_t k = 0; k < w; k++) add += warp_tot[k];
-  return x + add;
-}
-
-__global__ void __launch_bounds__(kLookbackThreads) k_scan_lookback(uint32_t* __restrict__ count, uint32_t nsub,
-                                                                    uint32_t* __restrict__ start,
-                                                                    unsigned long long* __restrict__ tstate,
-                                                                    uint32_t* __restrict__ ctr,
-                                                                    uint32_t* __restrict__ err, uint32_t silent) {
-  constexpr uint32_t kWarps = kLookbackThreads / 32;
-  __shared__ uint32_t warp_tot[kWarps];
-  __shared__ uint32_t s_tile, s_prefix;
+__global__ void __launch_bounds__(256) k_scan_lookback(const uint32_t* __restrict__ count,
+                                                       uint32_t* __restrict__ start,
+                                                       unsigned long long* __restrict__ tstate,
+                                                       uint32_t* __restrict__ ctr, uint32_t* __restrict__ err,
+                                                       uint32_t* __restrict__ zero, uint32_t silent) {
+  __shared__ uint32_t warp_tot[8];
+  __shared__ uint32_t s_tile, s_first[8], s_sum[8];
   __shared__ bool s_last;
-  if (threadIdx.x == 0) s_tile = atomicAdd(&ctr[0], 1u);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+  if (tid == 0) s_tile = atomicAdd(&ctr[0], 1u);
   __syncthreads();
   const uint32_t t = s_tile;
-  const bool mine = t * kLookbackSub + threadIdx.x / 256 < nsub;  // this thread's scan tile exists
-  const size_t base = (size_t)t * kLookbackThreads * 16 + threadIdx.x * 16;
+  if (zero && t == 0 && tid == 0) *zero = 0u;
+  const size_t base = (size_t)t * kScanTile + tid * 16;
   uint32_t v[16];
   uint32_t sum = 0;
-  if (mine) {
+  {
     const uint4* c4 = reinterpret_cast<const uint4*>(count + base);
 #pragma unroll
     for (int r = 0; r < 4; r++) {
@@ -237,244 +214,101 @@ __global__ void __launch_bounds__(kLookbackThreads) k_scan_lookback(uint32_t* __
 #pragma unroll
     for (int q = 0; q < 16; q++) sum += v[q];
   }
-  const uint32_t incl = block_incl_scan_big(sum, warp_tot);
-  if (threadIdx.x < 32) {
-    // warp 0: publish this supertile's sum, then look back 32 predecessors
-    // at a time (lane k reads supertile t-1-k; before 0 counts as an
-    // inclusive 0)
-    const uint32_t lane = threadIdx.x;
-    uint32_t total = 0;
-    for (uint32_t k = 0; k < kWarps; k++) total += warp_tot[k];
-    uint32_t excl = 0;
-    if (t == 0) {
-      if (lane == 0 && t != silent) atomicExch(&tstate[0], kTileIncl | total);
-    } else {
-      if (lane == 0 && t != silent) atomicExch(&tstate[t], kTileAgg | total);
-      __syncwarp();
-      volatile unsigned long long* vs = tstate;
-      int64_t top = (int64_t)t - 1;
-      uint32_t spins = 0;
-      for (;;) {
-        const int64_t idx = top - (int64_t)lane;
-        unsigned long long sv;
-        for (;;) {
-          sv = idx >= 0 ? (unsigned long long)vs[idx] : (unsigned long long)kTileIncl;
-          if (__all_sync(0xFFFFFFFFu, (sv >> 32) != 0ull)) break;
+  const uint32_t incl = block_incl_scan_256(sum, warp_tot);
+  uint32_t total = 0, excl = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) total += warp_tot[k];
+  if (tid == 0 && t != silent) atomicExch(&tstate[t], (t == 0 ? kTileIncl : kTileAgg) | total);
+  if (t != 0) {
+    volatile unsigned long long* vs = tstate;
+    uint32_t spins = 0;
+    for (int64_t top = (int64_t)t - 1;; top -= 256) {
+      // thread i reads predecessor top - i; before tile 0 counts as an inclusive 0
+      const int64_t idx = top - (int64_t)tid;
+      unsigned long long sv = kTileIncl;
+      if (idx >= 0) {
+        while (((sv = vs[idx]) >> 32) == 0ull) {
           if (++spins > kScanSpinLimit) {  // bounded: give up with a wrong prefix
-            if (lane == 0) atomicExch(err, 1u);
-            sv = (unsigned long long)kTileIncl;
+            atomicExch(err, 1u);
+            sv = kTileIncl;
             break;
           }
         }
-        const uint32_t flag = (uint32_t)(sv >> 32);
-        const uint32_t incl_lanes = __ballot_sync(0xFFFFFFFFu, flag == 2u);
-        // lanes up to the nearest inclusive prefix (all 32 if none)
-        const uint32_t upto = incl_lanes ? (uint32_t)(__ffs((int)incl_lanes) - 1) : 31u;
-        uint32_t val = lane <= upto ? (uint32_t)sv : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) val += __shfl_xor_sync(0xFFFFFFFFu, val, o);
-        excl += val;
-        if (incl_lanes) break;
-        top -= 32;
       }
-      if (lane == 0 && t != silent) atomicExch(&tstate[t], kTileIncl | (excl + total));
+      // predecessors up to the nearest inclusive prefix (all 256 if none)
+      const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (sv >> 32) == 2ull);
+      if (lane == 0) s_first[w] = inc ? w * 32u + (uint32_t)__ffs((int)inc) - 1u : 0xFFFFFFFFu;
+      __syncthreads();
+      uint32_t upto = 0xFFFFFFFFu;
+#pragma unroll
+      for (int k = 0; k < 8; k++) upto = min(upto, s_first[k]);
+      const uint32_t part = __reduce_add_sync(0xFFFFFFFFu, tid <= upto ? (uint32_t)sv : 0u);
+      if (lane == 0) s_sum[w] = part;
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 8; k++) excl += s_sum[k];
+      if (upto != 0xFFFFFFFFu) break;
     }
-    if (lane == 0) s_prefix = excl;
+    if (tid == 0 && t != silent) atomicExch(&tstate[t], kTileIncl | (excl + total));
   }
-  __syncthreads();
-  if (mine) {
-    uint32_t run = s_prefix + incl - sum;
+  {
+    uint32_t run = excl + incl - sum;
 #pragma unroll
     for (int q = 0; q < 16; q++) {
       const uint32_t x = v[q];
       v[q] = run;
       run += x;
     }
-    uint4* c4 = reinterpret_cast<uint4*>(count + base);
     uint4* s4 = reinterpret_cast<uint4*>(start + base);
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      const uint4 q = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
-      c4[r] = q;
-      s4[r] = q;  // the padded tail past the last key gets the particle count: never read
-    }
+    for (int r = 0; r < 4; r++)  // the padded tail past the last key gets the particle count: never read
+      s4[r] = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
   }
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     __threadfence();
     s_last = atomicAdd(&ctr[1], 1u) + 1u == gridDim.x;
   }
   __syncthreads();
   if (s_last) {
-    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) tstate[i] = 0ull;
-    if (threadIdx.x == 0) {
+    for (uint32_t i = tid; i < gridDim.x; i += 256u) tstate[i] = 0ull;
+    if (tid == 0) {
       ctr[0] = 0u;
       ctr[1] = 0u;
     }
   }
 }
 
-struct GatherArgs {
+// Writes a particle's sorted entries at final slot f.
+struct Gather2 {
   const float4* state;
   const float* mass;
   const uint8_t* phase;
-  float2* spos;
-  float2* svel;
-  float* smass;
-  uint8_t* sphase;
-  const uint32_t* pscene;  // batch: scene of each particle (id order), else null
-  uint32_t* sscene;
+  uint32_t *skey, *sid;
+  float2 *spos, *svel;
+  float* smass;            // null: uniform
+  uint8_t* sphase;         // null: uniform
+  const uint32_t* pscene;  // batch: scene of each particle (id order)
+  uint32_t* sscene;        // null: a single world
+  struct Row {
+    float4 st;
+    float m;
+    uint32_t sc;
+    uint8_t ph;
+  };
+  __device__ __forceinline__ Row load(uint32_t id) const {
+    return {state[id], smass ? mass[id] : 0.0f, sscene ? pscene[id] : 0u, sphase ? phase[id] : (uint8_t)0};
+  }
+  __device__ __forceinline__ void store(uint32_t f, uint32_t k, uint32_t id, const Row& r) const {
+    skey[f] = k;
+    sid[f] = id;
+    spos[f] = make_float2(r.st.x, r.st.y);
+    svel[f] = make_float2(r.st.z, r.st.w);
+    if (smass) smass[f] = r.m;
+    if (sphase) sphase[f] = r.ph;
+    if (sscene) sscene[f] = r.sc;
+  }
+  __device__ __forceinline__ void operator()(uint32_t f, uint32_t k, uint32_t id) const { store(f, k, id, load(id)); }
 };
-
-// The particle's sorted entries at final slot f (sid only when given: the
-// placement pass reads the previous sort's sid while it runs).
-__device__ __forceinline__ void gather_slot(uint32_t f, uint32_t k, uint32_t id, const GatherArgs& ga,
-                                            uint32_t* __restrict__ skey, uint32_t* __restrict__ sid) {
-  skey[f] = k;
-  if (sid) sid[f] = id;
-  const float4 st = ga.state[id];
-  ga.spos[f] = make_float2(st.x, st.y);
-  ga.svel[f] = make_float2(st.z, st.w);
-  if (ga.smass) ga.smass[f] = ga.mass[id];
-  if (ga.sphase) ga.sphase[f] = ga.phase[id];
-  if (ga.sscene) ga.sscene[f] = ga.pscene[id];
-}
-
-// tid entry of a slot whose particle k_place_final already put in its final
-// place (ids are below 2^31)
-constexpr uint32_t kPlacedFinal = 0x80000000u;
-
-// Placement for the 2D sort, with the common case finished in place: when a
-// run of equal keys in consecutive lanes is the whole bucket (its length
-// equals the bucket's count) and its ids ascend lane by lane, the run's
-// slots are already the final (key, id) order, so its particles are
-// gathered into sorted order here and their tid entries flagged; k_fixup
-// ranks only the other buckets and writes the flagged slots' sid (read here
-// as the previous order). Particles keep their cell from one substep
-// to the next almost always, and a bucket's particles arrive as one run in
-// the previous sort's order, so most buckets finish here.
-template <bool BY_SLOT>
-__global__ void __launch_bounds__(256) k_place_final(const uint32_t* __restrict__ key,
-                                                     const uint32_t* __restrict__ sid_prev, uint32_t n,
-                                                     uint32_t* __restrict__ cursor, const uint32_t* __restrict__ start,
-                                                     uint32_t* __restrict__ tkey, uint32_t* __restrict__ tid_out,
-                                                     uint32_t* __restrict__ skey, const uint32_t* __restrict__ order,
-                                                     GatherArgs ga) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t id = BY_SLOT ? sid_prev[s] : s;
-  const uint32_t k = key[id];
-  const uint32_t act = __activemask();  // a prefix of the warp's lanes
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t first, len, rank;
-  key_run(act, k, lane, &first, &len, &rank);
-  uint32_t base = 0;
-  if (first == lane) base = atomicAdd(&cursor[k], len);
-  base = __shfl_sync(act, base, first);
-  const uint32_t slot = base + rank;
-  const uint32_t tag = order ? __ldg(&order[id]) : id;
-  const uint32_t ptag = __shfl_sync(act, tag, lane ? lane - 1u : 0u);
-  const bool asc = lane == first || ptag < tag;
-  const uint32_t bad = __ballot_sync(act, !asc);
-  const uint32_t run = (len >= 32u ? 0xFFFFFFFFu : ((1u << len) - 1u)) << first;
-  if (len == __ldg(&start[k + 1]) - __ldg(&start[k]) && (bad & run) == 0u) {
-    gather_slot(slot, k, id, ga, skey, nullptr);
-    tid_out[slot] = id | kPlacedFinal;
-  } else {
-    tkey[slot] = k;
-    tid_out[slot] = id;
-  }
-}
-
-// Slot in the bucket from the cursor. BY_SLOT walks the previous sort's
-// order (keys nearly sorted: a warp holds few runs of equal keys, so few
-// atomics); otherwise particles are taken in id order.
-template <bool BY_SLOT>
-__global__ void __launch_bounds__(256) k_place(const uint32_t* __restrict__ key,
-                                               const uint32_t* __restrict__ sid_prev, uint32_t n,
-                                               uint32_t* __restrict__ cursor, uint32_t* __restrict__ tkey,
-                                               uint32_t* __restrict__ tid_out) {
-  const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= n) return;
-  const uint32_t id = BY_SLOT ? sid_prev[s] : s;
-  const uint32_t k = key[id];
-  // one atomic per run of equal keys in consecutive lanes; a run's lanes take
-  // consecutive slots (any order inside a bucket is fine: k_fixup ranks by id)
-  const uint32_t act = __activemask();
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t first, len, rank;
-  key_run(act, k, lane, &first, &len, &rank);
-  uint32_t base = 0;
-  if (first == lane) base = atomicAdd(&cursor[k], len);
-  base = __shfl_sync(act, base, first);
-  const uint32_t slot = base + rank;
-  tkey[slot] = k;
-  tid_out[slot] = id;
-}
-
-// Final slot = bucket start + rank of the id (or its order tag) among the
-// bucket's; the particle's state is gathered into that slot. With order
-// tags, the sentinel bucket of non-finite particles keeps its placement
-// slots: no walk visits it, and its size (a rank world's unused slots) would
-// make ranking quadratic.
-__device__ __forceinline__ void fixup_slot(uint32_t s, uint32_t id, const uint32_t* __restrict__ tkey,
-                                           const uint32_t* __restrict__ tid_in, const uint32_t* __restrict__ start,
-                                           uint32_t* __restrict__ skey, uint32_t* __restrict__ sid,
-                                           const uint32_t* __restrict__ order, uint32_t sentinel,
-                                           const GatherArgs& ga) {
-  if (id & kPlacedFinal) {  // k_place_final finished this bucket but its sid
-    sid[s] = id & ~kPlacedFinal;
-    return;
-  }
-  const uint32_t k = tkey[s];
-  const uint32_t lo = start[k], hi = start[k + 1];
-  uint32_t rank = 0;
-  if (order) {
-    if (k == sentinel) {
-      gather_slot(s, k, id, ga, skey, sid);
-      return;
-    }
-    const uint32_t tag = __ldg(&order[id]);
-    for (uint32_t j = lo; j < hi; j++) rank += __ldg(&order[__ldg(&tid_in[j])]) < tag ? 1u : 0u;
-  } else {
-    for (uint32_t j = lo; j < hi; j++) rank += __ldg(&tid_in[j]) < id ? 1u : 0u;
-  }
-  gather_slot(lo + rank, k, id, ga, skey, sid);
-}
-
-// SLOTS = 4: four slots per thread; where all four were finished by
-// k_place_final (the common case) one 16-byte load and store, the others one
-// by one. SLOTS = 1: one slot per thread. The same threads clear the bucket
-// counts for the next sort (the placement, which used them as cursors, has
-// finished): count_len is a multiple of the scan tile, so whole uint4 stores.
-template <int SLOTS>
-__global__ void __launch_bounds__(256) k_fixup(const uint32_t* __restrict__ tkey,
-                                               const uint32_t* __restrict__ tid_in,
-                                               const uint32_t* __restrict__ start, uint32_t n,
-                                               uint32_t* __restrict__ skey, uint32_t* __restrict__ sid,
-                                               const uint32_t* __restrict__ order, uint32_t sentinel,
-                                               uint32_t* __restrict__ count, uint32_t count_len, GatherArgs ga) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (4u * t < count_len) reinterpret_cast<uint4*>(count)[t] = make_uint4(0u, 0u, 0u, 0u);
-  if constexpr (SLOTS == 1) {
-    if (t < n) fixup_slot(t, tid_in[t], tkey, tid_in, start, skey, sid, order, sentinel, ga);
-    return;
-  }
-  const uint32_t s0 = 4u * t;
-  if (s0 >= n) return;
-  if (s0 + 3u < n) {
-    const uint4 v = *reinterpret_cast<const uint4*>(tid_in + s0);
-    if ((v.x & v.y & v.z & v.w) & kPlacedFinal) {
-      *reinterpret_cast<uint4*>(sid + s0) =
-          make_uint4(v.x & ~kPlacedFinal, v.y & ~kPlacedFinal, v.z & ~kPlacedFinal, v.w & ~kPlacedFinal);
-      return;
-    }
-    const uint32_t ids[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int q = 0; q < 4; q++) fixup_slot(s0 + q, ids[q], tkey, tid_in, start, skey, sid, order, sentinel, ga);
-    return;
-  }
-  for (uint32_t s = s0; s < n; s++) fixup_slot(s, tid_in[s], tkey, tid_in, start, skey, sid, order, sentinel, ga);
-}
 
 // ---------------------------------------------------------------- neighbour walk
 // Visit every candidate slot j of the particle in bucket `key`, in the
@@ -812,14 +646,17 @@ __device__ __forceinline__ uint32_t integrate_state(float2 pi, float2 vi, float 
 }
 
 // The integrate of the force passes: writes the new state, the next key and
-// its bucket count.
+// its bucket count, and the slot's id for the next sort (pid: its placement
+// walks this order while it writes sid).
 template <bool EXTRA = true>
-__device__ __forceinline__ void integrate_write(uint32_t id, float2 pi, float2 vi, float ax, float ay, float sx,
+__device__ __forceinline__ void integrate_write(uint32_t s, uint32_t id, uint32_t* __restrict__ pid, float2 pi,
+                                                float2 vi, float ax, float ay, float sx,
                                                 float sy, const StepParams& P, const DevBody* __restrict__ bodies,
                                                 float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
                                                 uint32_t* __restrict__ count_out,
                                                 uint32_t* __restrict__ defer = nullptr,
                                                 uint32_t* __restrict__ dcount = nullptr) {
+  pid[s] = id;
   float4 q;
   const uint32_t r = integrate_state<EXTRA>(pi, vi, ax, ay, sx, sy, P.dt, P, bodies, q);
   state_out[id] = q;
@@ -920,7 +757,7 @@ __global__ void __launch_bounds__(256) k_force_integrate(
     uint32_t n, const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
     uint32_t* __restrict__ count_out, float2* __restrict__ dbg_force, uint32_t* __restrict__ defer,
-    uint32_t* __restrict__ dcount) {
+    uint32_t* __restrict__ dcount, uint32_t* __restrict__ pid) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const StepParams& P = scene_params<BATCH>(P0, bt.ptab, BATCH ? bt.sscene[s] : 0u);
@@ -948,7 +785,7 @@ __global__ void __launch_bounds__(256) k_force_integrate(
   }
   const float ax = __fadd_rn(P.gx, __fdiv_rn(fx, rho_i));
   const float ay = __fadd_rn(P.gy, __fdiv_rn(fy, rho_i));
-  integrate_write<!PLAIN>(id, pi, vi, ax, ay, sx, sy, P, bodies, state_out, key_out, count_out, defer, dcount);
+  integrate_write<!PLAIN>(s, id, pid, pi, vi, ax, ay, sx, sy, P, bodies, state_out, key_out, count_out, defer, dcount);
 }
 
 // ---------------------------------------------------------------- closure force pass
@@ -977,7 +814,7 @@ __global__ void __launch_bounds__(256, 4) k_force_closure(
     const float* __restrict__ smass, const uint8_t* __restrict__ sphase, uint32_t n,
     const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, MlpDev mlp, ClosureIO io, float4* __restrict__ state_out,
-    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out) {
+    uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ pid) {
   extern __shared__ __align__(16) unsigned char closure_smem[];
   MlpSmem& sm = *reinterpret_cast<MlpSmem*>(closure_smem);
   __nv_bfloat16* sx_all = reinterpret_cast<__nv_bfloat16*>(closure_smem + sizeof(MlpSmem));
@@ -1044,7 +881,7 @@ __global__ void __launch_bounds__(256, 4) k_force_closure(
     io.rho_prev[id] = dqi.x;
     const float ax = __fadd_rn(__fadd_rn(P.gx, __fdiv_rn(fx, rho_i)), cx);
     const float ay = __fadd_rn(__fadd_rn(P.gy, __fdiv_rn(fy, rho_i)), cy);
-    integrate_write<!PLAIN>(id, pi, vi, ax, ay, sx, sy, P, bodies, state_out, key_out, count_out);
+    integrate_write<!PLAIN>(s, id, pid, pi, vi, ax, ay, sx, sy, P, bodies, state_out, key_out, count_out);
   }
 }
 
@@ -1211,30 +1048,26 @@ void enqueue_keys(const FluidBufs& b, uint32_t n, const GridPlan& g, cudaStream_
     k_keys<false><<<cdiv(n, 256), 256, 0, st>>>(b.state, n, g, b.batch, b.key, b.count);
 }
 
-// Bucket counts -> start table (count becomes the placement cursor).
+// Bucket counts -> start table.
 void enqueue_bucket_scan(const BucketSort& bs, uint32_t m, cudaStream_t st) {
   const uint32_t nt = cdiv(m, kScanTile);
   if (bs.tstate) {
-    k_scan_lookback<<<cdiv(nt, kLookbackSub), kLookbackThreads, 0, st>>>(bs.count, nt, bs.start, bs.tstate, bs.done,
-                                                                          bs.err, 0xFFFFFFFFu);
+    k_scan_lookback<<<nt, 256, 0, st>>>(bs.count, bs.start, bs.tstate, bs.done, bs.err, bs.list_n, 0xFFFFFFFFu);
   } else {
     k_scan_reduce<<<nt, 256, 0, st>>>(bs.count, bs.tilesum, nt, bs.done);
     k_scan_down<<<nt, 256, 0, st>>>(bs.count, bs.tilesum, m, bs.start);
   }
 }
 
-void enqueue_bucket_place(const BucketSort& bs, uint32_t n, uint32_t m, bool by_slot, cudaStream_t st) {
-  if (n == 0) return;
-  enqueue_bucket_scan(bs, m, st);
-  if (by_slot)
-    k_place<true><<<cdiv(n, 256), 256, 0, st>>>(bs.key, bs.sid_prev, n, bs.count, bs.tkey, bs.tid);
-  else
-    k_place<false><<<cdiv(n, 256), 256, 0, st>>>(bs.key, bs.sid_prev, n, bs.count, bs.tkey, bs.tid);
-}
-
 void enqueue_sort_and_ranges(const FluidBufs& b, uint32_t n, const StepParams& P, bool by_slot, cudaStream_t st) {
   if (n == 0) return;
   const uint32_t m = P.grid.sentinel + 1;  // all buckets and the non-finite sentinel
+  const Gather2 ga{b.state, b.mass, b.phase, b.skey, b.sid, b.spos, b.svel, (P.flags & F_MASS) ? b.smass : nullptr,
+                   (P.flags & F_PHASE) ? b.sphase : nullptr, b.batch.pscene, b.batch.ptab ? b.batch.sscene : nullptr};
+  if (!b.order && b.tstate && small_sort_applies(n, m)) {
+    launch_sort_small(b.key, n, m, b.start, b.count, b.count_len, ga, st);
+    return;
+  }
   BucketSort bs;
   bs.count = b.count;
   bs.tilesum = b.tilesum;
@@ -1243,38 +1076,13 @@ void enqueue_sort_and_ranges(const FluidBufs& b, uint32_t n, const StepParams& P
   bs.err = b.scan_err;
   bs.start = b.start;
   bs.key = b.key;
-  bs.sid_prev = b.sid;
+  bs.prev = b.pid;
   bs.tkey = b.tkey;
   bs.tid = b.tid;
-  GatherArgs ga;
-  ga.state = b.state;
-  ga.mass = b.mass;
-  ga.phase = b.phase;
-  ga.spos = b.spos;
-  ga.svel = b.svel;
-  ga.smass = (P.flags & F_MASS) ? b.smass : nullptr;
-  ga.sphase = (P.flags & F_PHASE) ? b.sphase : nullptr;
-  ga.pscene = b.batch.pscene;
-  ga.sscene = b.batch.ptab ? b.batch.sscene : nullptr;
-  enqueue_bucket_scan(bs, m, st);
-  if (by_slot)
-    k_place_final<true><<<cdiv(n, 256), 256, 0, st>>>(b.key, b.sid, n, b.count, b.start, b.tkey, b.tid, b.skey,
-                                                       b.order, ga);
-  else
-    k_place_final<false><<<cdiv(n, 256), 256, 0, st>>>(b.key, b.sid, n, b.count, b.start, b.tkey, b.tid, b.skey,
-                                                        b.order, ga);
-  // the fixup also clears the counts: the next sort's accumulate from zero
-  // (K6). Four slots per thread for one world (sort 31.6 against 32.1 us at
-  // 2^20 particles), one for a batch, whose many small buckets leave more
-  // slots to rank (sort 160 against 168 us for 512 scenes)
-  const uint32_t slots = b.batch.ptab ? 1u : 4u;
-  const uint32_t threads = std::max(cdiv(n, slots), cdiv(b.count_len, 4));
-  if (slots == 1)
-    k_fixup<1><<<cdiv(threads, 256), 256, 0, st>>>(b.tkey, b.tid, b.start, n, b.skey, b.sid, b.order, P.grid.sentinel,
-                                                   b.count, b.count_len, ga);
-  else
-    k_fixup<4><<<cdiv(threads, 256), 256, 0, st>>>(b.tkey, b.tid, b.start, n, b.skey, b.sid, b.order, P.grid.sentinel,
-                                                   b.count, b.count_len, ga);
+  bs.list = b.flist;
+  bs.list_n = b.flist_n;
+  bs.order = b.order;
+  enqueue_bucket_sort(bs, n, m, by_slot, ga, st);
 }
 
 // ---------------------------------------------------------------- adaptive resolution
@@ -1431,7 +1239,7 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
 #define PHIENG_FORCE_FAST_B(STG, D, BT, BAL)                                                                       \
   k_force_fast<STG, D, BT, BAL><<<g, bs, STG ? sm : 0, st>>>(b.spos, b.svel, b.sdq, b.skey, b.sid, n, b.start, P,  \
                                                              b.batch, b.bodies, b.nmask, b.state, b.key, b.count,  \
-                                                             dbg_force, b.defer, b.dcount)
+                                                             dbg_force, b.defer, b.dcount, b.pid)
 #define PHIENG_FORCE_FAST(STG, D, BT) PHIENG_FORCE_FAST_B(STG, D, BT, false)
     const bool stg = (b.stage & 2u) != 0;
     const bool bal = !stg && (b.stage & 4u) != 0;  // lanes balanced by neighbour count
@@ -1455,7 +1263,7 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
 #define PHIENG_FORCE(M, D, BT, PL)                                                                                  \
   k_force_integrate<M, D, BT, PL><<<g, bs, 0, st>>>(b.spos, b.svel, b.sdq, b.skey, b.sid, b.smass, n, b.start, P, \
                                                     b.batch, b.bodies, b.nmask, b.state, b.key, b.count, dbg_force, \
-                                                    b.defer, b.dcount)
+                                                    b.defer, b.dcount, b.pid)
   if (dbg_force) {
     if (m) PHIENG_FORCE(true, true, false, false);
     else PHIENG_FORCE(false, true, false, false);
@@ -1551,7 +1359,7 @@ void launch_closure(const FluidBufs& b, uint32_t n, const StepParams& P, const M
 #define PHIENG_CLOSURE_F(BT)                                                                                       \
   k_closure_fast<BT><<<cdiv(n, 256), 256, closure_smem_bytes(), st>>>(b.spos, b.svel, b.sdq, b.spres, b.skey,     \
                                                                       b.sid, n, b.start, P, b.batch, b.bodies,    \
-                                                                      b.nmask, mlp, io, b.state, b.key, b.count)
+                                                                      b.nmask, mlp, io, b.state, b.key, b.count, b.pid)
     if (bat) PHIENG_CLOSURE_F(true);
     else PHIENG_CLOSURE_F(false);
 #undef PHIENG_CLOSURE_F
@@ -1565,7 +1373,7 @@ void launch_closure(const FluidBufs& b, uint32_t n, const StepParams& P, const M
     const uint32_t blocks = min(cdiv(n, 128), (uint32_t)sms * 6u);
 #define PHIENG_CLOSURE_TC(BT)                                                                                       \
   k_closure_tc<BT><<<blocks, 128, kNetSmem, st>>>(b.spos, b.svel, b.sdq, b.spres, b.skey, b.sid, n, b.start, P,     \
-                                                  b.batch, b.bodies, b.nmask, mlp, io, b.state, b.key, b.count, io.err)
+                                                  b.batch, b.bodies, b.nmask, mlp, io, b.state, b.key, b.count, io.err, b.pid)
     if (bat) PHIENG_CLOSURE_TC(true);
     else PHIENG_CLOSURE_TC(false);
 #undef PHIENG_CLOSURE_TC
@@ -1576,7 +1384,7 @@ void launch_closure(const FluidBufs& b, uint32_t n, const StepParams& P, const M
 #define PHIENG_CLOSURE_V(M, PH, BT, PL)                                                                           \
   k_force_closure<M, PH, BT, PL, MODE><<<g, 256, sm, st>>>(b.spos, b.svel, b.sdq, b.spres, b.skey, b.sid,         \
                                                            b.smass, b.sphase, n, b.start, P, b.batch, b.bodies,   \
-                                                           b.nmask, mlp, io, b.state, b.key, b.count)
+                                                           b.nmask, mlp, io, b.state, b.key, b.count, b.pid)
 #define PHIENG_CLOSURE(M, PH, BT) PHIENG_CLOSURE_V(M, PH, BT, false)
   if (plain) {
     if (bat) PHIENG_CLOSURE_V(false, false, true, true);
@@ -1818,9 +1626,8 @@ void enqueue_buoyancy(const FluidBufs& b, const DynBufs& y, uint32_t n, const St
 
 void enqueue_scan_silent_tile(const FluidBufs& b, uint32_t m, cudaStream_t st) {
   const uint32_t nt = cdiv(m, kScanTile);
-  if (!b.tstate || cdiv(nt, kLookbackSub) < 2) return;
-  k_scan_lookback<<<cdiv(nt, kLookbackSub), kLookbackThreads, 0, st>>>(b.count, nt, b.start, b.tstate, b.done,
-                                                                        b.scan_err, 0u);
+  if (!b.tstate || nt < 2) return;
+  k_scan_lookback<<<nt, 256, 0, st>>>(b.count, b.start, b.tstate, b.done, b.scan_err, nullptr, 0u);
 }
 
 void enqueue_unsort_dp(const FluidBufs& b, uint32_t n, float* dens, float* pres, cudaStream_t st) {

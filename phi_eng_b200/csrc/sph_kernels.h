@@ -30,6 +30,9 @@ struct FluidBufs {
   uint32_t* tid = nullptr;
   uint32_t* skey = nullptr;  // sorted keys
   uint32_t* sid = nullptr;   // sorted slot -> particle id
+  uint32_t* pid = nullptr;   // the same as the last force pass left it: the next placement's order
+  uint32_t* flist = nullptr;    // placement slots left to k_fix_list, and their number
+  uint32_t* flist_n = nullptr;
   float2* spos = nullptr;    // sorted (x, y)
   float2* svel = nullptr;    // sorted (vx, vy)
   float* smass = nullptr;    // sorted mass (F_MASS)
@@ -44,7 +47,7 @@ struct FluidBufs {
   // sentinel bucket keeps its placement order (nothing visits it).
   uint32_t* order = nullptr;
   // per bucket grid (sized by the number of buckets B)
-  uint32_t* count = nullptr;    // particles per bucket, then the placement cursor
+  uint32_t* count = nullptr;    // particles per bucket; zero from a sort to the force pass after it
   uint32_t count_len = 0;       // B + 1 rounded up to the scan tile
   uint32_t* start = nullptr;    // bucket b holds sorted slots [start[b], start[b+1])
   uint32_t* tilesum = nullptr;  // scan tile sums / offsets
@@ -74,13 +77,6 @@ struct FluidBufs {
 
 // Scan tile of the bucket counts; count arrays are padded to a multiple.
 constexpr uint32_t kBucketScanTile = 4096;
-// Scan tiles per block of the single-pass (look-back) scan. One tile per
-// 256-thread block measured fastest on B200 for 2^20 buckets (9.7 us against
-// 12.0 us for four tiles per 1024-thread block and 13.9 us for four tiles
-// per 256-thread block): the shorter look-back chain of bigger blocks does
-// not make up for the SMs they leave idle.
-constexpr uint32_t kBucketScanSuper = 1;
-
 // K1: bucket key of every particle from its position (id order), and the
 // bucket counts the next sort starts from.
 void enqueue_keys(const FluidBufs& b, uint32_t n, const GridPlan& g, cudaStream_t st);
@@ -88,15 +84,12 @@ void enqueue_keys(const FluidBufs& b, uint32_t n, const GridPlan& g, cudaStream_
 // K2+K3+K4: counting sort of the particles by bucket key, ranked by id
 // inside each bucket (final order = (key, id)); fills the bucket range table
 // and gathers the particle state into sorted order.
-// by_slot: b.sid holds a permutation of [0, n) (the previous sort), walked
-// for locality; otherwise particles are placed in id order.
+// by_slot: b.pid holds a permutation of [0, n) (the ids in the slot order of
+// the last force pass), walked for locality; otherwise particles are placed in
+// id order.
 void enqueue_sort_and_ranges(const FluidBufs& b, uint32_t n, const StepParams& P, bool by_slot, cudaStream_t st);
 
-// The dimension-independent part of the bucket sort: scan the bucket counts
-// of keys [0, m) into the start table (count becomes the placement cursor),
-// then give every particle a slot inside its bucket (tkey / tid; the in-bucket
-// rank by id and the gather are the caller's). by_slot: sid_prev holds the
-// previous sort's order (walked for locality), else ids are taken in order.
+// The dimension-independent part of the bucket sort.
 struct BucketSort {
   uint32_t* count = nullptr;
   uint32_t* tilesum = nullptr;
@@ -105,11 +98,16 @@ struct BucketSort {
   uint32_t* err = nullptr;
   uint32_t* start = nullptr;
   const uint32_t* key = nullptr;
-  const uint32_t* sid_prev = nullptr;
+  const uint32_t* prev = nullptr;  // by_slot: the order to walk
   uint32_t* tkey = nullptr;
   uint32_t* tid = nullptr;
+  uint32_t* list = nullptr;  // by_slot: slots left to rank, and their number
+  uint32_t* list_n = nullptr;
+  const uint32_t* order = nullptr;
 };
-void enqueue_bucket_place(const BucketSort& bs, uint32_t n, uint32_t m, bool by_slot, cudaStream_t st);
+
+// Scan of the bucket counts of keys [0, m) into the start table.
+void enqueue_bucket_scan(const BucketSort& bs, uint32_t m, cudaStream_t st);
 
 // Adaptive resolution scratch: inverse sort permutation, merge flags, the
 // resampled particles (cap rows; a pass over n particles writes at most

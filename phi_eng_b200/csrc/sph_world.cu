@@ -81,7 +81,7 @@ struct World2 {
   bool keys_valid = false;   // key[] and the bucket counts match the state
   bool plan_valid = false;
   bool plan_locked = false;  // set by phieng_sph_set_grid: no automatic replan
-  uint32_t sid_perm_n = 0;   // d.sid is a permutation of [0, sid_perm_n)
+  uint32_t sid_perm_n = 0;   // d.pid is a permutation of [0, sid_perm_n)
   GridPlan plan{};
 
   int device = -1;
@@ -218,6 +218,8 @@ void free_particle_buffers(FluidBufs& d) {
   dfree(d.tid);
   dfree(d.skey);
   dfree(d.sid);
+  dfree(d.pid);
+  dfree(d.flist);
   dfree(d.spos);
   dfree(d.svel);
   dfree(d.smass);
@@ -254,6 +256,7 @@ bool ensure_device(World2* w) {
   if (!cuda_ok(w, cudaMalloc(&w->d.scalar, 128), "cudaMalloc(scalar)")) return false;
   if (!cuda_ok(w, cudaMemset(w->d.scalar, 0, 128), "cudaMemset(scalar)")) return false;
   w->d.done = w->d.scalar + 8;       // scan counters [8], [9]
+  w->d.flist_n = w->d.scalar + 25;
   w->d.scan_err = w->d.scalar + 12;  // set when a scan's look-back wait or a tensor-core wait gave up
   if (!cuda_ok(w, cudaMallocHost(&w->h_pinned, 64), "cudaMallocHost")) return false;
   w->device = dev;
@@ -274,7 +277,8 @@ bool ensure_capacity(World2* w, uint32_t need) {
   uint32_t c = std::max<uint32_t>(need, 1024);
   bool ok = dalloc(w, d.state, c) && dalloc(w, d.mass, c) && dalloc(w, d.phase, c) && dalloc(w, d.key, c) &&
             dalloc(w, d.tkey, c) && dalloc(w, d.tid, c) &&
-            dalloc(w, d.skey, c) && dalloc(w, d.sid, c) && dalloc(w, d.spos, (size_t)c + 1) && dalloc(w, d.svel, c) &&
+            dalloc(w, d.skey, c) && dalloc(w, d.sid, c) && dalloc(w, d.pid, c) && dalloc(w, d.flist, c) &&
+            dalloc(w, d.spos, (size_t)c + 1) && dalloc(w, d.svel, c) &&
             dalloc(w, d.smass, c) && dalloc(w, d.sphase, c) && dalloc(w, d.sdq, c) && dalloc(w, d.spres, c) &&
             dalloc(w, d.nmask, 3 * (size_t)c);
   if (ok && w->is_batch()) {
@@ -1004,7 +1008,6 @@ bool run_substep_adaptive(World2* w, float dt) {
   cudaStream_t st = w->stream;
   StepParams P = make_params(w, dt);
   enqueue_sort_and_ranges(w->d, w->n, P, w->sid_perm_n == w->n, st);
-  w->sid_perm_n = w->n;
   enqueue_density(w->d, w->n, P, st);
   const FluidConfig2Ffi& c = w->cfg;
   const float rest = std::max(c.rest_density, kEps);
@@ -1045,10 +1048,10 @@ bool run_substep_adaptive(World2* w, float dt) {
   P = make_params(w, dt);
   enqueue_keys(w->d, w->n, w->plan, st);
   enqueue_sort_and_ranges(w->d, w->n, P, false, st);
-  w->sid_perm_n = w->n;
   enqueue_density(w->d, w->n, P, st);
   enqueue_ghost_density(w->d, P, st);
   enqueue_force_integrate(w->d, w->n, P, nullptr, st);
+  w->sid_perm_n = w->n;
   if (!cuda_ok(w, cudaGetLastError(), "adaptive substep")) return false;
   w->substeps++;
   w->dp_on_device = true;
@@ -1079,7 +1082,6 @@ bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
     w->substeps_pending = true;
   else
     w->substeps += ss.steps;
-  w->sid_perm_n = w->n;
   w->host_state_valid = false;
   w->dp_on_device = true;
   w->keys_valid = true;
@@ -1406,11 +1408,11 @@ bool step_fluid_bodies(World2* w, PhiengBody2* bodies, uint32_t nb, float dt, co
   const size_t dlen = (size_t)((w->n + 1 + kBucketScanTile - 1) / kBucketScanTile) * kBucketScanTile;
   for (uint32_t k = 0; k < ns; k++) {
     enqueue_sort_and_ranges(dB, w->n, P, w->sid_perm_n == w->n, st);
-    w->sid_perm_n = w->n;
     enqueue_density(dB, w->n, P, st);
     enqueue_ghost_density(dB, P, st);
     if (any_dyn) cudaMemsetAsync(dB.dcount, 0, sizeof(uint32_t) * dlen, st);
     enqueue_force_integrate(dB, w->n, P, nullptr, st);
+    w->sid_perm_n = w->n;
     if (any_dyn) enqueue_dynamic_walls(dB, y, w->n, P, st);
     if (y.nbuoy) enqueue_buoyancy(dB, y, w->n, P, drag, sub, st);
     w->substeps++;
@@ -1456,7 +1458,6 @@ bool ensure_closure_buffers(World2* w) {
 void enqueue_sort_density(World2* w, const StepParams& P, float2* svp = nullptr) {
   enqueue_sort_and_ranges(w->d, w->n, P, w->sid_perm_n == w->n, w->stream);
   enqueue_density(w->d, w->n, P, w->stream, svp);
-  w->sid_perm_n = w->n;
   w->dp_on_device = true;
 }
 
@@ -2462,10 +2463,10 @@ int32_t phieng_sph_debug_scan_timeout(World2* w) {
   if (!w || !prepare(w)) return 0;
   const uint32_t m = w->plan.sentinel + 1;
   // at least two look-back blocks
-  if ((m + kBucketScanTile * kBucketScanSuper - 1) / (kBucketScanTile * kBucketScanSuper) < 2) return 0;
+  if ((m + kBucketScanTile - 1) / kBucketScanTile < 2) return 0;
   enqueue_scan_silent_tile(w->d, m, w->stream);
   if (!cuda_ok(w, cudaGetLastError(), "scan")) return 0;
-  w->keys_valid = false;  // the counts became cursors
+  w->keys_valid = false;  // the range table is wrong
   return scan_flag_ok(w) ? 1 : 0;
 }
 
@@ -2476,7 +2477,6 @@ uint32_t phieng_sph_debug_sorted(World2* w, uint32_t* ids, uint32_t* keys, uint3
   const StepParams P = make_params(w, 0.0f);
   enqueue_keys(w->d, w->n, w->plan, w->stream);
   enqueue_sort_and_ranges(w->d, w->n, P, false, w->stream);
-  w->sid_perm_n = w->n;
   w->keys_valid = false;  // the sort consumed the bucket counts
   uint32_t n = std::min(max, w->n);
   if (ids) cudaMemcpyAsync(ids, w->d.sid, 4ull * n, cudaMemcpyDeviceToHost, w->stream);
@@ -2492,7 +2492,6 @@ uint32_t phieng_sph_debug_neighbors(World2* w, uint32_t* counts, uint32_t* lists
   const StepParams P = make_params(w, 0.0f);
   enqueue_keys(w->d, w->n, w->plan, w->stream);
   enqueue_sort_and_ranges(w->d, w->n, P, false, w->stream);
-  w->sid_perm_n = w->n;
   w->keys_valid = false;  // the sort consumed the bucket counts
   size_t bytes = 4ull * w->n * (1 + (size_t)max_per);
   if (!ensure_tmp(w, bytes)) return 0;
@@ -2512,7 +2511,6 @@ uint32_t phieng_sph_debug_forces(World2* w, float* fxy, uint32_t max) {
   const StepParams P = make_params(w, 0.0f);
   enqueue_keys(w->d, w->n, w->plan, w->stream);
   enqueue_sort_and_ranges(w->d, w->n, P, false, w->stream);
-  w->sid_perm_n = w->n;
   w->keys_valid = false;  // the sort consumed the bucket counts
   enqueue_density(w->d, w->n, P, w->stream);
   if (!ensure_tmp(w, sizeof(float2) * (size_t)w->n)) return 0;
