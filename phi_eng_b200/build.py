@@ -37,7 +37,7 @@ UNITS = [
 ]
 HEADERS = ["sph_device.cuh", "sph_kernels.h", "sph_mlp.cuh", "sph_mlp_host.h", "sph_warp.cuh", "sph_host.h", "sph_snapshot.h",
            "sph_noise.cuh", "sph_fast.cuh", "sph_tc.cuh", "sph_tc_net.cuh",
-           "sph_closure_tc.cuh", "sph_sort_small.cuh", "sph_sort_runs.cuh", "sph3d_coop.cuh", "sph_small.cuh"]
+           "sph_closure_tc.cuh", "sph_sort_small.cuh", "sph_sort_runs.cuh", "sph_chain.cuh", "sph3d_coop.cuh", "sph_small.cuh"]
 
 
 def _mtime(p: str) -> float:

@@ -710,6 +710,7 @@ __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spo
                                                   const uint32_t* __restrict__ sq, StepParams3 P,
                                                   float2* __restrict__ sdq, float* __restrict__ spres,
                                                   uint32_t* __restrict__ nmask) {
+  chain_wait(spos, skey, smass, sphase, start, sq);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t k = skey[s];
@@ -1189,6 +1190,7 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
                                                 float4* __restrict__ vel_out, uint32_t* __restrict__ key_out,
                                                 uint32_t* __restrict__ count_out, float4* __restrict__ dbg,
                                                 uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, skey, sid, smass, start, bodies, nmask);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const uint32_t k = skey[s];
@@ -2054,7 +2056,7 @@ void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
   const bool wide = (P.flags & F_WIDE_NB) != 0;
   if (w->n <= kRowsMax3) {
 #define PHIENG_D3C(M, PH, WD)                                                                                \
-  k_density3_rows<M, PH, WD><<<cdiv(w->n, 32), 288, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, \
+  launch_chained(k_density3_rows<M, PH, WD>, cdiv(w->n, 32), 288, 0, st, w->spos, w->skey, w->smass, w->sphase, w->n, \
                                                              w->start, w->sq, P, w->sdq, w->spres, w->nmask)
 #define PHIENG_D3G(M, PH)                       \
   do {                                          \
@@ -2072,10 +2074,10 @@ void enqueue_density3(World3* w, const StepParams3& P, cudaStream_t st) {
 #define PHIENG_D3(M, PH)                                                                                     \
   do {                                                                                                       \
     if (wide)                                                                                                \
-      k_density3<M, PH, true><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P,  \
+      launch_chained(k_density3<M, PH, true>, g, 256, 0, st, w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P,  \
                                                  w->sdq, w->spres, w->nmask);                                \
     else                                                                                                     \
-      k_density3<M, PH, false><<<g, 256, 0, st>>>(w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P, \
+      launch_chained(k_density3<M, PH, false>, g, 256, 0, st, w->spos, w->skey, w->smass, w->sphase, w->n, w->start, w->sq, P, \
                                                   w->sdq, w->spres, w->nmask);                               \
   } while (0)
   if (m && ph) PHIENG_D3(true, true);
@@ -2095,7 +2097,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
   const bool fast = plain && !m && (P.flags & F_FAST);
   if (w->n <= (fast ? kCoopMaxFast3 : kCoopMax3)) {
 #define PHIENG_F3G(M, D, PL, FA)                                                                           \
-  k_force3_coop<M, D, PL, FA><<<cdiv(w->n, kCoopThreads / kCoopLanes), kCoopThreads, 0, st>>>(             \
+  launch_chained(k_force3_coop<M, D, PL, FA>, cdiv(w->n, kCoopThreads / kCoopLanes), kCoopThreads, 0, st,  \
       w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, P, w->dbodies, w->nmask, w->pos, \
       w->vel, w->key, w->count, dbg, w->pid)
     if (fast) {
@@ -2115,7 +2117,7 @@ void enqueue_force3(World3* w, const StepParams3& P, float4* dbg, cudaStream_t s
     return;
   }
 #define PHIENG_F3X(M, D, PL, FA)                                                                                    \
-  k_force3<M, D, PL, FA><<<g, kForceThreads3, 0, st>>>(w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
+  launch_chained(k_force3<M, D, PL, FA>, g, kForceThreads3, 0, st, w->spos, w->svel, w->sdq, w->skey, w->sid, w->smass, w->n, w->start, \
                                             P, w->dbodies, w->nmask, w->pos, w->vel, w->key, w->count, dbg, w->pid)
 #define PHIENG_F3(M, D, PL) PHIENG_F3X(M, D, PL, false)
   if (fast) {

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
                                                        const uint32_t* __restrict__ sq, StepParams3 P,
                                                        float2* __restrict__ sdq, float* __restrict__ spres,
                                                        uint32_t* __restrict__ nmask) {
+  chain_wait(spos, skey, smass, sphase, start, sq);
   __shared__ float terms[9][kRowTerms][32];
   __shared__ uint32_t row_cnt[9][32];  // neighbours of the row; bits 30, 31: it has a second word, no mask
   const uint32_t p = threadIdx.x & 31u, r = threadIdx.x >> 5;
@@ -133,6 +134,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_force3_coop(
     const uint32_t* __restrict__ nmask, float4* __restrict__ pos_out,
     float4* __restrict__ vel_out, uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out,
     float4* __restrict__ dbg, uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, skey, sid, smass, start, bodies, nmask);
   constexpr int G = kCoopLanes;
   static_assert(G == 8, "six lanes of a group hold the sums; lanes 0..7 expand rows 0..7");
   constexpr uint32_t kAll = 0xFFFFFFFFu, kGroups = kCoopThreads / G;

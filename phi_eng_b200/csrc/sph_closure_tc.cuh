@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(128, 6) k_closure_tc(
     const uint32_t* __restrict__ nmask, MlpDev mlp, ClosureIO io, float4* __restrict__ state_out,
     uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ err,
     uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, spres, skey, sid, start, bodies, nmask);
   extern __shared__ __align__(1024) unsigned char net_smem[];
   TcNet net = tc_net_init(net_smem, mlp);
   bool ok = true;
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(256, 4) k_closure_fast(
     const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
     const uint32_t* __restrict__ nmask, MlpDev mlp, ClosureIO io, float4* __restrict__ state_out,
     uint32_t* __restrict__ key_out, uint32_t* __restrict__ count_out, uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, spres, skey, sid, start, bodies, nmask);
   extern __shared__ __align__(16) unsigned char closure_smem[];
   MlpSmem& sm = *reinterpret_cast<MlpSmem*>(closure_smem);
   __nv_bfloat16* sx_all = reinterpret_cast<__nv_bfloat16*>(closure_smem + sizeof(MlpSmem));

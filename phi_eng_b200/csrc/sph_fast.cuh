@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(256) k_force_fast(
     const uint32_t* __restrict__ nmask, float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
     uint32_t* __restrict__ count_out, float2* __restrict__ dbg_force, uint32_t* __restrict__ defer,
     uint32_t* __restrict__ dcount, uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, skey, sid, start, bodies, nmask);
   static_assert(!(STAGE && BALANCE), "staging windows assume the block's own slot order");
   extern __shared__ __align__(16) float2 fast_win[];
   const uint32_t s = BALANCE ? balanced_slot(nmask, n) : blockIdx.x * blockDim.x + threadIdx.x;

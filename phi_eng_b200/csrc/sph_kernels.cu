@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(256) k_scan_lookback(const uint32_t* __restric
                                                        unsigned long long* __restrict__ tstate,
                                                        uint32_t* __restrict__ ctr, uint32_t* __restrict__ err,
                                                        uint32_t* __restrict__ zero, uint32_t silent) {
+  chain_wait(count, tstate, ctr);
   __shared__ uint32_t warp_tot[8];
   __shared__ uint32_t s_tile, s_first[8], s_sum[8];
   __shared__ bool s_last;
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(256) k_density(const float2* __restrict__ spos
                                                  const uint32_t* __restrict__ start, StepParams P0, BatchTab bt,
                                                  float2* __restrict__ sdq, float* __restrict__ spres,
                                                  uint32_t* __restrict__ nmask, float2* __restrict__ svp) {
+  chain_wait(spos, skey, smass, sphase, start);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const StepParams& P = scene_params<BATCH>(P0, bt.ptab, BATCH ? bt.sscene[s] : 0u);
@@ -758,6 +760,7 @@ __global__ void __launch_bounds__(256) k_force_integrate(
     const uint32_t* __restrict__ nmask, float4* __restrict__ state_out, uint32_t* __restrict__ key_out,
     uint32_t* __restrict__ count_out, float2* __restrict__ dbg_force, uint32_t* __restrict__ defer,
     uint32_t* __restrict__ dcount, uint32_t* __restrict__ pid) {
+  chain_wait(spos, svel, sdq, skey, sid, smass, start, bodies, nmask);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
   const StepParams& P = scene_params<BATCH>(P0, bt.ptab, BATCH ? bt.sscene[s] : 0u);
@@ -1052,7 +1055,8 @@ void enqueue_keys(const FluidBufs& b, uint32_t n, const GridPlan& g, cudaStream_
 void enqueue_bucket_scan(const BucketSort& bs, uint32_t m, cudaStream_t st) {
   const uint32_t nt = cdiv(m, kScanTile);
   if (bs.tstate) {
-    k_scan_lookback<<<nt, 256, 0, st>>>(bs.count, bs.start, bs.tstate, bs.done, bs.err, bs.list_n, 0xFFFFFFFFu);
+    launch_chained(k_scan_lookback, nt, 256, 0, st, bs.count, bs.start, bs.tstate, bs.done, bs.err, bs.list_n,
+                   0xFFFFFFFFu);
   } else {
     k_scan_reduce<<<nt, 256, 0, st>>>(bs.count, bs.tilesum, nt, bs.done);
     k_scan_down<<<nt, 256, 0, st>>>(bs.count, bs.tilesum, m, bs.start);
@@ -1205,8 +1209,8 @@ void enqueue_density(const FluidBufs& b, uint32_t n, const StepParams& P, cudaSt
     return;
   }
 #define PHIENG_DENSITY(M, PH, BT, HE)                                                                          \
-  k_density<M, PH, BT, HE><<<g, bs, 0, st>>>(b.spos, b.skey, b.smass, b.sphase, n, b.start, P, b.batch, b.sdq, \
-                                             b.spres, b.nmask, svp)
+  launch_chained(k_density<M, PH, BT, HE>, g, bs, 0, st, b.spos, b.skey, b.smass, b.sphase, n, b.start, P,     \
+                 b.batch, b.sdq, b.spres, b.nmask, svp)
 #define PHIENG_DENSITY_W(M, PH, BT)       \
   do {                                    \
     if (heq)                              \
@@ -1237,7 +1241,7 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
   if (fast_flags(P.flags)) {
     const size_t sm = 9 * fast_stage_cap(bs) * sizeof(float2);
 #define PHIENG_FORCE_FAST_B(STG, D, BT, BAL)                                                                       \
-  k_force_fast<STG, D, BT, BAL><<<g, bs, STG ? sm : 0, st>>>(b.spos, b.svel, b.sdq, b.skey, b.sid, n, b.start, P,  \
+  launch_chained(k_force_fast<STG, D, BT, BAL>, g, bs, STG ? sm : 0, st, b.spos, b.svel, b.sdq, b.skey, b.sid, n, b.start, P,  \
                                                              b.batch, b.bodies, b.nmask, b.state, b.key, b.count,  \
                                                              dbg_force, b.defer, b.dcount, b.pid)
 #define PHIENG_FORCE_FAST(STG, D, BT) PHIENG_FORCE_FAST_B(STG, D, BT, false)
@@ -1261,7 +1265,7 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
     return;
   }
 #define PHIENG_FORCE(M, D, BT, PL)                                                                                  \
-  k_force_integrate<M, D, BT, PL><<<g, bs, 0, st>>>(b.spos, b.svel, b.sdq, b.skey, b.sid, b.smass, n, b.start, P, \
+  launch_chained(k_force_integrate<M, D, BT, PL>, g, bs, 0, st, b.spos, b.svel, b.sdq, b.skey, b.sid, b.smass, n, b.start, P, \
                                                     b.batch, b.bodies, b.nmask, b.state, b.key, b.count, dbg_force, \
                                                     b.defer, b.dcount, b.pid)
   if (dbg_force) {
@@ -1357,7 +1361,7 @@ void launch_closure(const FluidBufs& b, uint32_t n, const StepParams& P, const M
   if (MODE == kModeClosure && fast_flags(P.flags) && mlp.engine == kMlpInferMmaSync) {
     // tolerance mode, network on mma.sync warp tiles
 #define PHIENG_CLOSURE_F(BT)                                                                                       \
-  k_closure_fast<BT><<<cdiv(n, 256), 256, closure_smem_bytes(), st>>>(b.spos, b.svel, b.sdq, b.spres, b.skey,     \
+  launch_chained(k_closure_fast<BT>, cdiv(n, 256), 256, closure_smem_bytes(), st, b.spos, b.svel, b.sdq, b.spres, b.skey,     \
                                                                       b.sid, n, b.start, P, b.batch, b.bodies,    \
                                                                       b.nmask, mlp, io, b.state, b.key, b.count, b.pid)
     if (bat) PHIENG_CLOSURE_F(true);
@@ -1372,7 +1376,7 @@ void launch_closure(const FluidBufs& b, uint32_t n, const StepParams& P, const M
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t blocks = min(cdiv(n, 128), (uint32_t)sms * 6u);
 #define PHIENG_CLOSURE_TC(BT)                                                                                       \
-  k_closure_tc<BT><<<blocks, 128, kNetSmem, st>>>(b.spos, b.svel, b.sdq, b.spres, b.skey, b.sid, n, b.start, P,     \
+  launch_chained(k_closure_tc<BT>, blocks, 128, kNetSmem, st, b.spos, b.svel, b.sdq, b.spres, b.skey, b.sid, n, b.start, P,     \
                                                   b.batch, b.bodies, b.nmask, mlp, io, b.state, b.key, b.count, io.err, b.pid)
     if (bat) PHIENG_CLOSURE_TC(true);
     else PHIENG_CLOSURE_TC(false);
@@ -1627,7 +1631,7 @@ void enqueue_buoyancy(const FluidBufs& b, const DynBufs& y, uint32_t n, const St
 void enqueue_scan_silent_tile(const FluidBufs& b, uint32_t m, cudaStream_t st) {
   const uint32_t nt = cdiv(m, kScanTile);
   if (!b.tstate || nt < 2) return;
-  k_scan_lookback<<<nt, 256, 0, st>>>(b.count, b.start, b.tstate, b.done, b.scan_err, nullptr, 0u);
+  launch_chained(k_scan_lookback, nt, 256, 0, st, b.count, b.start, b.tstate, b.done, b.scan_err, nullptr, 0u);
 }
 
 void enqueue_unsort_dp(const FluidBufs& b, uint32_t n, float* dens, float* pres, cudaStream_t st) {

@@ -9,6 +9,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sph_chain.cuh"
 #include "sph_kernels.h"
 #include "sph_warp.cuh"
 
@@ -47,6 +48,7 @@ __global__ void __launch_bounds__(256) k_place_runs(const uint32_t* __restrict__
   __shared__ uint32_t s_key[kSpan], s_tag[kSpan];
   __shared__ uint32_t s_head[kWords], s_fall[kWords];
   __shared__ uint32_t s_open, s_base;
+  chain_wait(key, prev, start, order);
   const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
   const uint32_t s = blockIdx.x * 256u + t, i = t + kRunMax;
   if (t == 0) s_open = 0u;
@@ -58,9 +60,9 @@ __global__ void __launch_bounds__(256) k_place_runs(const uint32_t* __restrict__
     id = prev[s];
     k = key[id];
     row = ga.load(id);
-    tag = order ? __ldg(&order[id]) : id;
-    lo = __ldg(&start[k]);
-    hi = __ldg(&start[k + 1]);
+    tag = order ? order[id] : id;
+    lo = start[k];
+    hi = start[k + 1];
   }
   s_key[i] = k;
   s_tag[i] = tag;
@@ -71,7 +73,7 @@ __global__ void __launch_bounds__(256) k_place_runs(const uint32_t* __restrict__
     if (sh < n) {
       th = prev[sh];
       kh = key[th];
-      if (order) th = __ldg(&order[th]);
+      if (order) th = order[th];
     }
     s_key[ih] = kh;
     s_tag[ih] = th;
@@ -148,6 +150,7 @@ __global__ void __launch_bounds__(256) k_place_runs(const uint32_t* __restrict__
 static __global__ void __launch_bounds__(256) k_place_all(const uint32_t* __restrict__ key, uint32_t n,
                                                    uint32_t* __restrict__ count, const uint32_t* __restrict__ start,
                                                    uint32_t* __restrict__ tkey, uint32_t* __restrict__ tid_out) {
+  chain_wait(key, start);
   const uint32_t id = blockIdx.x * blockDim.x + threadIdx.x;
   if (id >= n) return;
   const uint32_t k = key[id];
@@ -159,7 +162,7 @@ static __global__ void __launch_bounds__(256) k_place_all(const uint32_t* __rest
   uint32_t left = 0;
   if (first == lane) left = atomicSub(&count[k], len);
   left = __shfl_sync(act, left, first);
-  const uint32_t slot = __ldg(&start[k]) + left - len + rank;
+  const uint32_t slot = start[k] + left - len + rank;
   tkey[slot] = k;
   tid_out[slot] = id;
 }
@@ -180,10 +183,10 @@ __device__ __forceinline__ void fix_slot(uint32_t s, const uint32_t* __restrict_
   const uint32_t lo = start[k], hi = start[k + 1];
   uint32_t rank = 0;
   if (order) {
-    const uint32_t tag = __ldg(&order[id]);
-    for (uint32_t j = lo; j < hi; j++) rank += __ldg(&order[__ldg(&tid_in[j])]) < tag ? 1u : 0u;
+    const uint32_t tag = order[id];
+    for (uint32_t j = lo; j < hi; j++) rank += order[tid_in[j]] < tag ? 1u : 0u;
   } else {
-    for (uint32_t j = lo; j < hi; j++) rank += __ldg(&tid_in[j]) < id ? 1u : 0u;
+    for (uint32_t j = lo; j < hi; j++) rank += tid_in[j] < id ? 1u : 0u;
   }
   ga(lo + rank, k, id);
 }
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(256) k_fix_list(const uint32_t* __restrict__ l
                                                   const uint32_t* __restrict__ tid_in,
                                                   const uint32_t* __restrict__ start,
                                                   const uint32_t* __restrict__ order, uint32_t sentinel, Gather ga) {
+  chain_wait(list, list_n, tkey, tid_in, start, order);
   const uint32_t m = *list_n;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
     fix_slot(list[i], tkey, tid_in, start, order, sentinel, ga);
@@ -205,6 +209,7 @@ __global__ void __launch_bounds__(256) k_fix_all(uint32_t n, const uint32_t* __r
                                                  const uint32_t* __restrict__ tid_in,
                                                  const uint32_t* __restrict__ start,
                                                  const uint32_t* __restrict__ order, uint32_t sentinel, Gather ga) {
+  chain_wait(tkey, tid_in, start, order);
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) fix_slot(s, tkey, tid_in, start, order, sentinel, ga);
 }
@@ -217,13 +222,13 @@ inline void enqueue_bucket_sort(const BucketSort& bs, uint32_t n, uint32_t m, bo
   const uint32_t blocks = (n + 255u) / 256u;
   enqueue_bucket_scan(bs, m, st);
   if (by_slot) {
-    k_place_runs<<<blocks, 256, 0, st>>>(bs.key, bs.prev, n, bs.count, bs.start, bs.order, bs.tkey, bs.tid, bs.list,
-                                         bs.list_n, m - 1u, ga);
-    k_fix_list<<<blocks < 592u ? blocks : 592u, 256, 0, st>>>(bs.list, bs.list_n, bs.tkey, bs.tid, bs.start, bs.order,
-                                                              m - 1u, ga);
+    launch_chained(k_place_runs<Gather>, blocks, 256, 0, st, bs.key, bs.prev, n, bs.count, bs.start, bs.order, bs.tkey,
+                   bs.tid, bs.list, bs.list_n, m - 1u, ga);
+    launch_chained(k_fix_list<Gather>, blocks < 592u ? blocks : 592u, 256, 0, st, bs.list, bs.list_n, bs.tkey, bs.tid,
+                   bs.start, bs.order, m - 1u, ga);
   } else {
-    k_place_all<<<blocks, 256, 0, st>>>(bs.key, n, bs.count, bs.start, bs.tkey, bs.tid);
-    k_fix_all<<<blocks, 256, 0, st>>>(n, bs.tkey, bs.tid, bs.start, bs.order, m - 1u, ga);
+    launch_chained(k_place_all, blocks, 256, 0, st, bs.key, n, bs.count, bs.start, bs.tkey, bs.tid);
+    launch_chained(k_fix_all<Gather>, blocks, 256, 0, st, n, bs.tkey, bs.tid, bs.start, bs.order, m - 1u, ga);
   }
 }
 

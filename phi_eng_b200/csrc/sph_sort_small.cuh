@@ -18,6 +18,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "sph_chain.cuh"
+
 namespace phieng {
 
 constexpr uint32_t kSmallSortMax = 8192;      // particles: eight per thread
@@ -40,6 +42,7 @@ template <class Gather>
 __global__ void __launch_bounds__(1024) k_sort_small(const uint32_t* __restrict__ key, uint32_t n, uint32_t m,
                                                      uint32_t* __restrict__ start, uint32_t* __restrict__ count,
                                                      uint32_t count_len, Gather ga) {
+  chain_wait(key);
   extern __shared__ uint32_t sort_small_smem[];
   __shared__ uint32_t warp_tot[32];
   constexpr int kPer = kSmallSortMax / 1024;
@@ -122,7 +125,8 @@ inline void launch_sort_small(const uint32_t* key, uint32_t n, uint32_t m, uint3
                               uint32_t count_len, const Gather& ga, cudaStream_t st) {
   const size_t smem = small_sort_smem(n, m);
   cudaFuncSetAttribute(k_sort_small<Gather>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_sort_small<Gather><<<std::max<uint32_t>(1u, (n + 1023u) / 1024u * 4u), 1024, smem, st>>>(key, n, m, start, count, count_len, ga);
+  launch_chained(k_sort_small<Gather>, std::max<uint32_t>(1u, (n + 1023u) / 1024u * 4u), 1024, smem, st, key, n, m,
+                 start, count, count_len, ga);
 }
 
 }  // namespace phieng
