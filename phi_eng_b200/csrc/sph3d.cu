@@ -1512,7 +1512,9 @@ struct World3 {
   DevBody3* dbodies = nullptr;
   uint32_t bodies_cap = 0;
   unsigned int* h_pinned = nullptr;
-  cudaGraphExec_t gexec = nullptr;
+  cudaGraphExec_t gexec = nullptr;   // one substep
+  cudaGraphExec_t gsteps = nullptr;  // kGraphSteps of them, once gexec has run often enough
+  uint32_t gruns = 0;                // substeps run with gsig
   std::string gsig;
   bool profiling = false;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1556,6 +1558,8 @@ bool dalloc3(World3* w, T*& p, size_t count) {
 void release_graph3(World3* w) {
   if (w->gexec) cudaGraphExecDestroy(w->gexec);
   w->gexec = nullptr;
+  if (w->gsteps) cudaGraphExecDestroy(w->gsteps);
+  w->gsteps = nullptr;
   w->gsig.clear();
 }
 
@@ -2153,32 +2157,46 @@ void enqueue_substep3(World3* w, const StepParams3& P, cudaStream_t st) {
   if (w->profiling) cudaEventRecordWithFlags(w->ev[3], st, cudaEventRecordExternal);
 }
 
-bool run_substep3(World3* w, const StepParams3& P) {
-  std::string sig((const char*)&P, sizeof(P));
-  sig.append((const char*)&w->n, sizeof(w->n));
-  sig.push_back(w->profiling ? 'p' : '-');
-  sig.push_back(w->sid_perm_n == w->n ? 's' : '-');
-  if (!w->gexec || sig != w->gsig) {
-    release_graph3(w);
-    cudaGraph_t g = nullptr;
-    if (!ok3(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal))) return false;
-    enqueue_substep3(w, P, w->own_stream);
-    cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
-    if (!ok3(w, r)) return false;
-    r = cudaGraphInstantiate(&w->gexec, g, 0);
-    cudaGraphDestroy(g);
-    if (!ok3(w, r)) {
-      w->gexec = nullptr;
-      return false;
-    }
-    w->gsig = sig;
+bool capture_substeps3(World3* w, const StepParams3& P, uint32_t steps, cudaGraphExec_t* out) {
+  cudaGraph_t g = nullptr;
+  if (!ok3(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal))) return false;
+  for (uint32_t k = 0; k < steps; k++) enqueue_substep3(w, P, w->own_stream);
+  cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
+  if (!ok3(w, r)) return false;
+  r = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (!ok3(w, r)) {
+    *out = nullptr;
+    return false;
   }
-  if (!ok3(w, cudaGraphLaunch(w->gexec, w->stream))) return false;
-  w->sid_perm_n = w->n;
-  w->substeps++;
-  w->host_valid = false;
-  w->dp_dev = true;
-  w->keys_valid = true;
+  return true;
+}
+
+// `count` substeps from cached graphs, as the 2D step.
+bool run_substeps3(World3* w, const StepParams3& P, uint32_t count) {
+  while (count) {
+    std::string sig((const char*)&P, sizeof(P));
+    sig.append((const char*)&w->n, sizeof(w->n));
+    sig.push_back(w->profiling ? 'p' : '-');
+    sig.push_back(w->sid_perm_n == w->n ? 's' : '-');
+    if (!w->gexec || sig != w->gsig) {
+      release_graph3(w);
+      if (!capture_substeps3(w, P, 1, &w->gexec)) return false;
+      w->gsig = sig;
+      w->gruns = 0;
+    }
+    const bool many = count >= kGraphSteps && w->gruns >= kGraphAfter && w->sid_perm_n == w->n && !w->profiling;
+    if (many && !w->gsteps && !capture_substeps3(w, P, kGraphSteps, &w->gsteps)) return false;
+    const uint32_t k = many ? kGraphSteps : 1u;
+    if (!ok3(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream))) return false;
+    w->gruns = std::min(w->gruns + k, kGraphAfter);
+    w->sid_perm_n = w->n;
+    w->substeps += k;
+    w->host_valid = false;
+    w->dp_dev = true;
+    w->keys_valid = true;
+    count -= k;
+  }
   return true;
 }
 
@@ -2297,7 +2315,10 @@ bool run_substep3_adaptive(World3* w, float dt) {
   return true;
 }
 
-bool world_step3(World3* w, float dt) {
+// Steps of dt: *done of at most `steps`, more than one where every step runs
+// the same launches.
+bool world_step3(World3* w, float dt, uint32_t steps, uint32_t* done) {
+  *done = 1;
   if (w->cfg.enabled && w->n > 0 && dt > 0.0f) {
     if (w->cfg.adaptive_resolution && w->pos && w->dcap < std::max(resample_bound3(w->n), kMaxParticles3D)) {
       if (!ensure_host3(w)) return false;  // room for the splits: re-upload into larger buffers
@@ -2313,10 +2334,17 @@ bool world_step3(World3* w, float dt) {
       std::memcpy(&bits, &w->time, 4);
       enqueue_set_word(w->scalar + kClockWord3, bits, w->stream);
     }
-    for (uint32_t k = 0; k < ns; k++)
-      if (!(w->cfg.adaptive_resolution ? run_substep3_adaptive(w, dt / (float)ns) : run_substep3(w, P))) return false;
+    if (w->cfg.adaptive_resolution) {
+      for (uint32_t k = 0; k < ns; k++)
+        if (!run_substep3_adaptive(w, dt / (float)ns)) return false;
+    } else {
+      // no substeps to count and no clock to set: the steps differ in nothing
+      const bool cfl = w->cfg.cfl > 0.0f && w->cfg.max_substeps > 1;
+      if (!cfl && !(P.flags & F_TURB)) *done = steps;
+      if (!run_substeps3(w, P, ns * *done)) return false;
+    }
   }
-  w->time += dt;
+  for (uint32_t k = 0; k < *done; k++) w->time += dt;
   return true;
 }
 
@@ -2718,7 +2746,8 @@ void phieng_world3_free(World3* w) {
 
 void phieng_world3_step(World3* w, float dt) {
   if (!w || !std::isfinite(dt) || dt <= 0.0f) return;
-  world_step3(w, std::min(dt, kMaxDt));
+  uint32_t done;
+  world_step3(w, std::min(dt, kMaxDt), 1, &done);
 }
 
 void phieng_world3_set_gravity(World3* w, float gx, float gy, float gz) {
@@ -2985,8 +3014,8 @@ int32_t phieng_sph3_step_n(World3* w, float dt, uint32_t steps) {
   if (!w) return 0;
   if (!std::isfinite(dt) || dt <= 0.0f) return 1;
   const float d = std::min(dt, kMaxDt);
-  for (uint32_t s = 0; s < steps; s++)
-    if (!world_step3(w, d)) return 0;
+  for (uint32_t done = 0; steps; steps -= done)
+    if (!world_step3(w, d, steps, &done)) return 0;
   return 1;
 }
 

@@ -93,7 +93,9 @@ struct World2 {
   size_t d_tmp_bytes = 0;
   unsigned int* h_pinned = nullptr;
 
-  cudaGraphExec_t gexec = nullptr;
+  cudaGraphExec_t gexec = nullptr;   // one substep
+  cudaGraphExec_t gsteps = nullptr;  // kGraphSteps of them, once gexec has run often enough
+  uint32_t gruns = 0;                // substeps run with gsig
   std::string gsig;
 
   // phase timing: events recorded between the phases of every substep
@@ -234,6 +236,8 @@ void release_graph(World2* w) {
   if (w->gexec) cudaGraphExecDestroy(w->gexec);
   w->gexec = nullptr;
   w->gsig.clear();
+  if (w->gsteps) cudaGraphExecDestroy(w->gsteps);
+  w->gsteps = nullptr;
   if (w->cexec) cudaGraphExecDestroy(w->cexec);
   w->cexec = nullptr;
   w->csig.clear();
@@ -698,37 +702,51 @@ void enqueue_substep_body(World2* w, const StepParams& P, cudaStream_t st) {
   if (w->profiling) cudaEventRecordWithFlags(w->ev[3], st, cudaEventRecordExternal);
 }
 
-// One substep, replayed from a cached CUDA graph while the launch
-// parameters stay the same.
-bool run_substep(World2* w, const StepParams& P) {
-  // Buffer reallocations release the graph, so the parameters and the
-  // particle count identify it.
-  std::string sig((const char*)&P, sizeof(P));
-  sig.append((const char*)&w->n, sizeof(w->n));
-  sig.push_back(w->profiling ? 'p' : '-');
-  sig.push_back(w->sid_perm_n == w->n ? 's' : '-');
-  if (!w->gexec || sig != w->gsig) {
-    release_graph(w);
-    cudaGraph_t g = nullptr;
-    if (!cuda_ok(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
-      return false;
-    enqueue_substep_body(w, P, w->own_stream);
-    cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
-    if (!cuda_ok(w, r, "end capture")) return false;
-    r = cudaGraphInstantiate(&w->gexec, g, 0);
-    cudaGraphDestroy(g);
-    if (!cuda_ok(w, r, "graph instantiate")) {
-      w->gexec = nullptr;
-      return false;
-    }
-    w->gsig = sig;
+// A CUDA graph of `steps` substeps.
+bool capture_substeps(World2* w, const StepParams& P, uint32_t steps, cudaGraphExec_t* out) {
+  cudaGraph_t g = nullptr;
+  if (!cuda_ok(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
+    return false;
+  for (uint32_t k = 0; k < steps; k++) enqueue_substep_body(w, P, w->own_stream);
+  cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
+  if (!cuda_ok(w, r, "end capture")) return false;
+  r = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  if (!cuda_ok(w, r, "graph instantiate")) {
+    *out = nullptr;
+    return false;
   }
-  if (!cuda_ok(w, cudaGraphLaunch(w->gexec, w->stream), "graph launch")) return false;
-  w->sid_perm_n = w->n;
-  w->substeps++;
-  w->host_state_valid = false;
-  w->dp_on_device = true;
-  w->keys_valid = true;
+  return true;
+}
+
+// `count` substeps, replayed from cached CUDA graphs while the launch
+// parameters stay the same.
+bool run_substeps(World2* w, const StepParams& P, uint32_t count) {
+  while (count) {
+    // Buffer reallocations release the graphs, so the parameters and the
+    // particle count identify them.
+    std::string sig((const char*)&P, sizeof(P));
+    sig.append((const char*)&w->n, sizeof(w->n));
+    sig.push_back(w->profiling ? 'p' : '-');
+    sig.push_back(w->sid_perm_n == w->n ? 's' : '-');
+    if (!w->gexec || sig != w->gsig) {
+      release_graph(w);
+      if (!capture_substeps(w, P, 1, &w->gexec)) return false;
+      w->gsig = sig;
+      w->gruns = 0;
+    }
+    const bool many = count >= kGraphSteps && w->gruns >= kGraphAfter && w->sid_perm_n == w->n && !w->profiling;
+    if (many && !w->gsteps && !capture_substeps(w, P, kGraphSteps, &w->gsteps)) return false;
+    const uint32_t k = many ? kGraphSteps : 1u;
+    if (!cuda_ok(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream), "graph launch")) return false;
+    w->gruns = std::min(w->gruns + k, kGraphAfter);
+    w->sid_perm_n = w->n;
+    w->substeps += k;
+    w->host_state_valid = false;
+    w->dp_on_device = true;
+    w->keys_valid = true;
+    count -= k;
+  }
   return true;
 }
 
@@ -1104,18 +1122,19 @@ bool count_substeps(World2* w) {
 }
 
 // World2::step (world.rs:706-732) restricted to the fluid phase (1b).
-bool world_step(World2* w, float dt) {
+// Steps of dt: *done of at most `steps`, more than one where every step runs
+// the same launches.
+bool world_step(World2* w, float dt, uint32_t steps, uint32_t* done) {
+  *done = 1;
   if (w->is_batch()) {
     // every scene advances one substep of dt (batches take no CFL substeps)
     if (w->n > 0 && dt > 0.0f) {
       if (!prepare(w)) return false;
       if (!upload_scene_table(w, dt)) return false;
-      if (!run_substep(w, make_params(w, dt))) return false;
+      if (!run_substeps(w, make_params(w, dt), steps)) return false;
+      *done = steps;
     }
-    w->time += dt;
-    return true;
-  }
-  if (w->cfg.enabled && w->n > 0 && dt > 0.0f) {  // step_fluid guards (fluid.rs:550-552)
+  } else if (w->cfg.enabled && w->n > 0 && dt > 0.0f) {  // step_fluid guards (fluid.rs:550-552)
     if (unsupported(w, true, true)) return false;
     if (w->cfg.adaptive_resolution && w->d.state && w->d.cap < std::max(resample_bound(w->n), kMaxParticles2D)) {
       // room for the splits: bring the state home and upload it into larger buffers
@@ -1129,10 +1148,17 @@ bool world_step(World2* w, float dt) {
     const float sub = dt / (float)ns;
     const StepParams P = make_params(w, sub);
     set_clock(w, P, w->time);  // every CFL substep sees the step's start time
-    for (uint32_t k = 0; k < ns; k++)
-      if (!(w->cfg.adaptive_resolution ? run_substep_adaptive(w, sub) : run_substep(w, P))) return false;
+    if (w->cfg.adaptive_resolution) {
+      for (uint32_t k = 0; k < ns; k++)
+        if (!run_substep_adaptive(w, sub)) return false;
+    } else {
+      // no substeps to count and no clock to set: the steps differ in nothing
+      const bool cfl = w->cfg.cfl > 0.0f && w->cfg.max_substeps > 1;
+      if (!cfl && !(P.flags & F_TURB)) *done = steps;
+      if (!run_substeps(w, P, ns * *done)) return false;
+    }
   }
-  w->time += dt;
+  for (uint32_t k = 0; k < *done; k++) w->time += dt;
   return true;
 }
 
@@ -1144,10 +1170,7 @@ bool world_steps(World2* w, float dt, uint32_t steps) {
         dt > 0.0f) {
       if (!prepare(w, false) || !run_small(w, dt, steps, &done)) return false;
     }
-    if (!done) {
-      if (!world_step(w, dt)) return false;
-      done = 1;
-    }
+    if (!done && !world_step(w, dt, steps, &done)) return false;
     steps -= done;
   }
   return true;
@@ -2447,7 +2470,7 @@ int32_t phieng_sph_closure_step(World2* w, float dt_fine, uint32_t coarse_steps,
         for (uint32_t r = 0; r < w->closure_ratio; r++) {
           set_clock(w, Pf, tf);
           tf += dt_fine;
-          if (!run_substep(w, Pf)) return 0;
+          if (!run_substeps(w, Pf, 1)) return 0;
         }
         if (batch && !upload_scene_table(w, dtc)) return 0;
         if (k + 1 < coarse_steps) enqueue_sort_density(w, Pc, w->d_svp);
