@@ -892,14 +892,22 @@ __global__ void __launch_bounds__(256, 4) k_force_closure(
 // density pass, each as a maximum over particles (negative values count as
 // 0, a NaN as +inf): out[0] = largest per-particle density increase over the
 // step, (rho'_i - rho_i) / rho0; out[1] = largest compression after the step,
-// rho'_i / rho0 - 1; out[2] = largest compression before it. Float bits,
-// atomicMax (all values >= 0, so the bit order is the value order and the
-// maxima do not depend on the order of the atomics).
+// rho'_i / rho0 - 1; out[2] = largest compression before it. Blocks leave
+// their maxima in parts; the last one to finish (*ticket, zero between
+// launches) takes theirs and folds the step into the running maxima acc = (max
+// out[0], max out[1], max (out[1] - out[2])), the per-step value of each
+// criterion (jump, compression, growth). Against atomics on a cleared out and a
+// fold kernel: two launches less per coarse step, eight
+// steps of 2^20 particles 1579 -> 1537 us with the shorter gaps.
+constexpr uint32_t kCheckBlocks = 148u * 8u;
+
 template <bool PHASE, bool BATCH>
 __global__ void __launch_bounds__(256) k_closure_check(const float2* __restrict__ sdq, const uint32_t* __restrict__ sid,
                                                        const uint8_t* __restrict__ sphase, uint32_t n, StepParams P0,
                                                        BatchTab bt, const float* __restrict__ rho_prev,
-                                                       unsigned int* __restrict__ out) {
+                                                       float* parts, uint32_t* ticket, float* out, float* acc) {
+  chain_wait(sdq, sid, sphase, rho_prev);
+  __shared__ bool s_last;
   __shared__ float red[3][8];
   float v[3] = {0.0f, 0.0f, 0.0f};
   // grid-stride, then warp and block maxima: one atomic per block and value
@@ -926,7 +934,36 @@ __global__ void __launch_bounds__(256) k_closure_check(const float2* __restrict_
   if (threadIdx.x < 3) {
     float m = 0.0f;
     for (uint32_t k = 0; k < (blockDim.x >> 5); k++) m = fmaxf(m, red[threadIdx.x][k]);
-    atomicMax(&out[threadIdx.x], __float_as_uint(m));
+    parts[3 * blockIdx.x + threadIdx.x] = m;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+#pragma unroll
+  for (int c = 0; c < 3; c++) v[c] = 0.0f;
+  for (uint32_t k = threadIdx.x; k < gridDim.x; k += blockDim.x)
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] = fmaxf(v[c], __ldcg(&parts[3 * k + c]));
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[c] = fmaxf(v[c], __shfl_xor_sync(0xFFFFFFFFu, v[c], o));
+    if (lane == 0) red[c][wid] = v[c];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int c = 0; c < 3; c++) {
+      v[c] = 0.0f;
+      for (uint32_t k = 0; k < (blockDim.x >> 5); k++) v[c] = fmaxf(v[c], red[c][k]);
+      out[c] = v[c];
+    }
+    acc[0] = fmaxf(acc[0], v[0]);
+    acc[1] = fmaxf(acc[1], v[1]);
+    acc[2] = fmaxf(acc[2], __fsub_rn(v[1], v[2]));
+    *ticket = 0u;
   }
 }
 
@@ -1423,42 +1460,36 @@ void enqueue_closure_force(const FluidBufs& b, uint32_t n, const StepParams& P, 
   launch_closure<kModeClosure>(b, n, P, mlp, io, st);
 }
 
-// Running maxima of the three closure checks over a block of coarse steps:
-// acc = (max out[0], max out[1], max (out[1] - out[2])), the per-step value
-// of each criterion (jump, compression, growth); reset to -inf.
-__global__ void k_check_fold(const unsigned int* __restrict__ out, float* __restrict__ acc, int reset) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (reset) {
-    acc[0] = acc[1] = acc[2] = -INFINITY;
-    return;
-  }
-  const float v0 = __uint_as_float(out[0]), v1 = __uint_as_float(out[1]), v2 = __uint_as_float(out[2]);
-  acc[0] = fmaxf(acc[0], v0);
-  acc[1] = fmaxf(acc[1], v1);
-  acc[2] = fmaxf(acc[2], __fsub_rn(v1, v2));
+// The running maxima of the closure checks before a block of coarse steps.
+__global__ void k_check_reset(float* acc) {
+  if (threadIdx.x < 3) acc[threadIdx.x] = -INFINITY;
 }
 
-void enqueue_check_fold(const unsigned int* out, float* acc, bool reset, cudaStream_t st) {
-  k_check_fold<<<1, 32, 0, st>>>(out, acc, reset ? 1 : 0);
-}
+void enqueue_check_reset(float* acc, cudaStream_t st) { k_check_reset<<<1, 32, 0, st>>>(acc); }
 
 __global__ void k_set_word(unsigned int* p, unsigned int v) { *p = v; }
 
 void enqueue_set_word(unsigned int* p, uint32_t v, cudaStream_t st) { k_set_word<<<1, 1, 0, st>>>(p, v); }
 
-void enqueue_closure_check(const FluidBufs& b, uint32_t n, const StepParams& P, const float* rho_prev,
-                           unsigned int* out, cudaStream_t st) {
-  cudaMemsetAsync(out, 0, 3 * sizeof(unsigned int), st);
+uint32_t closure_check_words() { return 3u * kCheckBlocks + 1u; }
+
+void enqueue_closure_check(const FluidBufs& b, uint32_t n, const StepParams& P, const float* rho_prev, float* words,
+                           float* out, float* acc, cudaStream_t st) {
   if (n == 0) return;
   const bool ph = (P.flags & F_PHASE) != 0, bat = b.batch.ptab != nullptr;
-  const uint32_t g = min(cdiv(n, 256), 148u * 8u);
+  const uint32_t g = min(cdiv(n, 256), kCheckBlocks);
+  uint32_t* ticket = reinterpret_cast<uint32_t*>(words + 3u * kCheckBlocks);
+#define PHIENG_CHECK(PH, BT)                                                                                    \
+  launch_chained(k_closure_check<PH, BT>, g, 256, 0, st, b.sdq, b.sid, b.sphase, n, P, b.batch, rho_prev, words, \
+                 ticket, out, acc)
   if (bat) {
-    if (ph) k_closure_check<true, true><<<g, 256, 0, st>>>(b.sdq, b.sid, b.sphase, n, P, b.batch, rho_prev, out);
-    else k_closure_check<false, true><<<g, 256, 0, st>>>(b.sdq, b.sid, b.sphase, n, P, b.batch, rho_prev, out);
+    if (ph) PHIENG_CHECK(true, true);
+    else PHIENG_CHECK(false, true);
   } else {
-    if (ph) k_closure_check<true, false><<<g, 256, 0, st>>>(b.sdq, b.sid, b.sphase, n, P, b.batch, rho_prev, out);
-    else k_closure_check<false, false><<<g, 256, 0, st>>>(b.sdq, b.sid, b.sphase, n, P, b.batch, rho_prev, out);
+    if (ph) PHIENG_CHECK(true, false);
+    else PHIENG_CHECK(false, false);
   }
+#undef PHIENG_CHECK
 }
 
 // ---------------------------------------------------------------- bodies that react

@@ -184,11 +184,14 @@ void enqueue_closure_force(const FluidBufs& b, uint32_t n, const StepParams& P, 
                            const ClosureIO& io, cudaStream_t st);
 
 // Density checks after the coarse step's new state was sorted and its density
-// computed, into out[0..2] (zeroed first): largest per-particle increase over
-// the step, largest compression after it, largest compression before it
-// (relative to the rest density, float bits).
-void enqueue_closure_check(const FluidBufs& b, uint32_t n, const StepParams& P, const float* rho_prev,
-                           unsigned int* out, cudaStream_t st);
+// computed, into out[0..2]: largest per-particle increase over the step,
+// largest compression after it, largest compression before it (relative to the
+// rest density); folded into the block maxima acc[0..2] (jump, compression,
+// growth). words: closure_check_words() of scratch, zero before the first use.
+void enqueue_closure_check(const FluidBufs& b, uint32_t n, const StepParams& P, const float* rho_prev, float* words,
+                           float* out, float* acc, cudaStream_t st);
+uint32_t closure_check_words();
+void enqueue_check_reset(float* acc, cudaStream_t st);
 
 // Device buffers of a fluid phase with bodies that react (phieng_sph_step_fluid).
 struct DynBufs {
@@ -228,10 +231,6 @@ void enqueue_buoyancy(const FluidBufs& b, const DynBufs& y, uint32_t n, const St
 // tile's look-back wait runs out, sets b.scan_err and ends (the test of the
 // bounded waits). Leaves the bucket ranges wrong.
 void enqueue_scan_silent_tile(const FluidBufs& b, uint32_t m, cudaStream_t st);
-
-// Fold one coarse step's checks (out[0..2] of enqueue_closure_check) into
-// the block maxima acc[0..2] (jump, compression, growth), or reset them.
-void enqueue_check_fold(const unsigned int* out, float* acc, bool reset, cudaStream_t st);
 
 // *p = v, in stream order (the value travels as a launch argument, so the
 // host may reuse its copy at once): the world clock word read by the

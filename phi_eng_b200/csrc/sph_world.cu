@@ -143,6 +143,7 @@ struct World2 {
   float* d_rho_prev = nullptr;  // pre-step density (id order)
   float4* d_block_save = nullptr;  // state at the start of an optimistic block of coarse steps
   float2* d_svp = nullptr;         // sorted closure factors of the last closure density pass
+  float* d_check = nullptr;        // scratch of the density checks
   uint32_t closure_cap = 0;
   cudaGraphExec_t cexec = nullptr;
   std::string csig;
@@ -235,9 +236,9 @@ void free_particle_buffers(FluidBufs& d) {
 void release_graph(World2* w) {
   if (w->gexec) cudaGraphExecDestroy(w->gexec);
   w->gexec = nullptr;
-  w->gsig.clear();
   if (w->gsteps) cudaGraphExecDestroy(w->gsteps);
   w->gsteps = nullptr;
+  w->gsig.clear();
   if (w->cexec) cudaGraphExecDestroy(w->cexec);
   w->cexec = nullptr;
   w->csig.clear();
@@ -1466,9 +1467,12 @@ bool ensure_closure_buffers(World2* w) {
   dfree(w->d_rho_prev);
   dfree(w->d_block_save);
   dfree(w->d_svp);
+  dfree(w->d_check);
   w->closure_cap = 0;
   if (!dalloc(w, w->d_save, w->d.cap) || !dalloc(w, w->d_rho_prev, w->d.cap) ||
-      !dalloc(w, w->d_block_save, w->d.cap) || !dalloc(w, w->d_svp, w->d.cap))
+      !dalloc(w, w->d_block_save, w->d.cap) || !dalloc(w, w->d_svp, w->d.cap) ||
+      !dalloc(w, w->d_check, closure_check_words()) ||
+      !cuda_ok(w, cudaMemsetAsync(w->d_check, 0, sizeof(float) * closure_check_words(), w->stream), "check words"))
     return false;
   w->closure_cap = w->d.cap;
   release_graph(w);
@@ -1486,7 +1490,7 @@ void enqueue_sort_density(World2* w, const StepParams& P, float2* svp = nullptr)
 
 // One coarse step from a sorted state with its density: closure force pass,
 // then sort + density of the new state and the density check into
-// scalar[4]; replayed from a cached graph.
+// scalar[4], folded into the maxima at scalar[13]; replayed from a cached graph.
 bool run_coarse(World2* w, const StepParams& P, const MlpDev& mlp, const ClosureIO& io) {
   std::string sig((const char*)&P, sizeof(P));
   sig.append((const char*)&w->n, sizeof(w->n));
@@ -1501,7 +1505,8 @@ bool run_coarse(World2* w, const StepParams& P, const MlpDev& mlp, const Closure
     enqueue_closure_force(w->d, w->n, P, mlp, io, w->own_stream);
     enqueue_sort_and_ranges(w->d, w->n, P, true, w->own_stream);
     enqueue_density(w->d, w->n, P, w->own_stream, w->d_svp);
-    enqueue_closure_check(w->d, w->n, P, io.rho_prev, w->d.scalar + 4, w->own_stream);
+    float* sc = reinterpret_cast<float*>(w->d.scalar);
+    enqueue_closure_check(w->d, w->n, P, io.rho_prev, w->d_check, sc + 4, sc + 13, w->own_stream);
     cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
     if (!cuda_ok(w, r, "end capture")) return false;
     r = cudaGraphInstantiate(&w->cexec, g, 0);
@@ -1596,6 +1601,7 @@ void phieng_world_free(World2* w) {
     dfree(w->d_rho_prev);
     dfree(w->d_block_save);
     dfree(w->d_svp);
+    dfree(w->d_check);
     dfree(w->d_cbodies);
     dfree(w->d_poly);
     dfree(w->d_gpos);
@@ -2391,14 +2397,13 @@ int32_t phieng_sph_closure_step(World2* w, float dt_fine, uint32_t coarse_steps,
                                       w->stream),
                    "block save"))
         return 0;
-      enqueue_check_fold(w->d.scalar + 4, acc, true, w->stream);
+      enqueue_check_reset(acc, w->stream);
       float tb = w->time;
       for (uint32_t b = 0; b < nb; b++) {
         set_clock(w, Pc, tb);
         tb += dtc;
         if (!run_coarse(w, Pc, mlp, io)) return 0;
         w->sid_perm_n = w->n;
-        enqueue_check_fold(w->d.scalar + 4, acc, false, w->stream);
       }
       if (!cuda_ok(w, cudaMemcpyAsync(w->h_pinned, w->d.scalar + 4, 12 * sizeof(unsigned int), cudaMemcpyDeviceToHost,
                                       w->stream),
