@@ -62,26 +62,25 @@ PHASE_ALG_BYTES = dict(sort_ranges=ALG_BYTES["sort"] + ALG_BYTES["ranges"] + ALG
 
 # What this implementation moves per particle (each of its arrays read or
 # written once; B/N = buckets per particle):
-#   sort:    scan: read counts twice, write start + cursor, clear counts
-#            (20 B per bucket); place: read id 4 + key 4, write (key, id) 8;
-#            fixup: read (key, id) 8 + start 8, write (key, id) 8,
-#            gather state 16 -> write pos 8 + vel 8                = 72 + 20 B/N
+#   sort:    scan: read counts, write start, counts back to zero (12 B per
+#            bucket); place: read id 4 + key 4 + start 8, gather state 16 ->
+#            write (key, id) 8, pos 8 + vel 8                       = 56 + 12 B/N
 #   density: read pos 8 + key 4; write (density, q) 8 + pressure 4,
 #            three 32-bit neighbour-row masks 12                    = 36
 #   force:   read pos 8, vel 8, (density, q) 8, key 4, id 4, masks 12;
-#            write state 16 + next key 4                             = 64
+#            write state 16 + next key 4 + id by slot 4              = 68
 DENSITY_BYTES = 36
-FORCE_BYTES = 64
+FORCE_BYTES = 68
 # DRAM bytes (read + write) of one launch of the named kernel on the named
 # workload and precision mode, from an ncu capture (profiles/).
 PROFILED_TRAFFIC = {("dam_break_1m", "exact", "force_integrate"): 48.333312e6 + 1.921792e6,
                     ("dam_break_1m", "tolerance", "force_integrate"): 48.337664e6 + 1.710592e6}
 PROFILED_TRAFFIC_3D = {"force_integrate": 85.545216e6 + 14.838528e6}  # 100^3 3D dam break
-KERNELS_PER_STEP = 5  # single-pass scan, place, fixup, density, force
+KERNELS_PER_STEP = 5  # single-pass scan, place, fix, density, force
 
 
 def sort_bytes(buckets_per_particle: float) -> float:
-    return 72 + 20 * buckets_per_particle
+    return 56 + 12 * buckets_per_particle
 
 
 def hbm_peak():
@@ -356,15 +355,14 @@ def closure_line(sc, precision: int) -> dict:
 
 
 # 3D (fluid3.rs) chain, bytes per particle of each phase:
-#   sort:    place 16 (read key + previous slot id, write key, id); fixup 64
-#            + 8 (read key, id, start pair; write key, id; gather pos 16 +
-#            vel 16 -> write 32)                                  = 104 + 20 B/N
-#   density: read pos 16 + key 4; write (density, q) 8 + pressure 4 + nine
-#            32-bit row masks 36                                     = 68
-#   force:   read pos 16, vel 16, (density, q) 8, key 4, id 4, masks 36;
-#            write pos 16 + vel 16 + next key 4                       = 120
-DENSITY3_BYTES = 68
-FORCE3_BYTES = 120
+#   sort:    read id 4 + key 4 + start 8, gather pos 16 + vel 16 -> write
+#            (key, id) 8, pos + vel 32, cell word 4               = 92 + 12 B/N
+#   density: read pos 16 + key 4 + cell word 4; write (density, q) 8 +
+#            pressure 4 + nine 32-bit row masks and their flags 40    = 76
+#   force:   read pos 16, vel 16, (density, q) 8, key 4, id 4, masks 40;
+#            write pos 16 + vel 16 + next key 4 + id by slot 4        = 128
+DENSITY3_BYTES = 76
+FORCE3_BYTES = 128
 
 
 def fluid3d_line(steps: int, warmup: int, side: int = 100) -> dict:
@@ -422,7 +420,7 @@ def fluid3d_line(steps: int, warmup: int, side: int = 100) -> dict:
     ms, ph = timed()
     buckets = w.status().grid_buckets
     names = ["sort_ranges", "density", "force_integrate"]
-    bytes_pp = [104 + 20 * buckets / n, DENSITY3_BYTES, FORCE3_BYTES]
+    bytes_pp = [92 + 12 * buckets / n, DENSITY3_BYTES, FORCE3_BYTES]
     top = int(np.argmax(ph))
     peak, _ = hbm_peak()
     achieved = bytes_pp[top] * n / (ph[top] / 1000.0) / 1e9
@@ -457,7 +455,7 @@ def fluid3d_line(steps: int, warmup: int, side: int = 100) -> dict:
 
 
 # kernels per substep of a slab rank: halo pack + unpack, the world's five
-# (scan, placement, fixup, density, force), migrant pack + unpack + settle
+# (scan, placement, fix, density, force), migrant pack + unpack + settle
 SLAB_KERNELS_PER_SUBSTEP = 10
 
 

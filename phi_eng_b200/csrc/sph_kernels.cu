@@ -369,8 +369,10 @@ __device__ __forceinline__ float neighbour_density_term(float d2, float m, const
 // two cycles; the 3D pass has too many moves between the two and got slower, 165
 // -> 174 us). Otherwise the general form, one
 // candidate at a time with poly6's range test.
+// Batches: eight blocks per SM (32 registers instead of 39), 144 -> 140 us for
+// 4.6M particles; single worlds fit eight by themselves.
 template <bool MASS, bool PHASE, bool BATCH, bool HEQ>
-__global__ void __launch_bounds__(256) k_density(const float2* __restrict__ spos, const uint32_t* __restrict__ skey,
+__global__ void __launch_bounds__(256, BATCH ? 8 : 0) k_density(const float2* __restrict__ spos, const uint32_t* __restrict__ skey,
                                                  const float* __restrict__ smass,
                                                  const uint8_t* __restrict__ sphase, uint32_t n,
                                                  const uint32_t* __restrict__ start, StepParams P0, BatchTab bt,
@@ -752,8 +754,12 @@ __global__ void __launch_bounds__(256) k_ghost_density(const float2* __restrict_
   P.gq[g] = __fdiv_rn(p, __fmul_rn(rc, rc));
 }
 
+// Batches: 40 registers instead of 56, a few spilled. A scene's parameters come
+// from memory, so a thread waits more than in a single world, where six blocks
+// only cost spills (2^18 particles 378 -> 394 us for 10 steps): 4 steps of 512
+// scenes (4.6M particles) 2240 -> 2130 us.
 template <bool MASS, bool DEBUG, bool BATCH, bool PLAIN>
-__global__ void __launch_bounds__(256) k_force_integrate(
+__global__ void __launch_bounds__(256, BATCH ? 6 : 0) k_force_integrate(
     const float2* __restrict__ spos, const float2* __restrict__ svel, const float2* __restrict__ sdq,
     const uint32_t* __restrict__ skey, const uint32_t* __restrict__ sid, const float* __restrict__ smass,
     uint32_t n, const uint32_t* __restrict__ start, StepParams P0, BatchTab bt, const DevBody* __restrict__ bodies,
