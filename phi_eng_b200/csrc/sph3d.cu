@@ -3090,9 +3090,12 @@ int32_t phieng_sph3_set_state(World3* w, const float* xyzv, uint32_t n) {
     float2* rows = reinterpret_cast<float2*>(w->nmask);
     if (!ok3(w, cudaMemcpyAsync(rows, xyzv, 24 * (size_t)n, cudaMemcpyHostToDevice, w->stream))) return 0;
     k_unpack3<<<cdiv(n, 256), 256, 0, w->stream>>>(rows, n, w->pos, w->vel);
-    if (!ok3(w, cudaGetLastError())) return 0;
+    const cudaError_t launched = cudaGetLastError();
     Bounds3 b;
     for (uint32_t i = 0; i < n; i++) b.add(xyzv[6 * (size_t)i], xyzv[6 * (size_t)i + 1], xyzv[6 * (size_t)i + 2]);
+    // the rows are the caller's own: from page-locked memory the copy is still
+    // on its way here, and the caller may refill or free them at once
+    if (!ok3(w, cudaStreamSynchronize(w->stream)) || !ok3(w, launched)) return 0;
     plan_bounds3(w, b);
     w->dev_valid = true;
     w->host_valid = false;
