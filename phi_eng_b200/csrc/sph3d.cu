@@ -2161,8 +2161,13 @@ bool capture_substeps3(World3* w, const StepParams3& P, uint32_t steps, cudaGrap
   cudaGraph_t g = nullptr;
   if (!ok3(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal))) return false;
   for (uint32_t k = 0; k < steps; k++) enqueue_substep3(w, P, w->own_stream);
+  const cudaError_t launched = cudaGetLastError();  // a refused launch is missing from the graph
   cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
   if (!ok3(w, r)) return false;
+  if (!ok3(w, launched)) {
+    cudaGraphDestroy(g);
+    return false;
+  }
   r = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (!ok3(w, r)) {

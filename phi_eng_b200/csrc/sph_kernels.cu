@@ -1385,7 +1385,9 @@ cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is the kernel's, shared by all threads and worlds: always the
+  // largest world's, never this world's need
+  cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem_max());
   if (r == cudaSuccess && sh.blocks > 8)
     r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (r != cudaSuccess) return r;

@@ -112,6 +112,12 @@ __host__ __device__ inline SmallLayout small_layout(uint32_t n, uint32_t m, uint
   return L;
 }
 
+// Bytes of the largest world's shared arrays.
+inline size_t small_smem_max() {
+  return sizeof(uint32_t) *
+         small_layout(kSmallMax, kSmallKeys, kSmallShare, kSmallShare * kSmallLanes, true, true, false).words;
+}
+
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -124,7 +124,10 @@ template <class Gather>
 inline void launch_sort_small(const uint32_t* key, uint32_t n, uint32_t m, uint32_t* start, uint32_t* count,
                               uint32_t count_len, const Gather& ga, cudaStream_t st) {
   const size_t smem = small_sort_smem(n, m);
-  cudaFuncSetAttribute(k_sort_small<Gather>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit is the kernel's, shared by all threads and worlds: always the
+  // largest set's, never this set's need
+  cudaFuncSetAttribute(k_sort_small<Gather>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)small_sort_smem(kSmallSortMax, kSmallSortKeys));
   launch_chained(k_sort_small<Gather>, std::max<uint32_t>(1u, (n + 1023u) / 1024u * 4u), 1024, smem, st, key, n, m,
                  start, count, count_len, ga);
 }

@@ -709,8 +709,13 @@ bool capture_substeps(World2* w, const StepParams& P, uint32_t steps, cudaGraphE
   if (!cuda_ok(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
     return false;
   for (uint32_t k = 0; k < steps; k++) enqueue_substep_body(w, P, w->own_stream);
+  const cudaError_t launched = cudaGetLastError();  // a refused launch is missing from the graph
   cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
   if (!cuda_ok(w, r, "end capture")) return false;
+  if (!cuda_ok(w, launched, "captured launch")) {
+    cudaGraphDestroy(g);
+    return false;
+  }
   r = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (!cuda_ok(w, r, "graph instantiate")) {
@@ -1507,8 +1512,13 @@ bool run_coarse(World2* w, const StepParams& P, const MlpDev& mlp, const Closure
     enqueue_density(w->d, w->n, P, w->own_stream, w->d_svp);
     float* sc = reinterpret_cast<float*>(w->d.scalar);
     enqueue_closure_check(w->d, w->n, P, io.rho_prev, w->d_check, sc + 4, sc + 13, w->own_stream);
+    const cudaError_t launched = cudaGetLastError();
     cudaError_t r = cudaStreamEndCapture(w->own_stream, &g);
     if (!cuda_ok(w, r, "end capture")) return false;
+    if (!cuda_ok(w, launched, "captured launch")) {
+      cudaGraphDestroy(g);
+      return false;
+    }
     r = cudaGraphInstantiate(&w->cexec, g, 0);
     cudaGraphDestroy(g);
     if (!cuda_ok(w, r, "graph instantiate")) {
