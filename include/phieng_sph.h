@@ -219,7 +219,9 @@ uint32_t phieng_world_fluid_get(const World2* world, float* out, uint32_t max);
 typedef struct PhiengSphStatus {
   int32_t error;          /* last error (sticky until phieng_sph_clear_error) */
   uint32_t particles;     /* particle count */
-  uint64_t substeps;      /* fluid substeps run since creation */
+  uint64_t substeps;      /* fluid substeps run since creation (where the GPU takes a step's CFL
+                           * substep count, as far as the GPU has run: exact after a call that
+                           * synchronises) */
   uint32_t grid_log2_w;   /* bucket grid: columns = 1 << grid_log2_w */
   uint32_t grid_log2_h;   /* rows = 1 << grid_log2_h */
   uint32_t sort_passes;   /* passes of the bucket sort per substep (1) */

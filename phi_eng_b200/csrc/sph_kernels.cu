@@ -1365,6 +1365,7 @@ cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams
   A.count = b.count;
   A.count_len = b.count_len;
   A.substeps = ss.substeps;
+  A.substeps_host = ss.substeps_host;
   A.n = n;
   A.steps = ss.steps;
   A.dt = P.dt;

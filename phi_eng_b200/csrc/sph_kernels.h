@@ -147,7 +147,8 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
 // Whole steps of a small world in one launch of one thread-block cluster: the
 // state advanced by `steps` steps of P.dt, each one substep or, with
 // max_substeps > 1, the CFL count of its start state (sound speed c0, cfl_h =
-// cfl * max(h, EPS)); *substeps (if not null) grows by the substeps taken.
+// cfl * max(h, EPS)); *substeps (if not null) grows by the substeps taken, and
+// the new total is left in *substeps_host (page-locked host memory) too.
 // Leaves the sorted density values, the next keys and the bucket counts as the
 // chain of launches does; the keys before the call are not read. *applies =
 // false: not a small world, or one with terms the launch does not take;
@@ -156,7 +157,8 @@ struct SmallSteps {
   uint32_t steps = 1;
   uint32_t max_substeps = 1;
   float c0 = 0.0f, cfl_h = 0.0f;
-  unsigned int* substeps = nullptr;
+  unsigned long long* substeps = nullptr;
+  unsigned long long* substeps_host = nullptr;
 };
 cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss,
                                 cudaStream_t st, bool* applies);

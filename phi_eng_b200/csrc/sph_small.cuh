@@ -54,7 +54,8 @@ struct SmallArgs {
   uint32_t* key;
   uint32_t* count;
   uint32_t count_len;
-  unsigned int* substeps;  // += substeps taken (null: not counted)
+  unsigned long long* substeps;       // += substeps taken (null: not counted)
+  unsigned long long* substeps_host;  // the new total, in page-locked host memory
   uint32_t n, steps;
   float dt;  // of a step (before CFL substeps)
   SmallCfl cfl;
@@ -483,5 +484,9 @@ __global__ void __launch_bounds__(kSmallShare* kSmallLanes, 1)
       cluster_sync();  // the new states and keys; no block still reads this one's shared memory
     }
   }
-  if (A.substeps && rank == 0u && tid == 0u) *A.substeps += taken;
+  if (A.substeps && rank == 0u && tid == 0u) {
+    const unsigned long long total = *A.substeps + taken;
+    *A.substeps = total;
+    *const_cast<volatile unsigned long long*>(A.substeps_host) = total;
+  }
 }

@@ -34,7 +34,8 @@ constexpr uint32_t kMaxParticles2D = 4096;  // MAX_PARTICLES_2D (fluid.rs:30)
 // and has no cap of its own.
 inline uint32_t resample_bound(uint32_t n) { return n + std::min(n, kMaxParticles2D / 2); }
 constexpr uint32_t kClockWord = 16;         // scalar word holding the step's world clock (turbulence)
-constexpr uint32_t kSubstepWord = 24;       // scalar word counting the CFL substeps of whole-step launches
+constexpr uint32_t kSubstepWord = 26;       // scalar words (64 bits) counting the CFL substeps of whole-step launches
+constexpr uint32_t kSubstepPinned = 14;     // and the last total that arrived, in h_pinned
 constexpr uint32_t kSmallStepsPerLaunch = 64;
 
 // AmbientConfig2::default (ambient.rs): springs, drag and turbulence off, air
@@ -103,8 +104,7 @@ struct World2 {
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 
   int32_t error = PHIENG_SPH_OK;
-  uint64_t substeps = 0;
-  bool substeps_pending = false;  // the device counted more (kSubstepWord): count_substeps
+  uint64_t substeps = 0;  // without those the device counts (device_substeps)
 
   // Batch of independent scenes (empty for an ordinary world): scene k owns
   // particles [first, first + count) and bodies [body_first, +nbodies), and
@@ -264,6 +264,7 @@ bool ensure_device(World2* w) {
   w->d.flist_n = w->d.scalar + 25;
   w->d.scan_err = w->d.scalar + 12;  // set when a scan's look-back wait or a tensor-core wait gave up
   if (!cuda_ok(w, cudaMallocHost(&w->h_pinned, 64), "cudaMallocHost")) return false;
+  std::memset(w->h_pinned, 0, 64);
   w->device = dev;
   return true;
 }
@@ -1096,16 +1097,14 @@ bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
     ss.max_substeps = c.max_substeps;
     ss.c0 = cfl_sound_speed(c);
     ss.cfl_h = c.cfl * rmaxf(c.smoothing_length, kEps);
-    ss.substeps = w->d.scalar + kSubstepWord;
+    ss.substeps = reinterpret_cast<unsigned long long*>(w->d.scalar + kSubstepWord);
+    ss.substeps_host = reinterpret_cast<unsigned long long*>(w->h_pinned + kSubstepPinned);
   }
   bool applies = false;
   const cudaError_t r = enqueue_small_steps(w->d, w->n, make_params(w, dt), ss, w->stream, &applies);
   if (!cuda_ok(w, r, "whole-step launch")) return false;
   if (!applies) return true;
-  if (ss.substeps)
-    w->substeps_pending = true;
-  else
-    w->substeps += ss.steps;
+  if (!ss.substeps) w->substeps += ss.steps;
   w->host_state_valid = false;
   w->dp_on_device = true;
   w->keys_valid = true;
@@ -1114,17 +1113,10 @@ bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
   return true;
 }
 
-// The substeps that whole-step launches counted on the device, into substeps.
-bool count_substeps(World2* w) {
-  if (!w->substeps_pending) return true;
-  unsigned int* word = w->d.scalar + kSubstepWord;
-  if (!cuda_ok(w, cudaMemcpyAsync(w->h_pinned + 9, word, 4, cudaMemcpyDeviceToHost, w->stream), "substeps") ||
-      !cuda_ok(w, cudaMemsetAsync(word, 0, 4, w->stream), "substeps") ||
-      !cuda_ok(w, cudaStreamSynchronize(w->stream), "sync"))
-    return false;
-  w->substeps += w->h_pinned[9];
-  w->substeps_pending = false;
-  return true;
+// The substeps that whole-step launches counted on the device, as far as they
+// have run.
+uint64_t device_substeps(const World2* w) {
+  return w->h_pinned ? *reinterpret_cast<const volatile uint64_t*>(w->h_pinned + kSubstepPinned) : 0;
 }
 
 // World2::step (world.rs:706-732) restricted to the fluid phase (1b).
@@ -1949,14 +1941,12 @@ uint32_t phieng_world_fluid_get(const World2* cw, float* out, uint32_t max) {
 }
 
 // ---------------------------------------------------------------- extension
-int32_t phieng_sph_status(const World2* cw, PhiengSphStatus* out) {
-  if (!cw || !out) return 0;
-  World2* w = const_cast<World2*>(cw);
-  count_substeps(w);
+int32_t phieng_sph_status(const World2* w, PhiengSphStatus* out) {
+  if (!w || !out) return 0;
   std::memset(out, 0, sizeof(*out));
   out->error = w->error;
   out->particles = w->n;
-  out->substeps = w->substeps;
+  out->substeps = w->substeps + device_substeps(w);
   out->grid_log2_w = w->plan_valid ? w->plan.log2w : 0;
   out->grid_log2_h = w->plan_valid ? w->plan.log2h : 0;
   out->sort_passes = w->plan_valid ? 1 : 0;
