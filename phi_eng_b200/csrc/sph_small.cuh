@@ -391,10 +391,11 @@ __global__ void __launch_bounds__(kSmallShare* kSmallLanes, 1)
             float2 nd, dv;
             float c, w;
             fp.terms(spos[j], svel[j], sdq[j], P, nd, c, dv, w);
-            tb[l] = nd.x;
-            tb[G + l] = nd.y;
-            tb[2u * G + l] = dv.x;
-            tb[3u * G + l] = dv.y;
+            // a lane without a pair: all factors zero, also where the particle's own row is not finite
+            tb[l] = valid ? nd.x : 0.0f;
+            tb[G + l] = valid ? nd.y : 0.0f;
+            tb[2u * G + l] = valid ? dv.x : 0.0f;
+            tb[3u * G + l] = valid ? dv.y : 0.0f;
             tb[4u * G + l] = valid ? c : 0.0f;
             tb[5u * G + l] = valid ? w : 0.0f;
           } else {
