@@ -589,6 +589,10 @@ uint32_t phieng_sph_debug_forces(World2* world, float* fxy, uint32_t max);
  * world reports PHIENG_SPH_E_CUDA. Returns 1 if no wait ran out (then the
  * bound failed to trigger), 0 otherwise. Test hook for the bounded waits. */
 int32_t phieng_sph_debug_scan_timeout(World2* world);
+/* Step this world as on a GPU (a partition of one) that cannot hold the
+ * thread-block cluster of a small world's whole-step launch: pass by pass, the
+ * same results. 1 ok, 0 null. Test hook. */
+int32_t phieng_sph_debug_no_cluster(World2* world, int32_t on);
 
 /* Rebuild the grid from the current state and write the sorted order:
  * ids[s] = particle id at sorted slot s, keys[s] = its bucket key (either may

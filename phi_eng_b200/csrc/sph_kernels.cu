@@ -16,6 +16,8 @@
 // of neighbors() (fluid.rs:368-386), and accumulates per thread in that order
 // with no atomics, so sums are bit-identical to the reference's and runs are
 // bit-reproducible.
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "sph_kernels.h"
@@ -1328,6 +1330,7 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
 }
 
 // The variant's kernel for these flags.
+constexpr uint32_t kSmallVariants = 9;  // mass, phase, plain; tolerance mode
 template <bool FAST>
 const void* small_kernel(bool m, bool ph, bool plain) {
   if constexpr (FAST) return (const void*)k_small_steps<false, false, true, true>;
@@ -1343,13 +1346,35 @@ const void* small_kernel(bool m, bool ph, bool plain) {
   return (const void*)k_small_steps<false, false, false, false>;
 }
 
-cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss,
-                                cudaStream_t st, bool* applies) {
-  *applies = false;
+// Readies a variant's kernel for clusters of cfg's shape on the current device
+// (its shared-memory limit is the kernel's, shared by all threads and worlds:
+// always the largest world's, never one world's need) and asks whether such a
+// cluster fits there with that much: 16 blocks are more than every GPU must hold,
+// and of a partitioned one few SMs may be visible. Once per device, variant and shape.
+bool small_cluster_fits(const void* kernel, uint32_t variant, cudaLaunchConfig_t cfg) {
+  constexpr int kDevices = 64;
+  static std::atomic<signed char> known[kDevices][kSmallVariants][kSmallBlocks + 1] = {};  // 1: fits, -1: does not
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return false;
+  std::atomic<signed char>& k = known[dev][variant][cfg.gridDim.x];
+  if (k.load(std::memory_order_acquire) == 0) {
+    cfg.dynamicSmemBytes = small_smem_max();
+    int clusters = 0;
+    cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+    if (r == cudaSuccess && cfg.gridDim.x > 8)
+      r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (r == cudaSuccess) r = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
+    if (r != cudaSuccess) cudaGetLastError();
+    k.store(r == cudaSuccess && clusters > 0 ? 1 : -1, std::memory_order_release);
+  }
+  return k.load(std::memory_order_acquire) > 0;
+}
+
+bool enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss, cudaStream_t st) {
   const uint32_t keys = P.grid.sentinel + 1u;
-  if (n == 0 || n > kSmallMax || keys > kSmallKeys || P.nbodies > kSmallBodies || b.batch.ptab || b.order ||
+  if (ss.no_cluster || n == 0 || n > kSmallMax || keys > kSmallKeys || P.nbodies > kSmallBodies || b.batch.ptab || b.order ||
       (P.flags & (F_TURB | F_GHOST | F_POLY | F_DYNAMIC | F_WIDE_NB)))
-    return cudaSuccess;
+    return false;
   const bool fast = fast_flags(P.flags), plain = plain_flags(P.flags);
   const bool m = (P.flags & F_MASS) != 0, ph = (P.flags & F_PHASE) != 0;
   const void* kernel = fast ? small_kernel<true>(m, ph, plain) : small_kernel<false>(m, ph, plain);
@@ -1386,15 +1411,12 @@ cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  // the limit is the kernel's, shared by all threads and worlds: always the
-  // largest world's, never this world's need
-  cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem_max());
-  if (r == cudaSuccess && sh.blocks > 8)
-    r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (r != cudaSuccess) return r;
+  if (!small_cluster_fits(kernel, fast ? kSmallVariants - 1u : (m ? 4u : 0u) | (ph ? 2u : 0u) | (plain ? 1u : 0u), cfg))
+    return false;
   void* args[] = {&A, const_cast<StepParams*>(&P)};
-  *applies = true;
-  return cudaLaunchKernelExC(&cfg, kernel, args);
+  if (cudaLaunchKernelExC(&cfg, kernel, args) == cudaSuccess) return true;
+  cudaGetLastError();  // refused all the same: the chain of launches takes the step, or reports what is wrong
+  return false;
 }
 
 size_t closure_smem_bytes() { return sizeof(MlpSmem) + sizeof(__nv_bfloat16) * 256 * kXRow + sizeof(float) * 256 * 2; }

@@ -150,18 +150,18 @@ void enqueue_force_integrate(const FluidBufs& b, uint32_t n, const StepParams& P
 // cfl * max(h, EPS)); *substeps (if not null) grows by the substeps taken, and
 // the new total is left in *substeps_host (page-locked host memory) too.
 // Leaves the sorted density values, the next keys and the bucket counts as the
-// chain of launches does; the keys before the call are not read. *applies =
-// false: not a small world, or one with terms the launch does not take;
-// nothing was enqueued.
+// chain of launches does; the keys before the call are not read. false: not a
+// small world, or one with terms the launch does not take, or a GPU that cannot
+// hold the cluster; nothing was enqueued.
 struct SmallSteps {
   uint32_t steps = 1;
   uint32_t max_substeps = 1;
   float c0 = 0.0f, cfl_h = 0.0f;
   unsigned long long* substeps = nullptr;
   unsigned long long* substeps_host = nullptr;
+  bool no_cluster = false;  // as on a GPU that cannot hold the cluster
 };
-cudaError_t enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss,
-                                cudaStream_t st, bool* applies);
+bool enqueue_small_steps(const FluidBufs& b, uint32_t n, const StepParams& P, const SmallSteps& ss, cudaStream_t st);
 
 // Closure pass buffers: features (id order, 16 per particle) for the
 // features mode; pre-step state and density (id order) kept by the closure

@@ -166,6 +166,8 @@ struct World2 {
   ResampleBufs rs;
   uint32_t rs_cap = 0;
 
+  bool no_cluster = false;  // phieng_sph_debug_no_cluster
+
   // launch tuning (phieng_sph_set_tuning)
   float buckets_per_particle = 2.0f;
   // arithmetic of the plain density / force passes (phieng_sph_set_precision)
@@ -1085,12 +1087,11 @@ bool run_substep_adaptive(World2* w, float dt) {
 }
 
 // Up to `steps` steps of dt as one launch, for the worlds that take it
-// (enqueue_small_steps); *done = steps taken (0: not such a world). The world
-// is prepared but for its keys.
-bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
-  *done = 0;
+// (enqueue_small_steps): the steps taken (0: not such a world). The world is
+// prepared but for its keys.
+uint32_t run_small(World2* w, float dt, uint32_t steps) {
   const FluidConfig2Ffi& c = w->cfg;
-  if (w->profiling || c.adaptive_resolution || c.boundary_particles) return true;
+  if (w->profiling || c.adaptive_resolution || c.boundary_particles) return 0;
   SmallSteps ss;
   ss.steps = std::min(steps, kSmallStepsPerLaunch);
   if (c.cfl > 0.0f && c.max_substeps > 1) {
@@ -1100,17 +1101,14 @@ bool run_small(World2* w, float dt, uint32_t steps, uint32_t* done) {
     ss.substeps = reinterpret_cast<unsigned long long*>(w->d.scalar + kSubstepWord);
     ss.substeps_host = reinterpret_cast<unsigned long long*>(w->h_pinned + kSubstepPinned);
   }
-  bool applies = false;
-  const cudaError_t r = enqueue_small_steps(w->d, w->n, make_params(w, dt), ss, w->stream, &applies);
-  if (!cuda_ok(w, r, "whole-step launch")) return false;
-  if (!applies) return true;
+  ss.no_cluster = w->no_cluster;
+  if (!enqueue_small_steps(w->d, w->n, make_params(w, dt), ss, w->stream)) return 0;
   if (!ss.substeps) w->substeps += ss.steps;
   w->host_state_valid = false;
   w->dp_on_device = true;
   w->keys_valid = true;
   for (uint32_t k = 0; k < ss.steps; k++) w->time += dt;
-  *done = ss.steps;
-  return true;
+  return ss.steps;
 }
 
 // The substeps that whole-step launches counted on the device, as far as they
@@ -1166,7 +1164,8 @@ bool world_steps(World2* w, float dt, uint32_t steps) {
     uint32_t done = 0;
     if (!w->is_batch() && w->cfg.enabled && !w->cfg.adaptive_resolution && w->n > 0 && w->n <= kMaxParticles2D &&
         dt > 0.0f) {
-      if (!prepare(w, false) || !run_small(w, dt, steps, &done)) return false;
+      if (!prepare(w, false)) return false;
+      done = run_small(w, dt, steps);
     }
     if (!done && !world_step(w, dt, steps, &done)) return false;
     steps -= done;
@@ -2485,6 +2484,12 @@ int32_t phieng_sph_closure_step(World2* w, float dt_fine, uint32_t coarse_steps,
   }
   w->keys_valid = false;  // the last sort consumed the bucket counts
   return cuda_ok(w, cudaGetLastError(), "closure step") ? 1 : 0;
+}
+
+int32_t phieng_sph_debug_no_cluster(World2* w, int32_t on) {
+  if (!w) return 0;
+  w->no_cluster = on != 0;
+  return 1;
 }
 
 int32_t phieng_sph_debug_scan_timeout(World2* w) {
