@@ -836,16 +836,17 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
 // each parameter at once into shared memory, then one thread per parameter adds
 // them up (5.5 MB for 256 CTAs: 6.2 us; one thread reading and adding a parameter's
 // partials on 22 SMs took 15.6). Thread t < kAdamParams returns the
-// sum of parameter p0 + t.
+// sum of parameter p0 + t. Entries from `count` on are not read (a caller's
+// gradient vector ends there).
 constexpr int kAdamParams = 32, kAdamThreads = 256;
-__device__ __forceinline__ float sum_parts(const float* __restrict__ part, uint32_t nparts, int p0,
+__device__ __forceinline__ float sum_parts(const float* __restrict__ part, uint32_t nparts, int p0, int count,
                                            float (&buf)[256][kAdamParams]) {
   constexpr uint32_t kRows = 256 * kAdamParams / kAdamThreads;  // partials per thread
   const uint32_t i = threadIdx.x % kAdamParams, q = threadIdx.x / kAdamParams;
   float g = 0.0f;
   for (uint32_t base = 0; base < nparts; base += 256u) {
     if (base) __syncthreads();
-    if (p0 + (int)i <= kParams) {
+    if (p0 + (int)i < count) {
       float v[kRows];
 #pragma unroll
       for (uint32_t r = 0; r < kRows; r++) {
@@ -870,7 +871,7 @@ __global__ void __launch_bounds__(kAdamThreads)
                  float* __restrict__ loss) {
   __shared__ float buf[256][kAdamParams];
   const int p0 = blockIdx.x * kAdamParams, p = p0 + threadIdx.x;
-  const float g = sum_parts(part, nparts, p0, buf);
+  const float g = sum_parts(part, nparts, p0, kParams + 1, buf);
   if (threadIdx.x >= kAdamParams) return;
   if (p < kParams) grad[p] = g;
   if (p == kParams) *loss = __fmul_rn(g, inv_2b);
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(kAdamThreads)
     const int k = threadIdx.x - (kAdamThreads - 2);
     s_bc[k] = (float)(1.0 - pow(k == 0 ? (double)kBeta1 : (double)kBeta2, (double)t0 + 1.0));
   }
-  const float g = sum_parts(part, nparts, p0, buf);
+  const float g = sum_parts(part, nparts, p0, loss_hist ? kParams + 1 : kParams, buf);  // the last entry: the loss
   __syncthreads();
   if (threadIdx.x >= kAdamParams) return;
   if (p == kParams) {
