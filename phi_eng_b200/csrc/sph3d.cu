@@ -45,6 +45,14 @@ constexpr uint32_t kMaxParticles3D = 4096;  // MAX_PARTICLES_3D (fluid3.rs:28)
 // Most particles one 3D resample pass (fluid3.rs:923-990) can leave from n:
 // a split only happens while the output holds fewer than MAX_PARTICLES_3D - 1
 // particles, so at most MAX_PARTICLES_3D / 2 particles split.
+// Rows of the state kept on the host, so that further reads, and a read after a
+// write, stay host copies as long as the state stands. Written rows: 96 take 3 us
+// kept and 12 sent at once, 16,384 and more are faster sent. Read rows: up to 4,096
+// from the first read on (the packing kernel writes them there itself), above that
+// from the second read of the same state on (16,384 rows: 46 us from the device, 8
+// kept), and none above 131,072, where a read from the device takes no longer than
+// the host's loop did (262,144 rows: 339 against 419).
+constexpr uint32_t kSetRows = 8192, kKeepRows = 4096, kKeepRowsAgain = 131072;
 inline uint32_t resample_bound3(uint32_t n) { return n + std::min(n, kMaxParticles3D / 2); }
 constexpr uint32_t kMaskBits3 = 32;
 
@@ -1480,7 +1488,14 @@ struct World3 {
   bool bodies_dirty = true;
   uint32_t cap = kMaxParticles3D;
   uint32_t n = 0;
-  std::vector<float4> h_pos, h_vel;
+  std::vector<float4> h_pos, h_vel;  // the state while host_valid
+  // the state's first rows_n rows in the caller's layout, as read or set last
+  // (host_valid or not), in h_rows or, page-locked, behind h_pinned's words;
+  // read_past: this state was read past them
+  std::vector<float> h_rows;
+  const float* rows = nullptr;
+  uint32_t rows_n = 0;
+  bool read_past = false;
   std::vector<float> h_mass, h_dens, h_pres;  // density / pressure as of dp_dev == false
   std::vector<uint8_t> h_phase;
   bool mass_uniform = true, phase_uniform = true;
@@ -1584,7 +1599,7 @@ bool ensure_device3(World3* w) {
   if (!ok3(w, cudaStreamCreateWithFlags(&w->own_stream, cudaStreamNonBlocking))) return false;
   if (!w->user_stream) w->stream = w->own_stream;
   if (!ok3(w, cudaMalloc(&w->scalar, 128)) || !ok3(w, cudaMemset(w->scalar, 0, 128))) return false;
-  if (!ok3(w, cudaMallocHost(&w->h_pinned, 64))) return false;
+  if (!ok3(w, cudaMallocHost(&w->h_pinned, 64 + 24 * kKeepRows))) return false;
   w->device = dev;
   return true;
 }
@@ -1611,8 +1626,24 @@ bool ensure_capacity3(World3* w, uint32_t need) {
   return true;
 }
 
+// The host's copies no longer hold the state: the device has a newer one.
+void state_on_device3(World3* w) {
+  w->host_valid = false;
+  w->rows_n = 0;
+  w->read_past = false;
+}
+
 bool ensure_host3(World3* w) {
   if (w->host_valid) return true;
+  if (w->rows_n == w->n) {
+    for (uint32_t i = 0; i < w->n; i++) {
+      const float* q = w->rows + 6 * (size_t)i;
+      w->h_pos[i] = make_float4(q[0], q[1], q[2], 0.0f);
+      w->h_vel[i] = make_float4(q[3], q[4], q[5], 0.0f);
+    }
+    w->host_valid = true;
+    return true;
+  }
   if (!ok3(w, cudaMemcpyAsync(w->h_pos.data(), w->pos, sizeof(float4) * w->n, cudaMemcpyDeviceToHost, w->stream)) ||
       !ok3(w, cudaMemcpyAsync(w->h_vel.data(), w->vel, sizeof(float4) * w->n, cudaMemcpyDeviceToHost, w->stream)) ||
       !ok3(w, cudaStreamSynchronize(w->stream)))
@@ -1770,6 +1801,15 @@ void enqueue_keys3(World3* w, cudaStream_t st) {
   if (w->n) k_keys3<<<cdiv(w->n, 256), 256, 0, st>>>(w->pos, w->n, w->plan, w->key, w->count);
 }
 
+// Rows of the caller's layout into the device state (through the mask array,
+// which holds nothing between steps), in stream order.
+bool upload_rows3(World3* w, const float* rows) {
+  float2* d = reinterpret_cast<float2*>(w->nmask);
+  if (!ok3(w, cudaMemcpyAsync(d, rows, 24 * (size_t)w->n, cudaMemcpyHostToDevice, w->stream))) return false;
+  k_unpack3<<<cdiv(w->n, 256), 256, 0, w->stream>>>(d, w->n, w->pos, w->vel);
+  return ok3(w, cudaGetLastError());
+}
+
 bool prepare3(World3* w) {
   if (w->error != PHIENG_SPH_OK) return false;
   if (!ensure_device3(w)) return false;
@@ -1777,12 +1817,18 @@ bool prepare3(World3* w) {
     // adaptive resolution: room for what a resample pass can output
     if (!ensure_capacity3(w, w->cfg.adaptive_resolution ? std::max(resample_bound3(w->n), kMaxParticles3D) : w->n))
       return false;
-    if (!w->plan_valid) plan_grid3(w);
-    if (w->n && (!ok3(w, cudaMemcpyAsync(w->pos, w->h_pos.data(), sizeof(float4) * w->n, cudaMemcpyHostToDevice,
-                                         w->stream)) ||
-                 !ok3(w, cudaMemcpyAsync(w->vel, w->h_vel.data(), sizeof(float4) * w->n, cudaMemcpyHostToDevice,
-                                         w->stream))))
+    if (!w->plan_valid) {
+      if (!ensure_host3(w)) return false;
+      plan_grid3(w);
+    }
+    if (!w->host_valid) {
+      if (!upload_rows3(w, w->rows)) return false;
+    } else if (w->n && (!ok3(w, cudaMemcpyAsync(w->pos, w->h_pos.data(), sizeof(float4) * w->n,
+                                                cudaMemcpyHostToDevice, w->stream)) ||
+                        !ok3(w, cudaMemcpyAsync(w->vel, w->h_vel.data(), sizeof(float4) * w->n,
+                                                cudaMemcpyHostToDevice, w->stream)))) {
       return false;
+    }
     w->dev_valid = true;
     w->keys_valid = false;
   }
@@ -2197,7 +2243,7 @@ bool run_substeps3(World3* w, const StepParams3& P, uint32_t count) {
     w->gruns = std::min(w->gruns + k, kGraphAfter);
     w->sid_perm_n = w->n;
     w->substeps += k;
-    w->host_valid = false;
+    state_on_device3(w);
     w->dp_dev = true;
     w->keys_valid = true;
     count -= k;
@@ -2307,7 +2353,7 @@ bool run_substep3_adaptive(World3* w, float dt) {
   w->n = n2;
   recompute_uniformity3(w);
   w->aux_valid = true;
-  w->host_valid = false;
+  state_on_device3(w);
   P = make_params3(w, dt);
   enqueue_keys3(w, st);
   w->sid_perm_n = 0;
@@ -2386,6 +2432,7 @@ uint32_t add_particles3(World3* w, const float* xyz, const uint8_t* phases, uint
     w->h_phase.push_back(ph);
   }
   w->n += n;
+  w->rows_n = 0;
   recompute_uniformity3(w);
   w->dev_valid = w->aux_valid = w->plan_valid = w->keys_valid = false;
   return n;
@@ -2682,7 +2729,7 @@ bool step_fluid_bodies3(World3* w, PhiengBody3* bodies, uint32_t nb, float dt, c
     w->substeps++;
   }
   if (!ok3(w, cudaGetLastError())) return false;
-  w->host_valid = false;
+  state_on_device3(w);
   w->dp_dev = true;
   w->keys_valid = true;
   if (nb) {
@@ -2914,6 +2961,7 @@ int32_t phieng_world3_fluid_clear(World3* w) {
   w->dp_dev = false;
   recompute_uniformity3(w);
   w->host_valid = true;
+  w->rows_n = 0;
   w->dev_valid = w->aux_valid = w->plan_valid = w->keys_valid = false;
   return 1;
 }
@@ -2923,14 +2971,29 @@ uint32_t phieng_world3_fluid_get(const World3* cw, float* out, uint32_t max) {
   World3* w = const_cast<World3*>(cw);
   const uint32_t n = std::min(max, w->n);
   if (n && !w->host_valid) {
-    // rows made on the device (in the mask array, which holds nothing between
-    // steps), then one copy into the caller's buffer
-    float2* rows = reinterpret_cast<float2*>(w->nmask);
-    k_pack3<<<cdiv(n, 256), 256, 0, w->stream>>>(w->pos, w->vel, n, rows);
-    if (!ok3(w, cudaGetLastError()) ||
-        !ok3(w, cudaMemcpyAsync(out, rows, 24 * (size_t)n, cudaMemcpyDeviceToHost, w->stream)) ||
-        !ok3(w, cudaStreamSynchronize(w->stream)))
-      return 0;
+    if (w->rows_n < n) {
+      // rows made on the device: few straight into page-locked memory, the others
+      // in the mask array, which holds nothing between steps, then one copy
+      const bool few = n <= kKeepRows, keep = few || (n <= kKeepRowsAgain && w->read_past);
+      float* to = few ? reinterpret_cast<float*>(w->h_pinned + 16) : out;
+      if (keep && !few) {
+        if (w->h_rows.size() < 6 * (size_t)n) w->h_rows.resize(6 * (size_t)n);
+        to = w->h_rows.data();
+      }
+      float2* made = reinterpret_cast<float2*>(few ? to : reinterpret_cast<float*>(w->nmask));
+      k_pack3<<<cdiv(n, 256), 256, 0, w->stream>>>(w->pos, w->vel, n, made);
+      if (!ok3(w, cudaGetLastError()) ||
+          (!few && !ok3(w, cudaMemcpyAsync(to, made, 24 * (size_t)n, cudaMemcpyDeviceToHost, w->stream))) ||
+          !ok3(w, cudaStreamSynchronize(w->stream)))
+        return 0;
+      if (!keep) {
+        w->read_past = true;
+        return n;
+      }
+      w->rows = to;
+      w->rows_n = n;
+    }
+    std::memcpy(out, w->rows, 24 * (size_t)n);
     return n;
   }
   for (uint32_t i = 0; i < n; i++) {
@@ -2979,6 +3042,7 @@ int64_t phieng_sph3_fluid_block_load(World3* w, uint32_t version, const uint8_t*
   w->n = n;
   recompute_uniformity3(w);
   w->host_valid = true;
+  w->rows_n = 0;
   w->dp_dev = false;
   w->dev_valid = w->aux_valid = w->plan_valid = w->keys_valid = false;
   release_graph3(w);
@@ -3087,23 +3151,27 @@ int32_t phieng_sph3_set_state(World3* w, const float* xyzv, uint32_t n) {
   if (bad) return 0;
   if (n == w->n && n && w->pos && w->dcap >= n && w->error == PHIENG_SPH_OK && w->cfg.smoothing_length > 0.0f &&
       !w->cfg.adaptive_resolution) {
-    // the whole set, with its device arrays there: rows straight to the device
-    // (through the mask array, which holds nothing between steps); the grid is
-    // planned from their bounds. At 10^6 particles the host's copies and its
-    // pass over every particle for the plan took 18 ms, this takes 4.
+    // the whole set, with its device arrays there: the rows go to the device as
+    // they are and the grid is planned from their bounds. At 10^6 particles the
+    // host's copies and its pass over every particle for the plan took 18 ms,
+    // this takes 4. Few rows are kept here and uploaded by the next step; many
+    // go straight from the caller's buffer.
     if (!ensure_host_dp3(w)) return 0;
-    float2* rows = reinterpret_cast<float2*>(w->nmask);
-    if (!ok3(w, cudaMemcpyAsync(rows, xyzv, 24 * (size_t)n, cudaMemcpyHostToDevice, w->stream))) return 0;
-    k_unpack3<<<cdiv(n, 256), 256, 0, w->stream>>>(rows, n, w->pos, w->vel);
-    const cudaError_t launched = cudaGetLastError();
+    const bool keep = n <= kSetRows;
+    if (keep)
+      w->h_rows.assign(xyzv, xyzv + 6 * (size_t)n);
+    else if (!upload_rows3(w, xyzv))
+      return 0;
     Bounds3 b;
     for (uint32_t i = 0; i < n; i++) b.add(xyzv[6 * (size_t)i], xyzv[6 * (size_t)i + 1], xyzv[6 * (size_t)i + 2]);
-    // the rows are the caller's own: from page-locked memory the copy is still
-    // on its way here, and the caller may refill or free them at once
-    if (!ok3(w, cudaStreamSynchronize(w->stream)) || !ok3(w, launched)) return 0;
+    // from page-locked memory the copy is still on its way here, and the caller
+    // may refill or free the buffer at once
+    if (!keep && !ok3(w, cudaStreamSynchronize(w->stream))) return 0;
     plan_bounds3(w, b);
-    w->dev_valid = true;
-    w->host_valid = false;
+    state_on_device3(w);
+    w->rows = w->h_rows.data();
+    w->rows_n = keep ? n : 0;
+    w->dev_valid = !keep;
     w->keys_valid = false;
     return 1;
   }
@@ -3113,6 +3181,7 @@ int32_t phieng_sph3_set_state(World3* w, const float* xyzv, uint32_t n) {
     w->h_pos[i] = make_float4(q[0], q[1], q[2], 0.0f);
     w->h_vel[i] = make_float4(q[3], q[4], q[5], 0.0f);
   }
+  w->rows_n = 0;
   w->dev_valid = false;
   w->keys_valid = false;
   w->plan_valid = false;
