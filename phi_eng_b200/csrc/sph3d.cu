@@ -1513,7 +1513,6 @@ struct World3 {
   uint64_t substeps = 0;
   // device arrays
   uint32_t dcap = 0;
-  unsigned char* block = nullptr;  // the arrays of dcap entries that follow, in one allocation
   float4 *pos = nullptr, *vel = nullptr, *spos = nullptr, *svel = nullptr;
   float *mass = nullptr, *smass = nullptr, *spres = nullptr, *tmp = nullptr;
   uint8_t *phase = nullptr, *sphase = nullptr;
@@ -1580,8 +1579,10 @@ void release_graph3(World3* w) {
 }
 
 void free_particles3(World3* w) {
-  dfree3(w->block);
-  w->pos = nullptr;
+  dfree3(w->pos), dfree3(w->vel), dfree3(w->spos), dfree3(w->svel), dfree3(w->mass), dfree3(w->smass);
+  dfree3(w->spres), dfree3(w->tmp), dfree3(w->phase), dfree3(w->sphase), dfree3(w->key), dfree3(w->tkey);
+  dfree3(w->tid), dfree3(w->skey), dfree3(w->sid), dfree3(w->nmask), dfree3(w->sdq), dfree3(w->sq);
+  dfree3(w->pid), dfree3(w->flist);
   w->dcap = 0;
 }
 
@@ -1606,17 +1607,19 @@ bool ensure_device3(World3* w) {
 bool ensure_capacity3(World3* w, uint32_t need) {
   if (need <= w->dcap && w->pos) return true;
   cudaStreamSynchronize(w->stream);
-  const uint32_t least = std::max<uint32_t>(need, 1024);
-  uint32_t c = grown_capacity(w->dcap, least);
+  const uint32_t c = grown_capacity(w->dcap, std::max<uint32_t>(need, 1024));
   free_particles3(w);
   release_graph3(w);
-  auto arrays = [&](Carve& a) {
-    a(w->pos, c), a(w->vel, c), a(w->spos, c), a(w->svel, c), a(w->mass, c), a(w->smass, c), a(w->spres, c);
-    a(w->tmp, 2 * (size_t)c), a(w->phase, c), a(w->sphase, c), a(w->key, c), a(w->tkey, c), a(w->tid, c);
-    a(w->skey, c), a(w->sid, c), a(w->nmask, kMaskWords3 * (size_t)c), a(w->sdq, c), a(w->sq, (size_t)c + 4);
-    a(w->pid, c), a(w->flist, c);
-  };
-  if (!ok3(w, carve_device(w->block, c, least, arrays))) return false;
+  const bool ok = dalloc3(w, w->pos, c) && dalloc3(w, w->vel, c) && dalloc3(w, w->spos, c) && dalloc3(w, w->svel, c) &&
+                  dalloc3(w, w->mass, c) && dalloc3(w, w->smass, c) && dalloc3(w, w->spres, c) &&
+                  dalloc3(w, w->tmp, 2 * (size_t)c) && dalloc3(w, w->phase, c) && dalloc3(w, w->sphase, c) &&
+                  dalloc3(w, w->key, c) && dalloc3(w, w->tkey, c) && dalloc3(w, w->tid, c) && dalloc3(w, w->skey, c) &&
+                  dalloc3(w, w->sid, c) && dalloc3(w, w->nmask, kMaskWords3 * (size_t)c) && dalloc3(w, w->sdq, c) &&
+                  dalloc3(w, w->sq, (size_t)c + 4) && dalloc3(w, w->pid, c) && dalloc3(w, w->flist, c);
+  if (!ok) {
+    free_particles3(w);
+    return false;
+  }
   w->dcap = c;
   w->dev_valid = w->aux_valid = w->keys_valid = false;
   w->sid_perm_n = 0;

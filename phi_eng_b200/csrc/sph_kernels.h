@@ -22,7 +22,6 @@ struct BatchTab {
 // particle index); "sorted order" = (bucket key, id) order of the last sort.
 struct FluidBufs {
   uint32_t cap = 0;          // particle capacity of every per-particle array
-  unsigned char* block = nullptr;  // those arrays' one allocation (but for order)
   float4* state = nullptr;   // id order: (x, y, vx, vy)
   float* mass = nullptr;     // id order (used when F_MASS)
   uint8_t* phase = nullptr;  // id order (used when F_PHASE)

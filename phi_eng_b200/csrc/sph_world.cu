@@ -215,8 +215,23 @@ void dfree(T*& p) {
 
 void free_particle_buffers(FluidBufs& d) {
   dfree(d.order);  // order tags do not survive a reallocation
-  dfree(d.block);
-  d.state = nullptr;
+  dfree(d.state);
+  dfree(d.mass);
+  dfree(d.phase);
+  dfree(d.key);
+  dfree(d.tkey);
+  dfree(d.tid);
+  dfree(d.skey);
+  dfree(d.sid);
+  dfree(d.pid);
+  dfree(d.flist);
+  dfree(d.spos);
+  dfree(d.svel);
+  dfree(d.smass);
+  dfree(d.sphase);
+  dfree(d.sdq);
+  dfree(d.spres);
+  dfree(d.nmask);
   d.cap = 0;
 }
 
@@ -265,16 +280,15 @@ bool ensure_capacity(World2* w, uint32_t need) {
   FluidBufs& d = w->d;
   if (need <= d.cap && d.state) return true;
   cudaStreamSynchronize(w->stream);
-  const uint32_t least = std::max<uint32_t>(need, 1024);
-  uint32_t c = grown_capacity(d.cap, least);
+  const uint32_t c = grown_capacity(d.cap, std::max<uint32_t>(need, 1024));
   free_particle_buffers(d);
   release_graph(w);
-  auto arrays = [&](Carve& a) {
-    a(d.state, c), a(d.mass, c), a(d.phase, c), a(d.key, c), a(d.tkey, c), a(d.tid, c), a(d.skey, c), a(d.sid, c);
-    a(d.pid, c), a(d.flist, c), a(d.spos, (size_t)c + 1), a(d.svel, c), a(d.smass, c), a(d.sphase, c), a(d.sdq, c);
-    a(d.spres, c), a(d.nmask, 3 * (size_t)c);
-  };
-  bool ok = cuda_ok(w, carve_device(d.block, c, least, arrays), "cudaMalloc");
+  bool ok = dalloc(w, d.state, c) && dalloc(w, d.mass, c) && dalloc(w, d.phase, c) && dalloc(w, d.key, c) &&
+            dalloc(w, d.tkey, c) && dalloc(w, d.tid, c) &&
+            dalloc(w, d.skey, c) && dalloc(w, d.sid, c) && dalloc(w, d.pid, c) && dalloc(w, d.flist, c) &&
+            dalloc(w, d.spos, (size_t)c + 1) && dalloc(w, d.svel, c) &&
+            dalloc(w, d.smass, c) && dalloc(w, d.sphase, c) && dalloc(w, d.sdq, c) && dalloc(w, d.spres, c) &&
+            dalloc(w, d.nmask, 3 * (size_t)c);
   if (ok && w->is_batch()) {
     dfree(w->d_pscene);
     dfree(w->d_sscene);
