@@ -199,24 +199,35 @@ __device__ __forceinline__ bool quick_range(float x, float y, float z, float uni
 }
 
 // hit(j) for the slots j of [rs, re), ascending, that can hold a neighbour of
-// the particle with word qi: those that pass the quick test, or all. hit
-// returns whether the slot does hold one; those of the first 64 slots are the
-// row's mask (bit t of mask[t / 32]: slot rs + t). sq is readable up to three
-// entries past any slot.
+// the particle. hit returns whether the slot does hold one; those of the first 64
+// slots are the row's mask (bit t of mask[t / 32]: slot rs + t). In two forms.
+// This one calls it for every slot: for particles without the quick test, and for
+// long rows, where the quick test's hits come as one serial loop per 32 slots that
+// lasts as long as the warp's fullest lane.
 template <class F>
-__device__ __forceinline__ void row_candidates3(uint32_t rs, uint32_t re, bool quick, uint32_t qi,
-                                                const uint32_t* __restrict__ sq, uint32_t (&mask)[2], F&& hit) {
+__device__ __forceinline__ void row_candidates3_plain(uint32_t rs, uint32_t re, uint32_t (&mask)[2], F&& hit) {
   mask[0] = mask[1] = 0u;
-  if (!quick) {
+  uint32_t j = rs;
 #pragma unroll 1
-    for (uint32_t j = rs; j < re; j++) {
-      const bool nb = hit(j);
-      const uint32_t t = j - rs;
-      if (t < 32u) mask[0] |= (nb ? 1u : 0u) << t;
-      else if (t < 64u) mask[1] |= (nb ? 1u : 0u) << (t - 32u);
+  for (uint32_t word = 0; j < re; word++) {
+    const uint32_t end = word < 2u ? min(re, j + kMaskBits3) : re;
+    uint32_t m = 0, bit = 1u;
+#pragma unroll 4
+    for (; j < end; j++) {
+      m |= hit(j) ? bit : 0u;
+      bit <<= 1;
     }
-    return;
+    if (word == 0u) mask[0] = m;
+    else if (word == 1u) mask[1] = m;
   }
+}
+
+// This one only for those that pass the quick test with the particle's word qi.
+// sq is readable up to three entries past any slot.
+template <class F>
+__device__ __forceinline__ void row_candidates3(uint32_t rs, uint32_t re, uint32_t qi, const uint32_t* __restrict__ sq,
+                                                uint32_t (&mask)[2], F&& hit) {
+  mask[0] = mask[1] = 0u;
 #pragma unroll 1
   for (uint32_t a = rs & ~3u; a < re; a += 32u) {  // 32 slots, their results shifted into a word from the right
     const uint32_t end = min(a + 32u, re);
@@ -745,20 +756,33 @@ __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spo
     if (!seam) {
       // the rows' slot ranges, loaded up front
       uint32_t rsa[9], rea[9];
+      bool plain = !quick;
 #pragma unroll
       for (int r = 0; r < 9; r++) {
         const uint32_t row = row_base3(by, bz, r, g);
         rsa[r] = __ldg(&start[row + bx - 1u]);
         rea[r] = __ldg(&start[row + bx + 2u]);
+        plain = plain || rea[r] - rsa[r] > kMaskBits3;
       }
+      // plain: a row of more than 32 slots, or out of the quick test's range. All
+      // rows of the warp then: 262,144 particles 0.2 apart (h 0.5) 111 -> 102 us,
+      // 0.17 apart 168 -> 149, 0.25 apart and 40 km out 82 -> 53 (43 with the test)
+      if (!__any_sync(__activemask(), plain)) {
 #pragma unroll
-      for (int r = 0; r < 9; r++) {
-        const uint32_t len = rea[r] - rsa[r];
-        row_candidates3(rsa[r], rea[r], quick, qi, sq, m, hit);
-        nmask[(size_t)r * n + s] = m[0];
-        if (len > kMaskBits3) {
-          nmask[(size_t)(9 + r) * n + s] = m[1];
-          flags |= len > 2u * kMaskBits3 ? kNoMasks : 1u << r;
+        for (int r = 0; r < 9; r++) {
+          row_candidates3(rsa[r], rea[r], qi, sq, m, hit);
+          nmask[(size_t)r * n + s] = m[0];
+        }
+      } else {
+#pragma unroll 1
+        for (int r = 0; r < 9; r++) {
+          const RowRange3 q = row_range3(row_base3(by, bz, r, g), bx, false, g, start);
+          row_candidates3_plain(q.rs, q.re, m, hit);
+          nmask[(size_t)r * n + s] = m[0];
+          if (q.re - q.rs > kMaskBits3) {
+            nmask[(size_t)(9 + r) * n + s] = m[1];
+            flags |= q.re - q.rs > 2u * kMaskBits3 ? kNoMasks : 1u << r;
+          }
         }
       }
     } else {
@@ -766,7 +790,7 @@ __global__ void __launch_bounds__(256) k_density3(const float4* __restrict__ spo
       for (uint32_t t = 0; t < 18u; t++) {  // row t / 2's part before the wrap, then the one after it
         const RowRange3 q = row_range3(row_base3(by, bz, (int)(t / 2u), g), bx, true, g, start);
         const uint32_t rs = t & 1u ? q.rs2 : q.rs, re = t & 1u ? q.re2 : q.re;
-        row_candidates3(rs, re, quick, qi, sq, m, hit);
+        row_candidates3_plain(rs, re, m, hit);
         nmask[(size_t)(t / 2u + (t & 1u ? 9u : 0u)) * n + s] = m[0];
         flags |= re - rs > kMaskBits3 ? kNoMasks : 1u << t / 2u;
       }
@@ -1215,7 +1239,7 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
   if (k != g.sentinel) {
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
     const uint32_t flags = nmask[18 * (size_t)n + s];
-    if (!(flags & kNoMasks)) {
+    if (!__any_sync(__activemask(), flags & kNoMasks)) {
       // the nine rows' masks and first slots, loaded up front (independent
       // loads; none inside the divergent loops below)
       uint32_t mk[18], bs[18];
@@ -1255,22 +1279,36 @@ __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restr
         }
       }
     } else {
+      // particles without masks in the warp (rows too long for them): all its
+      // lanes walk, 32 candidates tested at a time, then their neighbours' pairs.
+      // With the pair inside the test a warp evaluated one for nearly every
+      // candidate, and lanes with masks went their own way first: 262,144
+      // particles 0.2 apart (h 0.5) 674 -> 412 us, in the tolerance mode 303 -> 205
+      // (0.25 apart, where all have masks: 80 and 38).
+      const bool seam = on_seam3(bx, g);
 #pragma unroll 1
-      for (int r = 0; r < 9; r++) {
-        const uint32_t row = row_base3(by, bz, r, g);
+      for (uint32_t t = 0; t < (seam ? 18u : 9u); t++) {  // on the seam a row's part before the wrap, then the one after it
+        const RowRange3 q = row_range3(row_base3(by, bz, (int)(seam ? t / 2u : t), g), bx, seam, g, start);
+        const bool after = seam && (t & 1u);
+        const uint32_t rs = after ? q.rs2 : q.rs, re = after ? q.re2 : q.re;
 #pragma unroll 1
-        for (int ox = -1; ox <= 1; ox++) {
-          const uint32_t bb = row | ((bx + (uint32_t)ox) & g.maskw);
-          const uint32_t e = __ldg(&start[bb + 1]);
-          for (uint32_t j = __ldg(&start[bb]); j < e; j++) {
-            const float4 a = __ldg(&spos[j]);
-            const float ex = __fsub_rn(a.x, pi.x), ey = __fsub_rn(a.y, pi.y), ez = __fsub_rn(a.z, pi.z);
-            if (dot3(ex, ey, ez, ex, ey, ez) < P.hg2 && j != s) {
-              if constexpr (FAST)
-                pair3_fast(j, pi, vi, rho_i, mq_i, spos, svel, sdq, P, f, sm);
-              else
-                pair3<MASS, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, P, f, sm);
-            }
+        for (uint32_t a = rs; a < re; a += kMaskBits3) {
+          const uint32_t end = min(a + kMaskBits3, re);
+          uint32_t m = 0, bit = 1u;
+#pragma unroll 4
+          for (uint32_t j = a; j < end; j++) {
+            const float4 c = __ldg(&spos[j]);
+            const float ex = __fsub_rn(c.x, pi.x), ey = __fsub_rn(c.y, pi.y), ez = __fsub_rn(c.z, pi.z);
+            m |= dot3(ex, ey, ez, ex, ey, ez) < P.hg2 ? bit : 0u;
+            bit <<= 1;
+          }
+          if (s - a < kMaskBits3) m &= ~(1u << (s - a));  // j != i
+          for (; m; m &= m - 1u) {
+            const uint32_t j = a + (uint32_t)(__ffs((int)m) - 1);
+            if constexpr (FAST)
+              pair3_fast(j, pi, vi, rho_i, mq_i, spos, svel, sdq, P, f, sm);
+            else
+              pair3<MASS, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, P, f, sm);
           }
         }
       }

@@ -11,6 +11,7 @@
 // order, so every result has the bits of the one-thread passes; the row masks
 // between the two passes are the same too.
 constexpr uint32_t kRowTerms = 32;      // density terms kept per row
+constexpr uint32_t kRowCount = 0xFFFFFFu;
 constexpr uint32_t kCoopPairs = 128;    // listed neighbours of a group
 constexpr uint32_t kCoopThreads = 256;  // block of the force pass
 // Lanes per particle of the force pass: 8 and 32 differ by 5 % on 64 to 4,096
@@ -21,14 +22,18 @@ constexpr int kCoopLanes = 8;
 // particles, density by rows against one thread per particle: 38.2 / 46.5,
 // 46.7 / 49.3, 53.4 / 52.1 us (tolerance mode). Force by eight lanes against one
 // thread, rows in both: exact 36.3 / 47.4, 52.2 / 56.3, 63.3 / 62.0; tolerance
-// mode 36.6 / 38.2, 51.9 / 46.7, 63.8 / 53.4.
+// mode 36.6 / 38.2, 51.9 / 46.7, 63.8 / 53.4. Of compressed sets only those of
+// several times the rest density are faster by one thread (0.2 apart at h 0.5 and
+// 32,768 particles: 12 steps 1,254 us against 1,394 before these passes' last change,
+// 0.12 apart 5,188 against 4,173).
 constexpr uint32_t kRowsMax3 = 49152;
 constexpr uint32_t kCoopMax3 = 49152, kCoopMaxFast3 = 24576;
 
 // Density + EOS. Warp r of a block walks row r of the block's 32 particles,
 // one per lane, and keeps the neighbours' terms; warp 0 then sums each
-// particle's terms row by row. A row with more than kRowTerms neighbours sends
-// its particle through a walk of all candidates by one thread.
+// particle's terms row by row. Of a row with more than kRowTerms neighbours
+// warp 0 walks all but the first 32 slots itself (the particle's 27 cells anew:
+// 32,768 particles 0.17 apart, h 0.5, 120 us instead of 48).
 template <bool MASS, bool PHASE, bool WIDE>
 __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict__ spos,
                                                        const uint32_t* __restrict__ skey,
@@ -40,7 +45,7 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
                                                        uint32_t* __restrict__ nmask) {
   chain_wait(spos, skey, smass, sphase, start, sq);
   __shared__ float terms[9][kRowTerms][32];
-  __shared__ uint32_t row_cnt[9][32];  // neighbours of the row; bits 30, 31: it has a second word, no mask
+  __shared__ uint32_t row_cnt[9][32];  // kRowCount: neighbours; 24..29: those of m[0]; 30, 31: a second word, no masks
   const uint32_t p = threadIdx.x & 31u, r = threadIdx.x >> 5;
   const uint32_t s = blockIdx.x * 32u + p;
   const bool active = s < n;
@@ -59,7 +64,7 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
     for (uint32_t part = 0; part < (seam ? 2u : 1u); part++) {
       uint32_t found[2];
       const uint32_t rs = part ? q.rs2 : q.rs, re = part ? q.re2 : q.re;
-      row_candidates3(rs, re, quick, qi, sq, found, [&](uint32_t j) {
+      auto hit = [&](uint32_t j) {
         const float4 a = __ldg(&spos[j]);
         const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
         const float d2 = dot3(dx, dy, dz, dx, dy, dz);
@@ -68,14 +73,19 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
         if (cnt < kRowTerms) terms[r][cnt][p] = __fmul_rn(MASS ? __ldg(&smass[j]) : P.mass, poly6_nb<WIDE>(d2, P));
         cnt += nb ? 1u : 0u;
         return nb;
-      });
+      };
+      // long rows plainly; up to 64 slots the quick test still pays here, where a
+      // warp waits for one row only (30 steps of a 4,096-particle column 709 us, with
+      // the line at 32 725; 16,384 particles 0.2 apart the same either way)
+      if (__any_sync(__activemask(), !quick || re - rs > 2u * kMaskBits3)) row_candidates3_plain(rs, re, found, hit);
+      else row_candidates3(rs, re, qi, sq, found, hit);
       if (part) m[1] = found[0];
       else m[0] = found[0], m[1] = found[1];
     }
     const uint32_t len = max(q.re - q.rs, q.re2 - q.rs2);
     kind = len > (seam ? 1u : 2u) * kMaskBits3 ? 2u : seam || len > kMaskBits3 ? 1u : 0u;
   }
-  row_cnt[r][p] = cnt | kind << 30;
+  row_cnt[r][p] = cnt | (uint32_t)__popc(m[0]) << 24 | kind << 30;
   if (active) {
     nmask[(size_t)r * n + s] = m[0];
     if (kind == 1u) nmask[(size_t)(9u + r) * n + s] = m[1];
@@ -83,32 +93,49 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
   __syncthreads();
   if (r != 0u || !active) return;
   float rho = 0.0f;
-  bool fits = true;
   uint32_t flags = 0u;
+  bool fits = true;
 #pragma unroll
   for (int q = 0; q < 9; q++) {
-    const uint32_t c = row_cnt[q][p] & 0x3FFFFFFFu, kd = row_cnt[q][p] >> 30;
+    const uint32_t kd = row_cnt[q][p] >> 30;
     flags |= kd == 0u ? 0u : kd == 1u ? 1u << q : kNoMasks;
-    fits = fits && c <= kRowTerms;
-    for (uint32_t i = 0; i < min(c, kRowTerms); i += 4) {
+    fits = fits && (row_cnt[q][p] & kRowCount) <= kRowTerms;
+  }
+  auto add_terms = [&](int q, uint32_t c) {
+    for (uint32_t i = 0; i < c; i += 4) {
 #pragma unroll
       for (uint32_t t = 0; t < 4; t++) {
         const float w = terms[q][i + t][p];
         rho = i + t < c ? __fadd_rn(rho, w) : rho;
       }
     }
-  }
-  if (!fits) {
-    rho = 0.0f;
+  };
+  if (fits) {
+#pragma unroll
+    for (int q = 0; q < 9; q++) add_terms(q, row_cnt[q][p] & kRowCount);
+  } else {
     const uint32_t bx = k & g.maskw, by = (k >> g.log2w) & g.maskh, bz = k >> (g.log2w + g.log2h);
+    const bool seam = on_seam3(bx, g);
 #pragma unroll 1
-    for (int q = 0; q < 27; q++) {
-      const uint32_t b = row_base3(by, bz, q / 3, g) | ((bx + (uint32_t)(q % 3) - 1u) & g.maskw);
-      const uint32_t e = __ldg(&start[b + 1]);
-      for (uint32_t j = __ldg(&start[b]); j < e; j++) {
-        const float4 a = __ldg(&spos[j]);
-        const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
-        rho = __fadd_rn(rho, contrib3(dot3(dx, dy, dz, dx, dy, dz), MASS ? __ldg(&smass[j]) : P.mass, P));
+    for (int q = 0; q < 9; q++) {
+      const uint32_t c = row_cnt[q][p] & kRowCount;
+      if (c <= kRowTerms) {
+        add_terms(q, c);
+        continue;
+      }
+      add_terms(q, row_cnt[q][p] >> 24 & 63u);  // those of the row's first 32 slots; then from there on
+      const RowRange3 rr = row_range3(row_base3(by, bz, q, g), bx, seam, g, start);
+#pragma unroll 1
+      for (uint32_t part = 0; part < (seam ? 2u : 1u); part++) {
+        const uint32_t e = part ? rr.re2 : rr.re;
+#pragma unroll 8
+        for (uint32_t j = part ? rr.rs2 : rr.rs + kMaskBits3; j < e; j++) {
+          const float4 a = __ldg(&spos[j]);
+          const float dx = __fsub_rn(a.x, pi.x), dy = __fsub_rn(a.y, pi.y), dz = __fsub_rn(a.z, pi.z);
+          const float d2 = dot3(dx, dy, dz, dx, dy, dz);
+          const float w = __fmul_rn(MASS ? __ldg(&smass[j]) : P.mass, poly6_nb<WIDE>(d2, P));
+          rho = d2 < P.hg2 ? __fadd_rn(rho, w) : rho;
+        }
       }
     }
   }
