@@ -67,6 +67,7 @@ constexpr uint32_t kMaskBits3 = 32;
 constexpr float kCellUnits = 64.0f;
 constexpr float kQuickUnits = 2097152.0f;  // 2^21
 constexpr int kQuickD2 = 4604;
+constexpr int kEverySlot = 1 << 20;  // more than any d . d: the test passes every slot
 
 struct GridPlan3 {
   int32_t cx0, cy0, cz0;
@@ -201,9 +202,9 @@ __device__ __forceinline__ bool quick_range(float x, float y, float z, float uni
 // hit(j) for the slots j of [rs, re), ascending, that can hold a neighbour of
 // the particle. hit returns whether the slot does hold one; those of the first 64
 // slots are the row's mask (bit t of mask[t / 32]: slot rs + t). In two forms.
-// This one calls it for every slot: for particles without the quick test, and for
-// long rows, where the quick test's hits come as one serial loop per 32 slots that
-// lasts as long as the warp's fullest lane.
+// This one calls it for every slot: in k_density3 for particles without the quick
+// test, and for long rows, where the quick test's hits come as one serial loop per
+// 32 slots that lasts as long as the warp's fullest lane.
 template <class F>
 __device__ __forceinline__ void row_candidates3_plain(uint32_t rs, uint32_t re, uint32_t (&mask)[2], F&& hit) {
   mask[0] = mask[1] = 0u;
@@ -222,11 +223,12 @@ __device__ __forceinline__ void row_candidates3_plain(uint32_t rs, uint32_t re, 
   }
 }
 
-// This one only for those that pass the quick test with the particle's word qi.
+// This one only for those that pass the quick test with the particle's word qi
+// (limit kEverySlot: all).
 // sq is readable up to three entries past any slot.
 template <class F>
 __device__ __forceinline__ void row_candidates3(uint32_t rs, uint32_t re, uint32_t qi, const uint32_t* __restrict__ sq,
-                                                uint32_t (&mask)[2], F&& hit) {
+                                                uint32_t (&mask)[2], F&& hit, int limit = kQuickD2) {
   mask[0] = mask[1] = 0u;
 #pragma unroll 1
   for (uint32_t a = rs & ~3u; a < re; a += 32u) {  // 32 slots, their results shifted into a word from the right
@@ -236,7 +238,7 @@ __device__ __forceinline__ void row_candidates3(uint32_t rs, uint32_t re, uint32
       const uint4 q = __ldg(reinterpret_cast<const uint4*>(sq + j));
       auto test = [&](uint32_t w) {
         const int d = (int)(w - qi);
-        bits = __funnelshift_l((uint32_t)__dp4a(d, d, -kQuickD2), bits, 1);  // negative: near
+        bits = __funnelshift_l((uint32_t)__dp4a(d, d, -limit), bits, 1);  // negative: near
       };
       test(q.x);
       test(q.y);

@@ -74,11 +74,7 @@ __global__ void __launch_bounds__(288) k_density3_rows(const float4* __restrict_
         cnt += nb ? 1u : 0u;
         return nb;
       };
-      // long rows plainly; up to 64 slots the quick test still pays here, where a
-      // warp waits for one row only (30 steps of a 4,096-particle column 709 us, with
-      // the line at 32 725; 16,384 particles 0.2 apart the same either way)
-      if (__any_sync(__activemask(), !quick || re - rs > 2u * kMaskBits3)) row_candidates3_plain(rs, re, found, hit);
-      else row_candidates3(rs, re, qi, sq, found, hit);
+      row_candidates3(rs, re, qi, sq, found, hit, quick ? kQuickD2 : kEverySlot);
       if (part) m[1] = found[0];
       else m[0] = found[0], m[1] = found[1];
     }
