@@ -2276,7 +2276,8 @@ bool run_substeps3(World3* w, const StepParams3& P, uint32_t count) {
       w->gsig = sig;
       w->gruns = 0;
     }
-    const bool many = count >= kGraphSteps && w->gruns >= kGraphAfter && w->sid_perm_n == w->n && !w->profiling;
+    const bool many =
+        use_long_graph(w->gsteps != nullptr, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
     if (many && !w->gsteps && !capture_substeps3(w, P, kGraphSteps, &w->gsteps)) return false;
     const uint32_t k = many ? kGraphSteps : 1u;
     if (!ok3(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream))) return false;

@@ -24,10 +24,16 @@ constexpr float kMaxDt = 1.0f / 15.0f;          // ffi.rs:80
 // parameters: from one graph to the next the GPU stands still for some 1.5 us
 // that kernels inside a graph do not cost (20 steps of 32,499 particles 432 ->
 // 404 us, 10 steps of 2^18 389 -> 376 us, of 2^20 932 -> 920 us). The longer
-// graph costs another capture, so it is only made for parameters that have run
-// kGraphAfter substeps.
+// graph costs another capture, some 70 us: it is made for parameters that have run
+// kGraphAfter substeps, or kGraphSoon where the call still has kGraphRest to go.
+// Calls of 20, 30 and 100 steps of 32,768 particles, each with a time step of its
+// own: 527, 821 and 2,227 us; always from kGraphSoon on 580, 841 and 2,219.
 constexpr uint32_t kGraphSteps = 4;
-constexpr uint32_t kGraphAfter = 16;
+constexpr uint32_t kGraphSoon = 16, kGraphRest = 32, kGraphAfter = 48;
+// Whether the longer graph runs next: `made` = it is there, `ran` substeps so far.
+inline bool use_long_graph(bool made, uint32_t ran, uint32_t left) {
+  return left >= kGraphSteps && (made || ran >= kGraphAfter || (ran >= kGraphSoon && left >= kGraphRest));
+}
 
 // Capacity for at least `least` particles in place of `had`: an eighth more where
 // a world grows, so that one that takes particles step by step seldom moves. Every

@@ -744,7 +744,8 @@ bool run_substeps(World2* w, const StepParams& P, uint32_t count) {
       w->gsig = sig;
       w->gruns = 0;
     }
-    const bool many = count >= kGraphSteps && w->gruns >= kGraphAfter && w->sid_perm_n == w->n && !w->profiling;
+    const bool many =
+        use_long_graph(w->gsteps != nullptr, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
     if (many && !w->gsteps && !capture_substeps(w, P, kGraphSteps, &w->gsteps)) return false;
     const uint32_t k = many ? kGraphSteps : 1u;
     if (!cuda_ok(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream), "graph launch")) return false;
