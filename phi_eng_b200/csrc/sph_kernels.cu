@@ -342,6 +342,41 @@ __device__ __forceinline__ void for_each_candidate(uint32_t key, const uint32_t*
   }
 }
 
+// f(j) for the neighbours j != s of the particle at pi in sorted slot s and
+// bucket key, in the reference's visit order: 32 candidates tested at a time, then
+// their hits. With f inside the test a warp runs it for nearly every candidate: 8
+// steps of 2^20 particles 0.12 apart (h 0.5), exact mode, 6,129 -> 5,797 us, of 16
+// scenes of 65,536 7,453 -> 6,859. Not for the tolerance mode, whose pairs
+// are short: 3,325 -> 3,569.
+template <class F>
+__device__ __forceinline__ void for_each_neighbour(uint32_t key, const uint32_t* __restrict__ start, const GridPlan& g,
+                                                   const float2* __restrict__ spos, float2 pi, float hg2, uint32_t s,
+                                                   F&& f) {
+  const uint32_t local = key - g.base;
+  const uint32_t bx = local & g.maskw, by = local >> g.log2w;
+  const bool seam = !(bx >= 1u && bx < g.maskw);
+#pragma unroll 1
+  for (uint32_t t = 0; t < (seam ? 9u : 3u); t++) {  // a row's slot range, on the seam bucket by bucket
+    const uint32_t row = g.base + (((by + (seam ? t / 3u : t) - 1u) & g.maskh) << g.log2w);
+    const uint32_t b0 = row + (seam ? (bx + t % 3u - 1u) & g.maskw : bx - 1u);
+    const uint32_t e = __ldg(&start[b0 + (seam ? 1u : 3u)]);
+#pragma unroll 1
+    for (uint32_t a = __ldg(&start[b0]); a < e; a += 32u) {
+      const uint32_t end = min(a + 32u, e);
+      uint32_t m = 0, bit = 1u;
+#pragma unroll 4
+      for (uint32_t j = a; j < end; j++) {
+        const float2 pj = __ldg(&spos[j]);
+        const float ex = __fsub_rn(pj.x, pi.x), ey = __fsub_rn(pj.y, pi.y);
+        m |= __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)) < hg2 ? bit : 0u;
+        bit <<= 1;
+      }
+      if (s - a < 32u) m &= ~(1u << (s - a));
+      for (; m; m &= m - 1u) f(a + (uint32_t)(__ffs((int)m) - 1));
+    }
+  }
+}
+
 // ---------------------------------------------------------------- K5 density
 // Per-row neighbour masks: for the candidate row oy (0..2 for oy = -1..1) of
 // a particle away from the wrap seam, bit t of nmask[oy * n + s] is set iff
@@ -595,14 +630,8 @@ __device__ __forceinline__ void neighbour_sums(uint32_t s, uint32_t k, uint32_t 
       pair_terms<MASS, FEAT, PLAIN>(w.next(), pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, svp, P, fx, fy, sx, sy,
                                     fa);
   } else {
-    for_each_candidate(k, start, g, [&](int jj) {
-      const uint32_t j = (uint32_t)jj;
-      const float2 pj = __ldg(&spos[j]);
-      const float ex = __fsub_rn(pj.x, pi.x);
-      const float ey = __fsub_rn(pj.y, pi.y);
-      const float d2 = __fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey));
-      if (d2 < P.hg2 && j != s)
-        pair_terms<MASS, FEAT, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, svp, P, fx, fy, sx, sy, fa);
+    for_each_neighbour(k, start, g, spos, pi, P.hg2, s, [&](uint32_t j) {
+      pair_terms<MASS, FEAT, PLAIN>(j, pi, vi, rho_i, q_i, m_i, spos, svel, sdq, smass, svp, P, fx, fy, sx, sy, fa);
     });
   }
 }
