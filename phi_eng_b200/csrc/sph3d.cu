@@ -67,6 +67,7 @@ constexpr uint32_t kMaskBits3 = 32;
 constexpr float kCellUnits = 64.0f;
 constexpr float kQuickUnits = 2097152.0f;  // 2^21
 constexpr int kQuickD2 = 4604;
+constexpr float kQuickMinH = 1e-15f;  // below, squares near the underflow round neighbours farther than that
 constexpr int kEverySlot = 1 << 20;  // more than any d . d: the test passes every slot
 
 struct GridPlan3 {
@@ -147,7 +148,7 @@ struct StepParams3 {
   const float4* hullv;
   uint32_t* defer;
   uint32_t* dcount;
-  float cell_units;  // kCellUnits / smoothing_length (NaN where that is not positive)
+  float cell_units;  // kCellUnits / smoothing_length (NaN below kQuickMinH)
 };
 
 // Static body: shape 0 sphere (a = radius), 1 box (a, b, c half extents),
@@ -2104,7 +2105,7 @@ StepParams3 make_params3(const World3* w, float dt) {
   P.flags = f;
   P.nbodies = (uint32_t)w->bodies.size();
   P.uniform_phase = w->phase_value;
-  P.cell_units = c.smoothing_length > 0.0f ? kCellUnits / c.smoothing_length : NAN;
+  P.cell_units = c.smoothing_length >= kQuickMinH ? kCellUnits / c.smoothing_length : NAN;
   if (w->precision == PHIENG_SPH_TOLERANCE) P.flags |= F_FAST;
   return P;
 }
