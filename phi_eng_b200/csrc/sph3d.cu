@@ -1845,6 +1845,7 @@ void enqueue_keys3(World3* w, cudaStream_t st) {
 // Rows of the caller's layout into the device state (through the mask array,
 // which holds nothing between steps), in stream order.
 bool upload_rows3(World3* w, const float* rows) {
+  OnDevice on(w->device);
   float2* d = reinterpret_cast<float2*>(w->nmask);
   if (!ok3(w, cudaMemcpyAsync(d, rows, 24 * (size_t)w->n, cudaMemcpyHostToDevice, w->stream))) return false;
   k_unpack3<<<cdiv(w->n, 256), 256, 0, w->stream>>>(d, w->n, w->pos, w->vel);
@@ -2245,6 +2246,7 @@ void enqueue_substep3(World3* w, const StepParams3& P, cudaStream_t st) {
 }
 
 bool capture_substeps3(World3* w, const StepParams3& P, uint32_t steps, cudaGraphExec_t* out) {
+  OnDevice on(w->device);
   cudaGraph_t g = nullptr;
   if (!ok3(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal))) return false;
   for (uint32_t k = 0; k < steps; k++) enqueue_substep3(w, P, w->own_stream);
@@ -3023,6 +3025,7 @@ uint32_t phieng_world3_fluid_get(const World3* cw, float* out, uint32_t max) {
         to = w->h_rows.data();
       }
       float2* made = reinterpret_cast<float2*>(few ? to : reinterpret_cast<float*>(w->nmask));
+      OnDevice on(w->device);
       k_pack3<<<cdiv(n, 256), 256, 0, w->stream>>>(w->pos, w->vel, n, made);
       if (!ok3(w, cudaGetLastError()) ||
           (!few && !ok3(w, cudaMemcpyAsync(to, made, 24 * (size_t)n, cudaMemcpyDeviceToHost, w->stream))) ||

@@ -35,6 +35,22 @@ inline bool use_long_graph(bool made, uint32_t ran, uint32_t left) {
   return left >= kGraphSteps && (made || ran >= kGraphAfter || (ran >= kGraphSoon && left >= kGraphRest));
 }
 
+// The world's device while in scope, for launches in calls that only copied or
+// replayed graphs before: those take a stream of any device, a kernel launch only
+// one of the calling thread's current device, and a new thread's is device 0.
+struct OnDevice {
+  int was = -1;
+  explicit OnDevice(int dev) {
+    int cur = -1;
+    if (dev >= 0 && cudaGetDevice(&cur) == cudaSuccess && cur != dev && cudaSetDevice(dev) == cudaSuccess) was = cur;
+  }
+  ~OnDevice() {
+    if (was >= 0) cudaSetDevice(was);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+};
+
 // Capacity for at least `least` particles in place of `had`: an eighth more where
 // a world grows, so that one that takes particles step by step seldom moves. Every
 // array that needs new device memory takes ~0.6 ms whatever its size, and there are

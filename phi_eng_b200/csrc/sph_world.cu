@@ -708,6 +708,7 @@ void enqueue_substep_body(World2* w, const StepParams& P, cudaStream_t st) {
 
 // A CUDA graph of `steps` substeps.
 bool capture_substeps(World2* w, const StepParams& P, uint32_t steps, cudaGraphExec_t* out) {
+  OnDevice on(w->device);
   cudaGraph_t g = nullptr;
   if (!cuda_ok(w, cudaStreamBeginCapture(w->own_stream, cudaStreamCaptureModeThreadLocal), "begin capture"))
     return false;
@@ -1103,6 +1104,7 @@ uint32_t run_small(World2* w, float dt, uint32_t steps) {
     ss.substeps_host = reinterpret_cast<unsigned long long*>(w->h_pinned + kSubstepPinned);
   }
   ss.no_cluster = w->no_cluster;
+  OnDevice on(w->device);
   if (!enqueue_small_steps(w->d, w->n, make_params(w, dt), ss, w->stream)) return 0;
   if (!ss.substeps) w->substeps += ss.steps;
   w->host_state_valid = false;
