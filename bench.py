@@ -72,10 +72,11 @@ PHASE_ALG_BYTES = dict(sort_ranges=ALG_BYTES["sort"] + ALG_BYTES["ranges"] + ALG
 DENSITY_BYTES = 36
 FORCE_BYTES = 68
 # DRAM bytes (read + write) of one launch of the named kernel on the named
-# workload and precision mode, from an ncu capture (profiles/).
-PROFILED_TRAFFIC = {("dam_break_1m", "exact", "force_integrate"): 48.333312e6 + 1.921792e6,
-                    ("dam_break_1m", "tolerance", "force_integrate"): 48.337664e6 + 1.710592e6}
-PROFILED_TRAFFIC_3D = {"force_integrate": 85.545216e6 + 14.838528e6}  # 100^3 3D dam break
+# workload and precision mode, from an ncu capture (profiles/counters.md).
+PROFILED_TRAFFIC = {("dam_break_1m", "exact", "force_integrate"): 48.324480e6 + 1.752960e6,
+                    ("dam_break_1m", "tolerance", "force_integrate"): 48.338432e6 + 1.776896e6}
+# 100^3 3D dam break
+PROFILED_TRAFFIC_3D = {"force_integrate": 89.606e6 + 18.430e6, "density": 24.777e6 + 3.967e6}
 KERNELS_PER_STEP = 5  # single-pass scan, place, fix, density, force
 
 
@@ -447,8 +448,8 @@ def fluid3d_line(steps: int, warmup: int, side: int = 100) -> dict:
             "roofline": {"bound": "hbm", "kernel": names[top], "bytes_per_particle": bytes_pp[top],
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": PROFILED_TRAFFIC_3D.get(names[top]) if side == 100 else None,
-                         "traffic_source": "ncu capture of the exact-mode force pass (the tolerance-mode pass "
-                                           "reads and writes the same arrays)"},
+                         "traffic_source": "ncu capture (the exact and the tolerance mode's force pass read and "
+                                           "write the same arrays, the density pass is one)"},
             "finite": bool(np.isfinite(s).all()),
             "cpu_baseline": {"value": 4096 * k / secs, "unit": METRIC, "cores": 1, "kind": "port",
                              "sample": f"{k} in-place steps of a 4096-particle 3D dam break (the reference's cap)"}}

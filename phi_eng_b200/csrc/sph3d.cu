@@ -1214,7 +1214,9 @@ __device__ __forceinline__ void finish3(uint32_t s, uint32_t id, uint32_t* __res
 // Force + XSPH + integrate + walls (fluid3.rs:1040-1176); writes the new
 // state (id order), the next key and its bucket count. DEBUG: forces only.
 // FAST (tolerance mode; PLAIN, uniform mass): pair3_fast's arithmetic.
-constexpr uint32_t kForceThreads3 = 128;  // 128-thread blocks: 286 -> 280 us at 1M (256, 5-block cap: 329 us)
+// 12 steps of 10^6 particles: 4,866 us, with 256 threads 4,952 (tolerance mode
+// 3,952 and 4,025); of 80,000 745 and 742 (628 and 620).
+constexpr uint32_t kForceThreads3 = 128;
 template <bool MASS, bool DEBUG, bool PLAIN, bool FAST = false>
 __global__ void __launch_bounds__(kForceThreads3) k_force3(const float4* __restrict__ spos, const float4* __restrict__ svel,
                                                 const float2* __restrict__ sdq, const uint32_t* __restrict__ skey,

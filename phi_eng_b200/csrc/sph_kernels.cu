@@ -947,8 +947,7 @@ __global__ void __launch_bounds__(256) k_closure_check(const float2* __restrict_
   __shared__ bool s_last;
   __shared__ float red[3][8];
   float v[3] = {0.0f, 0.0f, 0.0f};
-  // grid-stride, then warp and block maxima: one atomic per block and value
-  // (per-warp atomics on three addresses serialised to ~67 us at 2^20)
+  // grid-stride, then warp and block maxima, left in parts by the block
   for (uint32_t s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
     const StepParams& P = scene_params<BATCH>(P0, bt.ptab, BATCH ? bt.sscene[s] : 0u);
     const uint32_t ph = PHASE ? min((uint32_t)sphase[s], 3u) : P.uniform_phase;

@@ -16,8 +16,8 @@
 //                     sample dimension as K (tensor cores), dW3 and the bias
 //                     gradients in FP32; one partial vector per CTA.
 //   k_mlp_adam        per parameter: sum of the CTA partials in CTA order,
-//                     Adam, new FP32 master and its BF16 fragment images.
-//   k_mlp_advance     step counter + 1.
+//                     Adam, new FP32 master and its BF16 fragment images; the
+//                     last block adds one to the step counter.
 // No float atomics anywhere: a run is bit-reproducible.
 //
 // Minibatch sample k of step t is pair
