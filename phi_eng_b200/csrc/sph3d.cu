@@ -2270,6 +2270,7 @@ bool capture_substeps3(World3* w, const StepParams3& P, uint32_t steps, cudaGrap
 
 // `count` substeps from cached graphs, as the 2D step.
 bool run_substeps3(World3* w, const StepParams3& P, uint32_t count) {
+  uint32_t before = kGraphAfter;  // substeps run with these parameters when the call began
   while (count) {
     std::string sig((const char*)&P, sizeof(P));
     sig.append((const char*)&w->n, sizeof(w->n));
@@ -2281,8 +2282,9 @@ bool run_substeps3(World3* w, const StepParams3& P, uint32_t count) {
       w->gsig = sig;
       w->gruns = 0;
     }
+    before = std::min(before, w->gruns);
     const bool many =
-        use_long_graph(w->gsteps != nullptr, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
+        use_long_graph(w->gsteps != nullptr, before, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
     if (many && !w->gsteps && !capture_substeps3(w, P, kGraphSteps, &w->gsteps)) return false;
     const uint32_t k = many ? kGraphSteps : 1u;
     if (!ok3(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream))) return false;

@@ -24,15 +24,16 @@ constexpr float kMaxDt = 1.0f / 15.0f;          // ffi.rs:80
 // parameters: from one graph to the next the GPU stands still for some 1.5 us
 // that kernels inside a graph do not cost (20 steps of 32,499 particles 432 ->
 // 404 us, 10 steps of 2^18 389 -> 376 us, of 2^20 932 -> 920 us). The longer
-// graph costs another capture, some 70 us: it is made for parameters that have run
-// kGraphAfter substeps, or kGraphSoon where the call still has kGraphRest to go.
+// graph costs another capture, some 70 us: it is made for parameters that ran
+// kGraphAfter substeps before this call, or in it where kGraphRest are still to go.
 // Calls of 20, 30 and 100 steps of 32,768 particles, each with a time step of its
-// own: 527, 821 and 2,227 us; always from kGraphSoon on 580, 841 and 2,219.
+// own: 527, 821 and 2,227 us; always after kGraphAfter 580, 841 and 2,219.
 constexpr uint32_t kGraphSteps = 4;
-constexpr uint32_t kGraphSoon = 16, kGraphRest = 32, kGraphAfter = 48;
-// Whether the longer graph runs next: `made` = it is there, `ran` substeps so far.
-inline bool use_long_graph(bool made, uint32_t ran, uint32_t left) {
-  return left >= kGraphSteps && (made || ran >= kGraphAfter || (ran >= kGraphSoon && left >= kGraphRest));
+constexpr uint32_t kGraphAfter = 16, kGraphRest = 32;
+// Whether the longer graph runs next: `made` = it is there; substeps run with its
+// parameters before this call, so far, and left.
+inline bool use_long_graph(bool made, uint32_t before, uint32_t ran, uint32_t left) {
+  return left >= kGraphSteps && (made || before >= kGraphAfter || (ran >= kGraphAfter && left >= kGraphRest));
 }
 
 // The world's device while in scope, for launches in calls that only copied or

@@ -732,6 +732,7 @@ bool capture_substeps(World2* w, const StepParams& P, uint32_t steps, cudaGraphE
 // `count` substeps, replayed from cached CUDA graphs while the launch
 // parameters stay the same.
 bool run_substeps(World2* w, const StepParams& P, uint32_t count) {
+  uint32_t before = kGraphAfter;  // substeps run with these parameters when the call began
   while (count) {
     // Buffer reallocations release the graphs, so the parameters and the
     // particle count identify them.
@@ -745,8 +746,9 @@ bool run_substeps(World2* w, const StepParams& P, uint32_t count) {
       w->gsig = sig;
       w->gruns = 0;
     }
+    before = std::min(before, w->gruns);
     const bool many =
-        use_long_graph(w->gsteps != nullptr, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
+        use_long_graph(w->gsteps != nullptr, before, w->gruns, count) && w->sid_perm_n == w->n && !w->profiling;
     if (many && !w->gsteps && !capture_substeps(w, P, kGraphSteps, &w->gsteps)) return false;
     const uint32_t k = many ? kGraphSteps : 1u;
     if (!cuda_ok(w, cudaGraphLaunch(many ? w->gsteps : w->gexec, w->stream), "graph launch")) return false;
