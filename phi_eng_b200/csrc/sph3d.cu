@@ -46,13 +46,14 @@ constexpr uint32_t kMaxParticles3D = 4096;  // MAX_PARTICLES_3D (fluid3.rs:28)
 // a split only happens while the output holds fewer than MAX_PARTICLES_3D - 1
 // particles, so at most MAX_PARTICLES_3D / 2 particles split.
 // Rows of the state kept on the host, so that further reads, and a read after a
-// write, stay host copies as long as the state stands. Written rows: 96 take 3 us
-// kept and 12 sent at once, 16,384 and more are faster sent. Read rows: up to 4,096
-// from the first read on (the packing kernel writes them there itself), above that
-// from the second read of the same state on (16,384 rows: 46 us from the device, 8
-// kept), and none above 131,072, where a read from the device takes no longer than
-// the host's loop did (262,144 rows: 339 against 419).
-constexpr uint32_t kSetRows = 8192, kKeepRows = 4096, kKeepRowsAgain = 131072;
+// write, stay host copies as long as the state stands. Up to kKeepRows they lie in
+// page-locked memory, which the packing and unpacking kernels access themselves:
+// the rows written until the next step takes them, and the rows read from the first
+// read on. Of larger sets the rows read are kept from the second read of the same
+// state on (16,384 rows: 46 us from the device, 8 kept), and none above
+// kKeepRowsAgain, where a read from the device takes no longer than the host's loop
+// did (262,144 rows: 339 against 419).
+constexpr uint32_t kKeepRows = 4096, kKeepRowsAgain = 131072;
 inline uint32_t resample_bound3(uint32_t n) { return n + std::min(n, kMaxParticles3D / 2); }
 constexpr uint32_t kMaskBits3 = 32;
 
@@ -1533,12 +1534,14 @@ struct World3 {
   uint32_t n = 0;
   std::vector<float4> h_pos, h_vel;  // the state while host_valid
   // the state's first rows_n rows in the caller's layout, as read or set last
-  // (host_valid or not), in h_rows or, page-locked, behind h_pinned's words;
-  // read_past: this state was read past them
+  // (host_valid or not), in h_rows or in the page-locked row_window; read_past: this
+  // state was read past them; rows_taking: a launch that reads row_window may
+  // not have run yet
   std::vector<float> h_rows;
   const float* rows = nullptr;
   uint32_t rows_n = 0;
-  bool read_past = false;
+  bool read_past = false, rows_taking = false;
+  float* row_window() const { return reinterpret_cast<float*>(h_pinned + 16); }
   std::vector<float> h_mass, h_dens, h_pres;  // density / pressure as of dp_dev == false
   std::vector<uint8_t> h_phase;
   bool mass_uniform = true, phase_uniform = true;
@@ -1844,12 +1847,18 @@ void enqueue_keys3(World3* w, cudaStream_t st) {
   if (w->n) k_keys3<<<cdiv(w->n, 256), 256, 0, st>>>(w->pos, w->n, w->plan, w->key, w->count);
 }
 
-// Rows of the caller's layout into the device state (through the mask array,
-// which holds nothing between steps), in stream order.
+// Rows of the caller's layout into the device state, in stream order: the row window
+// is read by the kernel itself, others go through the mask array, which holds nothing
+// between steps.
 bool upload_rows3(World3* w, const float* rows) {
   OnDevice on(w->device);
-  float2* d = reinterpret_cast<float2*>(w->nmask);
-  if (!ok3(w, cudaMemcpyAsync(d, rows, 24 * (size_t)w->n, cudaMemcpyHostToDevice, w->stream))) return false;
+  const float2* d = reinterpret_cast<const float2*>(rows);
+  if (rows == w->row_window()) {
+    w->rows_taking = true;
+  } else {
+    d = reinterpret_cast<const float2*>(w->nmask);
+    if (!ok3(w, cudaMemcpyAsync(w->nmask, rows, 24 * (size_t)w->n, cudaMemcpyHostToDevice, w->stream))) return false;
+  }
   k_unpack3<<<cdiv(w->n, 256), 256, 0, w->stream>>>(d, w->n, w->pos, w->vel);
   return ok3(w, cudaGetLastError());
 }
@@ -3023,7 +3032,7 @@ uint32_t phieng_world3_fluid_get(const World3* cw, float* out, uint32_t max) {
       // rows made on the device: few straight into page-locked memory, the others
       // in the mask array, which holds nothing between steps, then one copy
       const bool few = n <= kKeepRows, keep = few || (n <= kKeepRowsAgain && w->read_past);
-      float* to = few ? reinterpret_cast<float*>(w->h_pinned + 16) : out;
+      float* to = few ? w->row_window() : out;
       if (keep && !few) {
         if (w->h_rows.size() < 6 * (size_t)n) w->h_rows.resize(6 * (size_t)n);
         to = w->h_rows.data();
@@ -3035,6 +3044,7 @@ uint32_t phieng_world3_fluid_get(const World3* cw, float* out, uint32_t max) {
           (!few && !ok3(w, cudaMemcpyAsync(to, made, 24 * (size_t)n, cudaMemcpyDeviceToHost, w->stream))) ||
           !ok3(w, cudaStreamSynchronize(w->stream)))
         return 0;
+      w->rows_taking = false;
       if (!keep) {
         w->read_past = true;
         return n;
@@ -3206,11 +3216,14 @@ int32_t phieng_sph3_set_state(World3* w, const float* xyzv, uint32_t n) {
     // this takes 4. Few rows are kept here and uploaded by the next step; many
     // go straight from the caller's buffer.
     if (!ensure_host_dp3(w)) return 0;
-    const bool keep = n <= kSetRows;
-    if (keep)
-      w->h_rows.assign(xyzv, xyzv + 6 * (size_t)n);
-    else if (!upload_rows3(w, xyzv))
+    const bool keep = n <= kKeepRows;
+    if (keep) {
+      if (w->rows_taking && !ok3(w, cudaStreamSynchronize(w->stream))) return 0;
+      w->rows_taking = false;
+      std::memcpy(w->row_window(), xyzv, 24 * (size_t)n);
+    } else if (!upload_rows3(w, xyzv)) {
       return 0;
+    }
     Bounds3 b;
     for (uint32_t i = 0; i < n; i++) b.add(xyzv[6 * (size_t)i], xyzv[6 * (size_t)i + 1], xyzv[6 * (size_t)i + 2]);
     // from page-locked memory the copy is still on its way here, and the caller
@@ -3218,7 +3231,7 @@ int32_t phieng_sph3_set_state(World3* w, const float* xyzv, uint32_t n) {
     if (!keep && !ok3(w, cudaStreamSynchronize(w->stream))) return 0;
     plan_bounds3(w, b);
     state_on_device3(w);
-    w->rows = w->h_rows.data();
+    w->rows = w->row_window();
     w->rows_n = keep ? n : 0;
     w->dev_valid = !keep;
     w->keys_valid = false;

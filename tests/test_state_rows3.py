@@ -1,6 +1,6 @@
 """Host copies of a 3D world's state: reads (whole, partial, repeated), writes and
 the calls between them always see the latest state, on both sides of the sizes
-at which the world keeps rows on the host (8,192 written, 4,096 and 131,072
+at which the world keeps rows on the host (4,096 written, 4,096 and 131,072
 read), against a world of the same particles that is only stepped and read."""
 import ctypes as C
 
@@ -138,4 +138,30 @@ def test_cfl_substeps_after_a_write(n):
     w.fluid.set_state(b)
     w.step_n(1 / 600, 2)
     np.testing.assert_array_equal(read(w, n), reference(b, 2, cfl=True))
+    w.close()
+
+
+@pytest.mark.parametrize("n", [64, 4096])
+def test_writes_in_quick_succession(n):
+    """A written state that its step has not taken yet is not overwritten by the next."""
+    import torch
+
+    a = [lattice(n, k) for k in range(6)]
+    w = world(a[0])
+    s = torch.cuda.Stream()
+    w.set_stream(s.cuda_stream)
+    got, busy = [], torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    for q in a:
+        with torch.cuda.stream(s):
+            for _ in range(8):
+                busy.fill_(1)  # the step below waits behind these
+        w.fluid.set_state(q)
+        w.step(1 / 600)
+    got.append(read(w, n))
+    np.testing.assert_array_equal(got[0], reference(a[-1], 1))
+    for q in a:
+        w.fluid.set_state(q)
+        w.debug_forces()  # takes the state without stepping
+    w.step(1 / 600)
+    np.testing.assert_array_equal(read(w, n), reference(a[-1], 1))
     w.close()
